@@ -331,6 +331,7 @@ struct OpArgs {
   const int* active; // contiguous only, nullable: rows of inactive solves are left as they are
   float kunit;       // 2 pi / L of the axis (deriv 2, 3)
   long ss_in;        // contiguous only: solve stride of in (0: ss)
+  const float* eadd; // contiguous only, nullable: per-solve value added to the last field
 };
 
 template <int N, int T, bool STRIDED>
@@ -389,6 +390,16 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_op(OpArgs a) {
     if (comp) {
 #pragma unroll
       for (int r = 0; r < B; ++r) w[r] = make_float2(w0[r].x - w[r].x, w0[r].y - w[r].y);
+    }
+    if constexpr (!STRIDED) {
+      if (a.eadd != nullptr && valid && c + 2 >= a.nf) {
+        const float e = a.eadd[(blockIdx.x * T + p) / a.rps];
+#pragma unroll
+        for (int n2 = 0; n2 < B; ++n2) {
+          if (two) w[n2].y += e;
+          else w[n2].x += e;
+        }
+      }
     }
     if (valid) {
 #pragma unroll

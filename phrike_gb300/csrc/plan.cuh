@@ -34,6 +34,7 @@ struct ps_plan_s {
   // 2D Euler from 256 rows: the last pass writes the right-hand side R (4
   // fields) and an elementwise kernel applies the RK stage and the clamp
   bool split2d = false;
+  bool spec = false;  // steps run on the truncated-spectra passes (spectral.cuh)
   float* R2 = nullptr;
   // 3D Euler with gravity: a second stage input (nc fields).  The last pass
   // reads the stage input for the gravity source one component pair at a

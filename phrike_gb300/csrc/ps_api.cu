@@ -22,6 +22,7 @@
 #include "mhd3d.cuh"
 #include "plan.cuh"
 #include "reduce.cuh"
+#include "spectral.cuh"
 
 namespace {
 
@@ -323,9 +324,10 @@ ps::StridedGeom geom_z(const ps_plan_s* p) {
 // One-axis operator on nf fields per solve (P, D or complementary P), axis 0 = x.
 // One-axis operator (deriv: 0 P, 1 D, 2 Laplacian factor L, 3 raw second derivative)
 // on nf fields.  ss_in (axis 0 only): solve stride of `in` when it is a field
-// subset of a wider state (0: the nf-field stride of `out`).
+// subset of a wider state (0: the nf-field stride of `out`).  add_eref (axis
+// 0, power-of-two plans): the last field leaves the energy-perturbation form.
 int apply_op(ps_plan p, int axis, const float* in, float* out, int nf, int deriv, float scale, cudaStream_t s,
-             bool complement = false, const int* active = nullptr, long ss_in = 0) {
+             bool complement = false, const int* active = nullptr, long ss_in = 0, bool add_eref = false) {
   ProfScope prof(p, s, PS_KIND_OP, 8.0 * nf * p->cells * p->nsolve);
   if (p->mr) return ps::mr_apply_op(p, axis, in, out, nf, deriv, scale, complement, active, ss_in, s);
   cudaError_t e;
@@ -347,6 +349,7 @@ int apply_op(ps_plan p, int axis, const float* in, float* out, int nf, int deriv
     a.deriv = deriv;
     a.scale = scale;
     a.complement = complement ? 1 : 0;
+    a.eadd = add_eref ? p->eref : nullptr;
     e = ps::dispatch_n_1d(p->n[0], [&](auto nc) { return ps::launch_op<decltype(nc)::value>(false, a, s); });
   } else {
     if (nf > 63) return fail(PS_ERR_INVALID, "at most 63 fields per operator call");
@@ -987,6 +990,263 @@ int steps_mhd(ps_plan p, float* U, int nsteps, double dt, const double* d_dt, do
 }
 
 // ---------------------------------------------------------------------------
+// Fixed-step and CFL stepping on the truncated-spectra passes (spectral.cuh):
+// 2D/3D Euler and ideal MHD on power-of-two grids with the 2/3 mask.  Gravity
+// and artificial viscosity add terms that are not band-limited and explicit
+// diffusion a Laplacian of the stage input, and without the mask nothing is
+// truncated: those plans, and the bare right-hand sides of ps_rhs and of
+// adaptive stepping, run the real-space passes.
+// ---------------------------------------------------------------------------
+bool spec_plan(const ps_plan_desc* d) {
+  if (d->ndim < 2 || is_lgl(d) || is_mr(d) || !d->dealias || d->av_mode != PS_AV_OFF) return false;
+  if (d->equations == PS_EQ_MHD) return d->mhd_resistivity == 0.0 && d->mhd_viscosity == 0.0;
+  for (int a = 0; a < d->ndim; ++a)
+    if (d->gravity[a] != 0.0) return false;
+  return true;
+}
+
+// Buffers of the truncated passes inside the plan's scratch (sizes in
+// spectral.cuh's wide rows; every length fits, the smallest grids included):
+// G holds the flux spectra (and the increment in the place of the first),
+// AB / Us the y-transformed operands, acc the spectral accumulator.
+struct SpecBufs {
+  int pitch, ncol;
+  long wide;        // complex elements of one wide array (all solves)
+  float2* G;
+  float2* A;        // 3D: P operand of the last axis; 2D: G
+  float2* Bo;       // 3D: D operand
+  float2* acc;
+  float* Bp;        // MHD: projected B of U^n, [nsolve][nd][cells]
+};
+
+SpecBufs spec_bufs(ps_plan p) {
+  SpecBufs b{};
+  b.pitch = ps::spec_pitch(p->n[0], p->nc);
+  b.ncol = ps::spec_cols(p->n[0], p->nc);
+  b.wide = (long)p->rows() * p->nsolve * b.pitch;
+  b.G = reinterpret_cast<float2*>(p->G);
+  b.acc = reinterpret_cast<float2*>(p->acc);
+  b.A = b.G;
+  b.Bo = b.G + b.wide;
+  if (p->mhd) b.Bp = p->Us;
+  if (p->nd == 3) {
+    const long part = (long)p->nsolve * p->n[2] * ps::spec_modes(p->n[1]) * b.pitch;
+    if (p->mhd) {  // A behind the projected B in Us (8 fields), B behind the three arrays of G (24 fields)
+      b.A = reinterpret_cast<float2*>(p->Us + (long)3 * p->cells * p->nsolve);
+      b.Bo = b.G + 3 * b.wide;
+    } else {
+      b.A = reinterpret_cast<float2*>(p->AB);
+      b.Bo = b.A + part;
+    }
+  }
+  return b;
+}
+
+// x rows: the state (U^n, or U^n plus the increment when inc) and, when flux,
+// its flux spectra.  Uw: where the state goes (px: the filtered U^n).
+int spec_x(ps_plan p, const SpecBufs& b, bool inc, bool flux, const float* U, float* Uw, bool px, bool use_bp,
+           float* speed, bool shift_in, bool shift_out, cudaStream_t s, const int* act) {
+  ps::SpecXArgs a{};
+  a.U = U;
+  a.Uw = Uw;
+  a.Bp = use_bp ? b.Bp : nullptr;
+  a.nproj = p->nd;
+  a.D = b.G;
+  a.G = b.G;
+  a.gs = b.wide;
+  a.pitch = b.pitch;
+  a.fs = p->cells;
+  a.ssU = p->ss(p->nc);
+  a.rps = p->rows();
+  a.rows = a.rps * p->nsolve;
+  a.row0 = 0;
+  a.nrow = a.rows;
+  a.ax = p->ax(0);
+  a.gamma = (float)p->desc.gamma;
+  a.rho_min = p->mhd ? (float)p->desc.mhd_rho_min : 1e-8f;  // clamp floors (solver.py:467, 876-877)
+  a.p_min = p->mhd ? (float)p->desc.mhd_p_min : 1e-10f;
+  a.speed = speed;
+  a.eref = p->eref;
+  a.active = act;
+  a.px = px ? 1 : 0;
+  a.shift_in = shift_in ? 1 : 0;
+  a.shift_out = shift_out ? 1 : 0;
+  const double wide = 8.0 * b.ncol * a.rows;
+  ProfScope prof(p, s, PS_KIND_X, wide * ((inc ? 1 : 0) + (flux ? p->nd : 0)) +
+                                      4.0 * p->cells * p->nsolve * p->nc * (1 + (Uw ? 1 : 0)));
+  cudaError_t e = ps::dispatch_n(p->n[0], [&](auto nn) {
+    constexpr int N = decltype(nn)::value;
+    return p->mhd ? ps::launch_spec_x<N, 1>(p->nd, inc, flux, a, s) : ps::launch_spec_x<N, 0>(p->nd, inc, flux, a, s);
+  });
+  if (e != cudaSuccess) return cuda_fail(e, "x pass");
+  return PS_OK;
+}
+
+// from the flux spectra to the stage's increment spectra (wide rows in G)
+int spec_stage(ps_plan p, const SpecBufs& b, int stage, double dt, const double* d_dt, cudaStream_t s,
+               const int* act) {
+  cudaError_t e;
+  const int planes = p->n[2] * p->nsolve;
+  const int My = ps::spec_modes(p->n[1]);
+  const double wide = 8.0 * b.ncol * p->rows() * p->nsolve;
+  const double part = wide * My / p->n[1];
+  if (p->nd == 3) {
+    ps::SpecFArgs f{};
+    f.G = b.G;
+    f.gs = b.wide;
+    f.out = b.A;
+    f.os = b.Bo - b.A;
+    f.pitch = b.pitch;
+    f.ncol = b.ncol;
+    f.plane0 = 0;
+    f.pps = p->n[2];
+    f.ax = p->ax(1);
+    f.active = act;
+    ProfScope prof(p, s, PS_KIND_Y, 3.0 * wide + 2.0 * part);
+    e = ps::dispatch_n(p->n[1], [&](auto nn) { return ps::launch_spec_f<decltype(nn)::value>(f, planes, s); });
+    if (e != cudaSuccess) return cuda_fail(e, "y pass");
+  }
+  {
+    ps::SpecCArgs c{};
+    c.a = b.A;
+    c.b = b.Bo;
+    c.out = b.A;
+    c.acc = b.acc;
+    c.ncol = b.ncol;
+    const int ax = p->nd - 1;
+    if (p->nd == 3) {  // [solve][z][ky][col]
+      c.os = b.pitch;
+      c.as = (long)My * b.pitch;
+      c.nouter = My;
+    } else {  // [solve][y][col]
+      c.as = b.pitch;
+      c.nouter = 1;
+    }
+    c.ss = (long)p->n[ax] * c.nouter * b.pitch;
+    c.acc_as = (long)c.nouter * b.pitch;
+    c.acc_os = c.os;
+    c.acc_ss = (long)ps::spec_modes(p->n[ax]) * c.nouter * b.pitch;
+    c.ax = p->ax(ax);
+    c.stage = stage;
+    c.rk2 = (p->desc.scheme == PS_SCHEME_RK2) ? 1 : 0;
+    c.dt_dev = d_dt;
+    c.dt = dt;
+    c.active = act;
+    const double in = p->nd == 3 ? part : wide;
+    const double ac = in * ps::spec_modes(p->n[ax]) / p->n[ax];
+    ProfScope prof(p, s, PS_KIND_LAST, 3.0 * in + ac * (stage == 0 || stage == 3 ? 1 : 2));
+    e = ps::dispatch_n(p->n[ax], [&](auto nn) { return ps::launch_spec_c<decltype(nn)::value>(c, p->nsolve, s); });
+    if (e != cudaSuccess) return cuda_fail(e, "last pass");
+  }
+  if (p->nd == 3) {
+    ps::SpecIArgs i{};
+    i.in = b.A;
+    i.D = b.G;
+    i.pitch = b.pitch;
+    i.ncol = b.ncol;
+    i.plane0 = 0;
+    i.pps = p->n[2];
+    i.ax = p->ax(1);
+    i.active = act;
+    ProfScope prof(p, s, PS_KIND_Y, part + wide);
+    e = ps::dispatch_n(p->n[1], [&](auto nn) { return ps::launch_spec_i<decltype(nn)::value>(i, planes, s); });
+    if (e != cudaSuccess) return cuda_fail(e, "y inverse pass");
+  }
+  return PS_OK;
+}
+
+// nsteps RK steps of a batch.  The end-of-step filter is the real-space
+// operator along z and y and, for Euler, along x in the next step's first x
+// pass.  Where the filter is the mask alone a 3D Euler step needs it only
+// once per call: the first step's filter leaves the state inside the mask,
+// every later increment lies inside it too (its spectra are stored truncated,
+// and 3D has no clamp), and the projection of a sum of such fields is the sum.
+int steps_spec(ps_plan p, float* U, int nsteps, double dt, const double* d_dt, double* d_t, const double* d_tend,
+               cudaStream_t s) {
+  int rc;
+  const SpecBufs b = spec_bufs(p);
+  const bool cfl = d_t != nullptr;
+  const int* act = cfl ? p->active : nullptr;
+  const double* dtp = cfl ? p->dt : d_dt;
+  const bool euler = !p->mhd;
+  const bool rk2 = p->desc.scheme == PS_SCHEME_RK2;
+  const bool substages = p->mhd && p->desc.mhd_project_substages && p->desc.mhd_divergence_clean;
+  const bool mask_only = euler && p->nd == 3 && !p->desc.filter_enabled;
+  float* UE = U + (long)(p->nc - 1) * p->cells;
+  const long ssU = p->ss(p->nc);
+  if (euler) {
+    PS_CU(ps::launch_eref_set(UE, ssU, p->nsolve, p->eref, s), "energy reference");
+    // CFL runs shift the whole batch up front (solves may never start);
+    // fixed steps subtract E_ref on the first step's loads
+    if (cfl) PS_CU(ps::launch_energy_shift(UE, p->cells, ssU, p->nsolve, p->eref, -1.0f, s), "energy shift");
+  }
+  if (cfl) {
+    PS_CU(cudaMemsetAsync(p->speed, 0, sizeof(float) * p->nsolve, s), "speed reset");
+    PS_CU(ps::launch_fill_int(p->active, p->nsolve, 1, s), "active reset");
+  }
+  if (substages) {
+    // the projection of the stage states replaces U^n's B by its projection;
+    // later steps start from a projected state
+    const size_t w = (size_t)p->nd * p->cells * sizeof(float);
+    PS_CU(cudaMemcpy2DAsync(b.Bp, w, U + 5 * p->cells, ssU * sizeof(float), w, p->nsolve, cudaMemcpyDeviceToDevice, s),
+          "B copy");
+    rc = (p->nd == 3) ? project3(p, b.Bp, b.Bp + p->cells, b.Bp + 2 * p->cells, nullptr, 3 * p->cells, act, s)
+                      : project(p, b.Bp, b.Bp + p->cells, nullptr, 2 * p->cells, act, s);
+    if (rc != PS_OK) return rc;
+  }
+  bool pending_px = false, begun = false;
+  for (int it = 0; it < nsteps; ++it) {
+    const bool due = euler ? filter_due(p, p->step_counter) : (p->step_counter % p->desc.filter_interval) == 0;
+    const bool filt = due && !(mask_only && it > 0);
+    const bool last_step = it + 1 == nsteps;
+    const bool sh = euler && !cfl && it == 0;  // U still holds E
+    if (!begun && (rc = spec_x(p, b, false, true, U, pending_px ? U : nullptr, pending_px, false,
+                               cfl ? p->speed : nullptr, sh, false, s, act)) != PS_OK)
+      return rc;
+    begun = false;
+    pending_px = false;
+    if (cfl)
+      PS_CU(ps::launch_step_control(p->speed, p->desc.cfl, p->hmin(), d_t, d_tend, p->nsolve, p->dt, p->active, s,
+                                    p->dt_diff()),
+            "step control");
+    const bool use_bp = substages && it == 0;
+    for (int stage = 0; stage < 4; ++stage) {
+      if (rk2 && (stage == 1 || stage == 2)) continue;  // midpoint RK2
+      if ((rc = spec_stage(p, b, stage, dt, dtp, s, act)) != PS_OK) return rc;
+      if (stage < 3) {
+        rc = spec_x(p, b, true, true, U, nullptr, false, use_bp, nullptr, sh, false, s, act);
+      } else if (!last_step && !cfl && !due) {
+        // nothing between this step's state and the next one's fluxes
+        rc = spec_x(p, b, true, true, U, U, false, use_bp, nullptr, sh, false, s, act);
+        begun = true;
+      } else if (!last_step && !cfl && euler && !filt) {
+        rc = spec_x(p, b, true, true, U, U, false, false, nullptr, sh, false, s, act);
+        begun = true;
+      } else {
+        rc = spec_x(p, b, true, false, U, U, false, use_bp, nullptr, sh, euler && !cfl && last_step && !filt, s, act);
+      }
+      if (rc != PS_OK) return rc;
+    }
+    if (filt) {
+      for (int ax = p->nd - 1; ax >= 1; --ax)
+        if ((rc = apply_op(p, ax, U, U, p->nc, 0, 1.0f, s, true, act)) != PS_OK) return rc;
+      if (euler && !last_step) {
+        pending_px = true;
+      } else {
+        const bool back = euler && !cfl;  // E' -> E in the same pass
+        if ((rc = apply_op(p, 0, U, U, p->nc, 0, 1.0f, s, true, act, 0, back)) != PS_OK) return rc;
+        if (!euler && (rc = project_state(p, U, act, s)) != PS_OK) return rc;
+      }
+    }
+    if (cfl)
+      PS_CU(ps::launch_step_advance(d_t, p->dt, p->speed, p->active, p->steps_done, p->nsolve, s), "step advance");
+    p->step_counter += 1;
+  }
+  if (euler && cfl) PS_CU(ps::launch_energy_shift(UE, p->cells, ssU, p->nsolve, p->eref, 1.0f, s), "energy shift");
+  return PS_OK;
+}
+
+// ---------------------------------------------------------------------------
 // Adaptive embedded RK (adaptive.py:23-437 driven by the run loops of
 // solver.py).  1D: whole attempt loops in k_ark1d.  2D/3D and MHD: one launch
 // sequence per attempt, every decision on the device (adaptive.cu).
@@ -1192,6 +1452,7 @@ int create(const ps_plan_desc* d, int nsolve, ps_plan* out) {
     if (stage_buffer3d(d) && (rc = dalloc(p, &p->Us2, p->nc * c)) != PS_OK) return cleanup(rc);
   }
   p->av = av_params(d);
+  p->spec = spec_plan(d);
   if (p->nd == 2 && !lgl && !mr) {
     const int cap = p->mhd ? ((p->n[1] >= 1024) ? 8 : 16) : ((p->n[1] >= 1024) ? 4 : (p->n[1] >= 256) ? 8 : 16);
     p->tcols = ps::tile_cols_2d(p->n[0], p->n[1], nsolve, p->mhd);
@@ -1408,6 +1669,7 @@ int ps_run_steps(ps_plan p, float* U, int nsteps, double dt, const double* d_dt,
   if (nsteps == 0) return PS_OK;
   cudaStream_t s = (cudaStream_t)stream;
   if (p->lgl) return ps::lgl_steps(p, U, nsteps, dt, d_dt, nullptr, nullptr, s);
+  if (p->spec) return steps_spec(p, U, nsteps, dt, d_dt, nullptr, nullptr, s);
   if (p->mhd) return steps_mhd(p, U, nsteps, dt, d_dt, nullptr, nullptr, s);
   if (p->nd == 1) return step_1d(p, U, nsteps, dt, d_dt, nullptr, nullptr, s);
   return steps_nd(p, U, nsteps, dt, d_dt, nullptr, nullptr, s);
@@ -1419,6 +1681,7 @@ int ps_run_cfl(ps_plan p, float* U, int nsteps, double* d_t, const double* d_ten
   if (nsteps == 0) return PS_OK;
   cudaStream_t s = (cudaStream_t)stream;
   if (p->lgl) return ps::lgl_steps(p, U, nsteps, 0.0, nullptr, d_t, d_tend, s);
+  if (p->spec) return steps_spec(p, U, nsteps, 0.0, nullptr, d_t, d_tend, s);
   if (p->mhd) return steps_mhd(p, U, nsteps, 0.0, nullptr, d_t, d_tend, s);
   if (p->nd == 1) return step_1d(p, U, nsteps, 0.0, nullptr, d_t, d_tend, s);
   return steps_nd(p, U, nsteps, 0.0, nullptr, d_t, d_tend, s);

@@ -1,0 +1,596 @@
+// Fixed-step and CFL stepping of 2D/3D Euler and MHD on power-of-two Fourier
+// grids with the flux spectra kept truncated between the passes.
+//
+// The separable operators (euler_passes.cuh) are applied to every axis by one
+// forward transform only; the inverse transforms act on the contracted
+// right-hand side alone.  Per RK stage:
+//   k_spec_x (x rows)      : U_s = U^n + increment (inverse x transform of its
+//                            spectra), clamp, fluxes, forward x transforms,
+//                            G_d = D_x F^x, P_x F^y, P_x F^z
+//   k_spec_f (y, 3D only)  : forward y, A = P_y G_x + D_y G_y, B = P_y G_z
+//   k_spec_c (last axis)   : forward, k = -(P A + D B), RK accumulator in
+//                            spectral space, stage increment, inverse
+//   k_spec_i (y, 3D only)  : inverse y of the increment
+// The dealias mask drops every mode above N/3 before a pass stores its
+// output, so a transformed axis holds M = 2 (N/3) + 1 of its N modes: the
+// intermediate arrays carry 2/3 of the real-space words per transformed axis
+// and the later transforms run on 2/3 of the pencils.  Against the passes
+// that return to real space after each axis a 3D Euler stage moves 49 words
+// per cell instead of 75 and runs 22 complex pencil transforms per cell
+// instead of 37; a 3D MHD stage moves 77 words instead of 230 (and needs no
+// projection per stage, see steps_spec).  Measured per step against those
+// passes: Taylor-Green 256^3 4.95 -> 3.88 ms, KHI 512^2 x 16 1.06 -> 0.96 ms,
+// Orszag-Tang 512^2 0.456 -> 0.319 ms, 3D MHD 128^3 2.29 -> 1.41 ms.
+//
+// Two real fields travel as one complex field: every operator maps real
+// fields to real fields, so it acts on f + i g as on f and g, and no pass but
+// the x inverse ever looks at the halves.  A "wide" row holds the columns of
+// all component pairs side by side, [pair][mode m]; m counts the kept modes,
+// 0..KM then -KM..-1.  The fifth field of 3D Euler (the energy) stands alone
+// and stores its non-negative modes only.  The y and z passes see plain
+// columns and do not depend on the equations.
+#pragma once
+#include "euler_passes.cuh"
+#include "mhd_passes.cuh"
+
+namespace ps {
+
+// Kept modes of a masked axis and the shape of a wide row.
+__host__ __device__ constexpr int spec_km(int n) { return n / 3; }
+__host__ __device__ constexpr int spec_modes(int n) { return 2 * (n / 3) + 1; }
+// columns of a wide row: full pairs, then half spectra of a single last field
+__host__ __device__ constexpr int spec_cols(int nx, int nc) {
+  return (nc / 2) * spec_modes(nx) + (nc % 2) * (spec_km(nx) + 1);
+}
+// row pitch in complex elements (64-byte rows)
+__host__ __device__ constexpr int spec_pitch(int nx, int nc) { return (spec_cols(nx, nc) + 7) / 8 * 8; }
+
+struct SpecXArgs {
+  const float* U;     // U^n [nsolve][NC][cells]
+  float* Uw;          // nullable: the state after the x filter (no increment) or after the increment is written here
+  const float* Bp;    // MHD, nullable: [nsolve][nproj][cells], the projected B of U^n
+  int nproj;          // fields of B the projection covers (2 in 2D, 3 in 3D)
+  const float2* D;    // increment spectra, wide rows (with an increment)
+  float2* G;          // flux spectra, ND wide arrays
+  long gs;            // complex elements between the arrays of G
+  int pitch;          // complex elements per wide row
+  long fs, ssU;       // elements per field, per solve
+  int rows, rps;      // rows of all solves, of one solve
+  int row0, nrow;     // rows of this launch; D and G hold rows [row0, row0 + nrow)
+  AxisOps ax;
+  float gamma;
+  float rho_min, p_min;
+  float* speed;       // nullable: per-solve max wave speed of the state the fluxes are taken of
+  const float* eref;  // Euler: E_ref per solve
+  const int* active;
+  int px;             // apply the complementary x filter to the loaded state and write it to Uw
+  int shift_in;       // U holds E (subtract E_ref on load)
+  int shift_out;      // Uw takes E (add E_ref on store)
+};
+
+template <int N, int T>
+struct SpecXSmem {
+  AxisSmem<N> ax;
+  float2 buf[Pencil<N, T, false>::BUF];
+  float red[32];
+};
+
+// Column of mode k (0..N-1) inside one pair's M columns, or -1 if masked.
+template <int N>
+__device__ __forceinline__ int spec_col(int k) {
+  constexpr int KM = spec_km(N);
+  if (k <= KM) return k;
+  if (k >= N - KM) return k - (N - 2 * KM - 1);
+  return -1;
+}
+// Whether register r of a pencil thread can hold a kept mode (compile time;
+// N <= 256: k = t + A (r / A) + B (r % A), t in [0, A)).  Transforms whose
+// masked outputs are never read lose the butterflies that produce them.
+template <int N>
+constexpr bool spec_keeps(int r) {
+  if (N > 256) return true;
+  const int lo = Shape<N>::A * (r / Shape<N>::A) + Shape<N>::B * (r % Shape<N>::A);
+  const int hi = lo + Shape<N>::A - 1;
+  return lo <= spec_km(N) || hi >= N - spec_km(N);
+}
+
+template <int DIR, int C>
+__device__ __forceinline__ float mhd3_flux(float rho, float ux, float uy, float uz, float ps, float eps, float ub,
+                                           float Bx, float By, float Bz) {
+  const float un = (DIR == 0) ? ux : (DIR == 1) ? uy : uz;
+  const float Bn = (DIR == 0) ? Bx : (DIR == 1) ? By : Bz;
+  const float mn = rho * un;
+  if constexpr (C == 0) return mn;
+  if constexpr (C == 1) return mn * ux + ((DIR == 0) ? ps : 0.0f) - Bn * Bx;
+  if constexpr (C == 2) return mn * uy + ((DIR == 1) ? ps : 0.0f) - Bn * By;
+  if constexpr (C == 3) return mn * uz + ((DIR == 2) ? ps : 0.0f) - Bn * Bz;
+  if constexpr (C == 4) return eps * un - Bn * ub;
+  if constexpr (C == 5) return (DIR == 0) ? 0.0f : un * Bx - ux * Bn;
+  if constexpr (C == 6) return (DIR == 1) ? 0.0f : un * By - uy * Bn;
+  return (DIR == 2) ? 0.0f : un * Bz - uz * Bn;  // C == 7
+}
+
+// x rows.  INC: the state is U^n plus the increment of a.D; FLUX: fluxes of
+// the state are transformed and stored.  The thread's B points of every
+// component stay in registers (q[c][n2]); a switch over the job index keeps
+// one transform body for all jobs.  PHYS 0 Euler, 1 MHD (8 components).
+template <int N, int T, int ND, int PHYS, bool INC, bool FLUX>
+__global__ void __launch_bounds__(Shape<N>::A * T) k_spec_x(SpecXArgs a) {
+  constexpr int NC = (PHYS == 1) ? 8 : ND + 2;
+  constexpr int NP = NC / 2;            // packed pairs
+  constexpr bool ODD = (NC % 2) != 0;   // a single last field
+  constexpr int NJ = NP + (ODD ? 1 : 0);
+  constexpr int A = Shape<N>::A, B = Shape<N>::B;
+  constexpr int KM = spec_km(N), M = spec_modes(N);
+  using PF = Pencil<N, T, false>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  auto& S = *reinterpret_cast<SpecXSmem<N, T>*>(smem_raw);
+
+  const int t = threadIdx.x % A;
+  const int p = threadIdx.x / A;
+  const int lrow = blockIdx.x * T + p;  // row of the launch
+  const int rend = min(a.row0 + a.nrow, a.rows);
+  const int row = a.row0 + lrow;
+  const int sol = (row < rend ? row : rend - 1) / a.rps;
+  const bool live = a.active == nullptr || a.active[sol] != 0;
+  const bool valid = row < rend && live;
+  {  // a CTA whose rows all belong to inactive solves has nothing to do
+    const int r0 = a.row0 + blockIdx.x * T, r1 = min(r0 + T, rend) - 1;
+    bool any = a.active == nullptr;
+    for (int s2 = r0 / a.rps; !any && s2 <= r1 / a.rps; ++s2) any = a.active[s2] != 0;
+    if (!any) return;
+  }
+  PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
+  load_axis<N>(S.ax, a.ax);
+  const long rbase = (long)sol * a.ssU + (long)(row % a.rps) * N + t;
+  const float er = (PHYS == 0) ? a.eref[sol] : 0.0f;
+  const float eshift = a.shift_in ? er : 0.0f;
+  const float g1 = a.gamma - 1.0f;
+  const float pref = g1 * er;
+  constexpr int CE = (PHYS == 1) ? 4 : NC - 1;  // energy component
+  float q[NC][B];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) {
+      float v = (c == 0) ? 1.0f : 0.0f;
+      if (valid) v = a.U[c * a.fs + rbase + A * n2];  // may alias a.Uw: plain load
+      if (PHYS == 0 && c == CE && valid) v -= eshift;
+      q[c][n2] = v;
+    }
+  }
+  __syncthreads();
+
+  // q[c] (and q[c + 1]) <- op on the pair of job j
+  auto put = [&](int j, auto&& f) {
+    sfor<0, NJ>([&](auto jc) {
+      constexpr int J = decltype(jc)::value;
+      if (j == J) f(jc);
+    });
+  };
+
+  if constexpr (INC) {
+    const float2* Drow = a.D + (long)lrow * a.pitch;
+#pragma unroll 1
+    for (int j = 0; j < NJ; ++j) {
+      float2 v[B];
+      const bool single = ODD && j == NP;
+      const float2* d = Drow + j * M;
+      sfor<0, B>([&](auto rc) {
+        constexpr int r = decltype(rc)::value;
+        v[r] = make_float2(0.0f, 0.0f);
+        if constexpr (spec_keeps<N>(r)) {
+          const int k = pf.kidx(r);
+          int m = spec_col<N>(k);
+          if (ODD && single && m > KM) m = N - k;  // half spectra: X(-k) = conj X(k)
+          if (valid && m >= 0) v[r] = d[m];
+          if (ODD && single && k > KM) v[r].y = -v[r].y;
+        }
+      });
+      pf.inv(v);
+      put(j, [&](auto jc) {
+        constexpr int c = 2 * decltype(jc)::value;
+        constexpr bool two = c + 1 < NC;
+#pragma unroll
+        for (int n2 = 0; n2 < B; ++n2) {
+          q[c][n2] += v[n2].x;
+          if constexpr (two) q[c + 1][n2] += v[n2].y;
+        }
+      });
+    }
+    if constexpr (PHYS == 1) {
+#pragma unroll
+      for (int n2 = 0; n2 < B; ++n2) {
+        float u[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) u[c] = q[c][n2];
+        clamp_mhd(u, a.gamma, a.rho_min, a.p_min);
+        // the stage projection: the increment of B is solenoidal mode by mode
+        // (the induction flux u_i B_j - u_j B_i is antisymmetric), so it only
+        // replaces U^n's B by its projection; E keeps the thermal pressure
+        if (a.Bp != nullptr && valid) {
+#pragma unroll
+          for (int c = 5; c < 8; ++c) {
+            if (c - 5 >= a.nproj) break;
+            const long o = (long)(row % a.rps) * N + t + A * n2;  // within a field
+            const float b = u[c] + (a.Bp[((long)sol * a.nproj + c - 5) * a.fs + o] - a.U[c * a.fs + rbase + A * n2]);
+            u[4] += 0.5f * (b * b - u[c] * u[c]);
+            u[c] = b;
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < 8; ++c) q[c][n2] = u[c];
+      }
+    } else if constexpr (ND == 2) {
+      const float pmin_shift = a.p_min - pref;
+#pragma unroll
+      for (int n2 = 0; n2 < B; ++n2) {
+        float u[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) u[c] = q[c][n2];
+        clamp_state<ND>(u, a.gamma, a.rho_min, pmin_shift);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) q[c][n2] = u[c];
+      }
+    }
+    if (a.Uw != nullptr && valid) {
+      const float so = (PHYS == 0 && a.shift_out) ? er : 0.0f;
+#pragma unroll
+      for (int c = 0; c < NC; ++c)
+#pragma unroll
+        for (int n2 = 0; n2 < B; ++n2)
+          a.Uw[c * a.fs + rbase + A * n2] = (PHYS == 0 && c == CE) ? q[c][n2] + so : q[c][n2];
+    }
+  } else if (a.px) {  // fused x factor of the end-of-step filter (complementary form)
+#pragma unroll 1
+    for (int j = 0; j < NJ; ++j) {
+      float2 v[B];
+      put(j, [&](auto jc) {
+        constexpr int c = 2 * decltype(jc)::value;
+        constexpr int c1 = (c + 1 < NC) ? c + 1 : c;
+#pragma unroll
+        for (int n2 = 0; n2 < B; ++n2) v[n2] = make_float2(q[c][n2], (c + 1 < NC) ? q[c1][n2] : 0.0f);
+      });
+      pf.fwd(v);
+#pragma unroll
+      for (int r = 0; r < B; ++r) {
+        const float s = (1.0f / N) - S.ax.P[pf.kidx(r)];
+        v[r].x *= s;
+        v[r].y *= s;
+      }
+      pf.inv(v);
+      put(j, [&](auto jc) {
+        constexpr int c = 2 * decltype(jc)::value;
+        constexpr int c1 = (c + 1 < NC) ? c + 1 : c;
+#pragma unroll
+        for (int n2 = 0; n2 < B; ++n2) {
+          q[c][n2] -= v[n2].x;
+          if (valid) a.Uw[c * a.fs + rbase + A * n2] = q[c][n2];
+          if constexpr (c + 1 < NC) {
+            q[c1][n2] -= v[n2].y;
+            if (valid) a.Uw[c1 * a.fs + rbase + A * n2] = q[c1][n2];
+          }
+        }
+      });
+    }
+  }
+  if constexpr (FLUX) {
+    // conservative -> primitive in registers; CFL speed
+    constexpr int NV = (PHYS == 1) ? 3 : ND;
+    float smax = 0.0f;
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) {
+      const float rho = q[0][n2];
+      const float rinv = 1.0f / rho;
+      float kin = 0.0f;
+      float vel[NV];
+#pragma unroll
+      for (int d = 0; d < NV; ++d) {
+        vel[d] = q[1 + d][n2] * rinv;
+        kin = fmaf(vel[d], vel[d], kin);
+        q[1 + d][n2] = vel[d];
+      }
+      if constexpr (PHYS == 0) {
+        const float pr = g1 * (q[CE][n2] - 0.5f * rho * kin);
+        q[CE][n2] = pr;
+        if (a.speed != nullptr && valid) {
+          const float cs = sqrtf(a.gamma * (pr + pref) * rinv);
+          float um = fabsf(vel[0]);
+          if (ND == 3) um = fmaxf(um, fmaxf(fabsf(vel[1]), fabsf(vel[NV - 1])));
+          smax = fmaxf(smax, um + cs);  // 2D keeps |u_x| + a only (equations.py:137-147)
+        }
+      } else if (a.speed != nullptr && valid) {  // equations.py:874-887, 1040-1061
+        const float b2 = q[5][n2] * q[5][n2] + q[6][n2] * q[6][n2] + q[7][n2] * q[7][n2];
+        const float pr = g1 * (q[4][n2] - 0.5f * rho * kin - 0.5f * b2);
+        float um = fmaxf(fabsf(vel[0]), fabsf(vel[1]));
+        if (ND == 3) um = fmaxf(um, fabsf(vel[2]));
+        smax = fmaxf(smax, um + sqrtf(fmaxf(a.gamma * pr / rho + b2 / rho, 0.0f)));
+      }
+    }
+    if (a.speed != nullptr) {
+      const int s0 = (a.row0 + blockIdx.x * T) / a.rps;
+      const int s1 = (min((int)(a.row0 + blockIdx.x * T + T), rend) - 1) / a.rps;
+      if (s0 == s1) {
+        const float m = block_max(smax, S.red);
+        if (threadIdx.x == 0) atomic_max_nonneg(a.speed + s0, m);
+      } else if (valid) {  // rows of several small solves in one CTA
+        atomic_max_nonneg(a.speed + sol, smax);
+      }
+    }
+    const float href = a.gamma * er;
+    const float ig1 = 1.0f / g1;
+    // F^dir_c at point n2
+    auto fx = [&](auto dirc, auto cc, int n2) -> float {
+      constexpr int dir = decltype(dirc)::value, c = decltype(cc)::value;
+      if constexpr (PHYS == 1) {
+        const float b2 = q[5][n2] * q[5][n2] + q[6][n2] * q[6][n2] + q[7][n2] * q[7][n2];
+        const float v2 = q[1][n2] * q[1][n2] + q[2][n2] * q[2][n2] + q[3][n2] * q[3][n2];
+        const float ps = g1 * (q[4][n2] - 0.5f * q[0][n2] * v2 - 0.5f * b2) + 0.5f * b2;
+        const float ub = q[1][n2] * q[5][n2] + q[2][n2] * q[6][n2] + q[3][n2] * q[7][n2];
+        return mhd3_flux<dir, c>(q[0][n2], q[1][n2], q[2][n2], q[3][n2], ps, q[4][n2] + ps, ub, q[5][n2], q[6][n2],
+                                 q[7][n2]);
+      } else {
+        const float rho = q[0][n2], ua = q[1 + dir][n2], pr = q[NC - 1][n2];
+        if constexpr (c == 0) return rho * ua;
+        if constexpr (c == NC - 1) {
+          float kin = 0.0f;
+#pragma unroll
+          for (int d = 0; d < ND; ++d) kin = fmaf(q[1 + d][n2], q[1 + d][n2], kin);
+          const float Ep = fmaf(pr, ig1, 0.5f * rho * kin);  // E' = E - E_ref
+          return ((Ep + pr) + href) * ua;                    // (E + p) u_dir
+        }
+        const float rv = rho * ua * q[c][n2];
+        return (c - 1 == dir) ? rv + pr : rv;
+      }
+    };
+#pragma unroll 1
+    for (int job = 0; job < ND * NJ; ++job) {
+      // the state's registers are opaque per job: without this the compiler
+      // keeps flux terms shared by several jobs live across the loop (16
+      // registers each) and spills
+#pragma unroll
+      for (int c = 0; c < NC; ++c)
+#pragma unroll
+        for (int n2 = 0; n2 < B; ++n2) asm volatile("" : "+f"(q[c][n2]));
+      float2 v[B];
+      sfor<0, ND * NJ>([&](auto jc) {
+        constexpr int J = decltype(jc)::value;
+        constexpr int dir = J / NJ, c = 2 * (J % NJ);
+        constexpr int c1 = (c + 1 < NC) ? c + 1 : c;
+        if (job == J) {
+#pragma unroll
+          for (int n2 = 0; n2 < B; ++n2) {
+            v[n2].x = fx(std::integral_constant<int, dir>{}, std::integral_constant<int, c>{}, n2);
+            v[n2].y = (c + 1 < NC) ? fx(std::integral_constant<int, dir>{}, std::integral_constant<int, c1>{}, n2) : 0.0f;
+          }
+        }
+      });
+      const int dir = job / NJ, j = job % NJ;
+      const bool single = ODD && j == NP;
+      pf.fwd(v);
+      float2* g = a.G + dir * a.gs + (long)lrow * a.pitch + j * M;
+      sfor<0, B>([&](auto rc) {
+        constexpr int r = decltype(rc)::value;
+        if constexpr (spec_keeps<N>(r)) {
+          const int k = pf.kidx(r);
+          const int m = spec_col<N>(k);
+          float2 w;
+          if (dir == 0) {
+            const float dd = S.ax.d[k];
+            w = make_float2(-v[r].y * dd, v[r].x * dd);
+          } else {
+            const float s = S.ax.P[k];
+            w = make_float2(v[r].x * s, v[r].y * s);
+          }
+          if (valid && m >= 0 && !(ODD && single && m > KM)) g[m] = w;
+        }
+      });
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Strided passes over wide columns: T adjacent columns per CTA, A threads per
+// column.  Points and modes go straight between global memory and registers:
+// a tile row is T * 8 bytes (whole 32-byte sectors), all of a pencil's loads
+// are issued before its transform, and the next pencil's loads overlap it.
+// ---------------------------------------------------------------------------
+struct SpecFArgs {
+  const float2* G;   // ND wide arrays, planes [plane][N][pitch] of the launch
+  long gs;
+  float2* out;       // A, then B at out + os: [plane of all][M][pitch]
+  long os;
+  int pitch, ncol;
+  int plane0;        // first plane of the launch (G holds planes from plane0)
+  int pps;           // planes per solve
+  AxisOps ax;
+  const int* active;
+};
+
+template <int N, int T>
+struct SpecSmem {
+  AxisSmem<N> ax;
+  float2 buf[Pencil<N, T, true>::BUF];
+};
+
+template <int N, int T>
+constexpr int spec_min_blocks() {
+  return (512 / (Shape<N>::A * T)) > 0 ? (512 / (Shape<N>::A * T)) : 1;
+}
+
+template <int N, int T>
+__global__ void __launch_bounds__(Shape<N>::A * T, spec_min_blocks<N, T>()) k_spec_f(SpecFArgs a) {
+  constexpr int A = Shape<N>::A, B = Shape<N>::B, M = spec_modes(N);
+  using PF = Pencil<N, T, true>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  auto& S = *reinterpret_cast<SpecSmem<N, T>*>(smem_raw);
+  const int p = threadIdx.x % T, t = threadIdx.x / T;
+  const int col = blockIdx.x * T + p;
+  const int plane = a.plane0 + blockIdx.y;
+  if (a.active != nullptr && a.active[plane / a.pps] == 0) return;
+  const bool valid = col < a.ncol;
+  PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
+  const float2* in = a.G + ((long)blockIdx.y * N + t) * a.pitch + col;
+  const long step = (long)A * a.pitch;
+  float2 v0[B], v1[B];
+#pragma unroll
+  for (int n2 = 0; n2 < B; ++n2) v0[n2] = valid ? in[n2 * step] : make_float2(0.0f, 0.0f);
+#pragma unroll
+  for (int n2 = 0; n2 < B; ++n2) v1[n2] = valid ? in[a.gs + n2 * step] : make_float2(0.0f, 0.0f);
+  load_axis<N>(S.ax, a.ax);
+  __syncthreads();
+  pf.fwd(v0);
+  pf.fwd(v1);
+  float2* out = a.out + (long)plane * M * a.pitch + col;
+  sfor<0, B>([&](auto rc) {
+    constexpr int r = decltype(rc)::value;
+    if constexpr (spec_keeps<N>(r)) {
+      const int k = pf.kidx(r);
+      const int m = spec_col<N>(k);
+      const float P = S.ax.P[k], d = S.ax.d[k];
+      if (valid && m >= 0)
+        out[(long)m * a.pitch] =
+            make_float2(fmaf(P, v0[r].x, -d * v1[r].y), fmaf(P, v0[r].y, d * v1[r].x));
+    }
+  });
+#pragma unroll
+  for (int n2 = 0; n2 < B; ++n2) v0[n2] = valid ? in[2 * a.gs + n2 * step] : make_float2(0.0f, 0.0f);
+  pf.fwd(v0);
+  out += a.os;
+  sfor<0, B>([&](auto rc) {
+    constexpr int r = decltype(rc)::value;
+    if constexpr (spec_keeps<N>(r)) {
+      const int k = pf.kidx(r);
+      const int m = spec_col<N>(k);
+      const float P = S.ax.P[k];
+      if (valid && m >= 0) out[(long)m * a.pitch] = make_float2(P * v0[r].x, P * v0[r].y);
+    }
+  });
+}
+
+// Last axis: k = -(P a + D b), RK bookkeeping in spectral space, increment
+// back along the axis.  RK4: the accumulator holds sum_i w_i k_i of the
+// stages so far; stages 0..2 return wnext k, stage 3 returns the whole
+// increment of the step (rk_update_incr's weights).
+struct SpecCArgs {
+  const float2* a;   // P operand; [outer][N][..] with the strides below
+  const float2* b;   // D operand
+  float2* out;       // increment; may alias a
+  float2* acc;       // accumulator [solve][M][outer][..] (strides acc_as, acc_os)
+  long as, os, ss;   // axis, outer and solve strides (complex elements)
+  long acc_as, acc_os, acc_ss;
+  int ncol, nouter;
+  AxisOps ax;
+  int stage;         // 0..3
+  int rk2;
+  const double* dt_dev;
+  double dt;
+  const int* active;
+  int sol0;
+};
+
+template <int N, int T>
+__global__ void __launch_bounds__(Shape<N>::A * T, spec_min_blocks<N, T>()) k_spec_c(SpecCArgs a) {
+  constexpr int A = Shape<N>::A, B = Shape<N>::B;
+  using PF = Pencil<N, T, true>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  auto& S = *reinterpret_cast<SpecSmem<N, T>*>(smem_raw);
+  const int p = threadIdx.x % T, t = threadIdx.x / T;
+  const int col = blockIdx.x * T + p;
+  const int sol = a.sol0 + blockIdx.y / a.nouter;
+  const int outer = blockIdx.y % a.nouter;
+  if (a.active != nullptr && a.active[sol] == 0) return;
+  const bool valid = col < a.ncol;
+  PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
+  const long base = (long)sol * a.ss + (long)outer * a.os + (long)t * a.as + col;
+  const long step = (long)A * a.as;
+  float2 w[B], z2[B];
+#pragma unroll
+  for (int n2 = 0; n2 < B; ++n2) w[n2] = valid ? a.a[base + n2 * step] : make_float2(0.0f, 0.0f);
+#pragma unroll
+  for (int n2 = 0; n2 < B; ++n2) z2[n2] = valid ? a.b[base + n2 * step] : make_float2(0.0f, 0.0f);
+  load_axis<N>(S.ax, a.ax);
+  const float dt = (a.dt_dev != nullptr) ? (float)a.dt_dev[sol] : (float)a.dt;
+  const RKCoef rk = rk_coef(a.stage, dt, a.rk2);
+  __syncthreads();
+  pf.fwd(w);
+  pf.fwd(z2);
+  float2* acc = a.acc + (long)sol * a.acc_ss + (long)outer * a.acc_os + col;
+  sfor<0, B>([&](auto rc) {
+    constexpr int r = decltype(rc)::value;
+    float2 inc = make_float2(0.0f, 0.0f);
+    if constexpr (spec_keeps<N>(r)) {
+      const int k = pf.kidx(r);
+      const int m = spec_col<N>(k);
+      if (m >= 0) {
+        const float P = -S.ax.P[k], d = -S.ax.d[k];
+        const float2 kk = make_float2(fmaf(P, w[r].x, -d * z2[r].y), fmaf(P, w[r].y, d * z2[r].x));
+        if (a.stage == 3) {
+          const float2 s = valid ? acc[m * a.acc_as] : make_float2(0.0f, 0.0f);
+          inc = make_float2(fmaf(rk.wacc, kk.x, s.x), fmaf(rk.wacc, kk.y, s.y));
+        } else {
+          float2 s = make_float2(0.0f, 0.0f);
+          if (a.stage != 0 && valid) s = acc[m * a.acc_as];
+          if (valid) acc[m * a.acc_as] = make_float2(fmaf(rk.wacc, kk.x, s.x), fmaf(rk.wacc, kk.y, s.y));
+          inc = make_float2(rk.wnext * kk.x, rk.wnext * kk.y);
+        }
+      }
+    }
+    w[r] = inc;
+  });
+  pf.inv(w);
+  if (valid) {
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) a.out[base + n2 * step] = w[n2];
+  }
+}
+
+// 3D: inverse y transform of the increment, [plane][M][pitch] -> wide rows.
+struct SpecIArgs {
+  const float2* in;
+  float2* D;         // planes from plane0: [plane][N][pitch]
+  int pitch, ncol;
+  int plane0, pps;
+  AxisOps ax;
+  const int* active;
+};
+
+template <int N, int T>
+__global__ void __launch_bounds__(Shape<N>::A * T, spec_min_blocks<N, T>()) k_spec_i(SpecIArgs a) {
+  constexpr int A = Shape<N>::A, B = Shape<N>::B, M = spec_modes(N);
+  using PF = Pencil<N, T, true>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  auto& S = *reinterpret_cast<SpecSmem<N, T>*>(smem_raw);
+  const int p = threadIdx.x % T, t = threadIdx.x / T;
+  const int col = blockIdx.x * T + p;
+  const int plane = a.plane0 + blockIdx.y;
+  if (a.active != nullptr && a.active[plane / a.pps] == 0) return;
+  const bool valid = col < a.ncol;
+  PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
+  const float2* in = a.in + (long)plane * M * a.pitch + col;
+  float2 v[B];
+  sfor<0, B>([&](auto rc) {
+    constexpr int r = decltype(rc)::value;
+    v[r] = make_float2(0.0f, 0.0f);
+    if constexpr (spec_keeps<N>(r)) {
+      const int m = spec_col<N>(pf.kidx(r));
+      if (valid && m >= 0) v[r] = in[(long)m * a.pitch];
+    }
+  });
+  load_axis<N>(S.ax, a.ax);
+  __syncthreads();
+  pf.inv(v);
+  if (valid) {
+    float2* out = a.D + ((long)blockIdx.y * N + t) * a.pitch + col;
+    const long step = (long)A * a.pitch;
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) out[n2 * step] = v[n2];
+  }
+}
+
+template <int N, int PHYS> cudaError_t launch_spec_x(int nd, bool inc, bool flux, const SpecXArgs& a, cudaStream_t s);
+template <int N> cudaError_t launch_spec_f(const SpecFArgs& a, int planes, cudaStream_t s);
+template <int N> cudaError_t launch_spec_c(const SpecCArgs& a, int nsol, cudaStream_t s);
+template <int N> cudaError_t launch_spec_i(const SpecIArgs& a, int planes, cudaStream_t s);
+
+}  // namespace ps
