@@ -1042,10 +1042,11 @@ SpecBufs spec_bufs(ps_plan p) {
   return b;
 }
 
-// x rows: the state (U^n, or U^n plus the increment when inc) and, when flux,
-// its flux spectra.  Uw: where the state goes (px: the filtered U^n).
-int spec_x(ps_plan p, const SpecBufs& b, bool inc, bool flux, const float* U, float* Uw, bool px, bool use_bp,
-           float* speed, bool shift_in, bool shift_out, cudaStream_t s, const int* act) {
+// The row passes: the state (U^n, or U^n plus the increment when inc) and,
+// when flux, its flux spectra; in 3D with the y transforms on either side.
+// Uw: where the state goes (px: the filtered U^n).
+int spec_rows(ps_plan p, const SpecBufs& b, bool inc, bool flux, const float* U, float* Uw, bool px, bool use_bp,
+              float* speed, bool shift_in, bool shift_out, cudaStream_t s, const int* act) {
   ps::SpecXArgs a{};
   a.U = U;
   a.Uw = Uw;
@@ -1059,8 +1060,6 @@ int spec_x(ps_plan p, const SpecBufs& b, bool inc, bool flux, const float* U, fl
   a.ssU = p->ss(p->nc);
   a.rps = p->rows();
   a.rows = a.rps * p->nsolve;
-  a.row0 = 0;
-  a.nrow = a.rows;
   a.ax = p->ax(0);
   a.gamma = (float)p->desc.gamma;
   a.rho_min = p->mhd ? (float)p->desc.mhd_rho_min : 1e-8f;  // clamp floors (solver.py:467, 876-877)
@@ -1071,87 +1070,86 @@ int spec_x(ps_plan p, const SpecBufs& b, bool inc, bool flux, const float* U, fl
   a.px = px ? 1 : 0;
   a.shift_in = shift_in ? 1 : 0;
   a.shift_out = shift_out ? 1 : 0;
+  ps::SpecFArgs f{};
+  f.G = b.G;
+  f.gs = b.wide;
+  f.out = b.A;
+  f.os = b.Bo - b.A;
+  f.pitch = b.pitch;
+  f.ncol = b.ncol;
+  f.pps = p->n[2];
+  f.ax = p->ax(1);
+  f.active = act;
+  ps::SpecIArgs i{};
+  i.in = b.A;
+  i.D = b.G;
+  i.pitch = b.pitch;
+  i.ncol = b.ncol;
+  i.pps = p->n[2];
+  i.ax = p->ax(1);
+  i.active = act;
+  f.planes = i.planes = p->n[2] * p->nsolve;
   const double wide = 8.0 * b.ncol * a.rows;
-  ProfScope prof(p, s, PS_KIND_X, wide * ((inc ? 1 : 0) + (flux ? p->nd : 0)) +
-                                      4.0 * p->cells * p->nsolve * p->nc * (1 + (Uw ? 1 : 0)));
-  cudaError_t e = ps::dispatch_n(p->n[0], [&](auto nn) {
-    constexpr int N = decltype(nn)::value;
-    return p->mhd ? ps::launch_spec_x<N, 1>(p->nd, inc, flux, a, s) : ps::launch_spec_x<N, 0>(p->nd, inc, flux, a, s);
-  });
-  if (e != cudaSuccess) return cuda_fail(e, "x pass");
+  const double part = wide * ps::spec_modes(p->n[1]) / p->n[1];
+  cudaError_t e;
+  if (inc && p->nd == 3) {
+    ProfScope prof(p, s, PS_KIND_Y, part + wide);
+    e = ps::dispatch_n(p->n[1], [&](auto nn) { return ps::launch_spec_i<decltype(nn)::value>(i, s); });
+    if (e != cudaSuccess) return cuda_fail(e, "y inverse pass");
+  }
+  {
+    ProfScope prof(p, s, PS_KIND_X, wide * ((inc ? 1 : 0) + (flux ? p->nd : 0)) +
+                                        4.0 * p->cells * p->nsolve * p->nc * (1 + (Uw ? 1 : 0)));
+    e = ps::dispatch_n(p->n[0], [&](auto nn) {
+      constexpr int N = decltype(nn)::value;
+      return p->mhd ? ps::launch_spec_x<N, 1>(p->nd, inc, flux, a, s) : ps::launch_spec_x<N, 0>(p->nd, inc, flux, a, s);
+    });
+    if (e != cudaSuccess) return cuda_fail(e, "x pass");
+  }
+  if (flux && p->nd == 3) {
+    ProfScope prof(p, s, PS_KIND_Y, 3.0 * wide + 2.0 * part);
+    e = ps::dispatch_n(p->n[1], [&](auto nn) { return ps::launch_spec_f<decltype(nn)::value>(f, s); });
+    if (e != cudaSuccess) return cuda_fail(e, "y pass");
+  }
   return PS_OK;
 }
 
-// from the flux spectra to the stage's increment spectra (wide rows in G)
-int spec_stage(ps_plan p, const SpecBufs& b, int stage, double dt, const double* d_dt, cudaStream_t s,
-               const int* act) {
-  cudaError_t e;
-  const int planes = p->n[2] * p->nsolve;
+// last axis: from the flux spectra to the stage's increment spectra
+int spec_last(ps_plan p, const SpecBufs& b, int stage, double dt, const double* d_dt, cudaStream_t s,
+              const int* act) {
   const int My = ps::spec_modes(p->n[1]);
-  const double wide = 8.0 * b.ncol * p->rows() * p->nsolve;
-  const double part = wide * My / p->n[1];
-  if (p->nd == 3) {
-    ps::SpecFArgs f{};
-    f.G = b.G;
-    f.gs = b.wide;
-    f.out = b.A;
-    f.os = b.Bo - b.A;
-    f.pitch = b.pitch;
-    f.ncol = b.ncol;
-    f.plane0 = 0;
-    f.pps = p->n[2];
-    f.ax = p->ax(1);
-    f.active = act;
-    ProfScope prof(p, s, PS_KIND_Y, 3.0 * wide + 2.0 * part);
-    e = ps::dispatch_n(p->n[1], [&](auto nn) { return ps::launch_spec_f<decltype(nn)::value>(f, planes, s); });
-    if (e != cudaSuccess) return cuda_fail(e, "y pass");
+  const int ax = p->nd - 1;
+  ps::SpecCArgs c{};
+  c.a = b.A;
+  c.b = b.Bo;
+  c.out = b.A;
+  c.acc = b.acc;
+  c.ncol = b.ncol;
+  c.nsolve = p->nsolve;
+  if (p->nd == 3) {  // [solve][z][ky][col]
+    c.os = b.pitch;
+    c.as = (long)My * b.pitch;
+    c.nouter = My;
+  } else {  // [solve][y][col]
+    c.as = b.pitch;
+    c.nouter = 1;
   }
-  {
-    ps::SpecCArgs c{};
-    c.a = b.A;
-    c.b = b.Bo;
-    c.out = b.A;
-    c.acc = b.acc;
-    c.ncol = b.ncol;
-    const int ax = p->nd - 1;
-    if (p->nd == 3) {  // [solve][z][ky][col]
-      c.os = b.pitch;
-      c.as = (long)My * b.pitch;
-      c.nouter = My;
-    } else {  // [solve][y][col]
-      c.as = b.pitch;
-      c.nouter = 1;
-    }
-    c.ss = (long)p->n[ax] * c.nouter * b.pitch;
-    c.acc_as = (long)c.nouter * b.pitch;
-    c.acc_os = c.os;
-    c.acc_ss = (long)ps::spec_modes(p->n[ax]) * c.nouter * b.pitch;
-    c.ax = p->ax(ax);
-    c.stage = stage;
-    c.rk2 = (p->desc.scheme == PS_SCHEME_RK2) ? 1 : 0;
-    c.dt_dev = d_dt;
-    c.dt = dt;
-    c.active = act;
-    const double in = p->nd == 3 ? part : wide;
-    const double ac = in * ps::spec_modes(p->n[ax]) / p->n[ax];
-    ProfScope prof(p, s, PS_KIND_LAST, 3.0 * in + ac * (stage == 0 || stage == 3 ? 1 : 2));
-    e = ps::dispatch_n(p->n[ax], [&](auto nn) { return ps::launch_spec_c<decltype(nn)::value>(c, p->nsolve, s); });
-    if (e != cudaSuccess) return cuda_fail(e, "last pass");
-  }
-  if (p->nd == 3) {
-    ps::SpecIArgs i{};
-    i.in = b.A;
-    i.D = b.G;
-    i.pitch = b.pitch;
-    i.ncol = b.ncol;
-    i.plane0 = 0;
-    i.pps = p->n[2];
-    i.ax = p->ax(1);
-    i.active = act;
-    ProfScope prof(p, s, PS_KIND_Y, part + wide);
-    e = ps::dispatch_n(p->n[1], [&](auto nn) { return ps::launch_spec_i<decltype(nn)::value>(i, planes, s); });
-    if (e != cudaSuccess) return cuda_fail(e, "y inverse pass");
-  }
+  c.ss = (long)p->n[ax] * c.nouter * b.pitch;
+  c.acc_as = (long)c.nouter * b.pitch;
+  c.acc_os = c.os;
+  c.acc_ss = (long)ps::spec_modes(p->n[ax]) * c.nouter * b.pitch;
+  c.ax = p->ax(ax);
+  c.stage = stage;
+  c.rk2 = (p->desc.scheme == PS_SCHEME_RK2) ? 1 : 0;
+  c.dt_dev = d_dt;
+  c.dt = dt;
+  c.active = act;
+  const double in = 8.0 * b.ncol * p->n[ax] * c.nouter * p->nsolve;
+  const double ac = in * ps::spec_modes(p->n[ax]) / p->n[ax];
+  ProfScope prof(p, s, PS_KIND_LAST, 3.0 * in + ac * (stage == 0 || stage == 3 ? 1 : 2));
+  cudaError_t e =
+      ps::dispatch_n(p->n[ax], [&](auto nn) { return ps::launch_spec_c<decltype(nn)::value>(c, s); });
+  if (e != cudaSuccess) return cuda_fail(e, "last pass");
   return PS_OK;
 }
 
@@ -1200,7 +1198,7 @@ int steps_spec(ps_plan p, float* U, int nsteps, double dt, const double* d_dt, d
     const bool filt = due && !(mask_only && it > 0);
     const bool last_step = it + 1 == nsteps;
     const bool sh = euler && !cfl && it == 0;  // U still holds E
-    if (!begun && (rc = spec_x(p, b, false, true, U, pending_px ? U : nullptr, pending_px, false,
+    if (!begun && (rc = spec_rows(p, b, false, true, U, pending_px ? U : nullptr, pending_px, false,
                                cfl ? p->speed : nullptr, sh, false, s, act)) != PS_OK)
       return rc;
     begun = false;
@@ -1212,18 +1210,18 @@ int steps_spec(ps_plan p, float* U, int nsteps, double dt, const double* d_dt, d
     const bool use_bp = substages && it == 0;
     for (int stage = 0; stage < 4; ++stage) {
       if (rk2 && (stage == 1 || stage == 2)) continue;  // midpoint RK2
-      if ((rc = spec_stage(p, b, stage, dt, dtp, s, act)) != PS_OK) return rc;
+      if ((rc = spec_last(p, b, stage, dt, dtp, s, act)) != PS_OK) return rc;
       if (stage < 3) {
-        rc = spec_x(p, b, true, true, U, nullptr, false, use_bp, nullptr, sh, false, s, act);
+        rc = spec_rows(p, b, true, true, U, nullptr, false, use_bp, nullptr, sh, false, s, act);
       } else if (!last_step && !cfl && !due) {
         // nothing between this step's state and the next one's fluxes
-        rc = spec_x(p, b, true, true, U, U, false, use_bp, nullptr, sh, false, s, act);
+        rc = spec_rows(p, b, true, true, U, U, false, use_bp, nullptr, sh, false, s, act);
         begun = true;
       } else if (!last_step && !cfl && euler && !filt) {
-        rc = spec_x(p, b, true, true, U, U, false, false, nullptr, sh, false, s, act);
+        rc = spec_rows(p, b, true, true, U, U, false, false, nullptr, sh, false, s, act);
         begun = true;
       } else {
-        rc = spec_x(p, b, true, false, U, U, false, use_bp, nullptr, sh, euler && !cfl && last_step && !filt, s, act);
+        rc = spec_rows(p, b, true, false, U, U, false, use_bp, nullptr, sh, euler && !cfl && last_step && !filt, s, act);
       }
       if (rc != PS_OK) return rc;
     }

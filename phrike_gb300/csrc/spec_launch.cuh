@@ -1,6 +1,8 @@
 // Launchers of the truncated-spectra passes (spectral.cuh), instantiated per
 // pencil length in kern_spec_n*.cu.
 #pragma once
+#include <atomic>
+
 #include "launch.cuh"
 #include "spectral.cuh"
 
@@ -11,7 +13,7 @@ namespace ps {
 // SM.  A pencil's arithmetic does not depend on it.
 template <int NN, typename F>
 cudaError_t dispatch_spec_cols(int ncol, long outer, F&& f) {
-  constexpr int TMAX = (NN >= 1024) ? 8 : 16;
+  constexpr int TMAX = (NN >= 512) ? 8 : 16;
   constexpr int TMIN = cmax_int(4, 32 / Shape<NN>::A);
   if constexpr (TMAX >= 16 && TMIN < 16)
     if ((ncol + 15) / 16 * outer >= 2L * 148) return f(std::integral_constant<int, 16>{});
@@ -25,7 +27,7 @@ cudaError_t spec_x_T(const SpecXArgs& a, cudaStream_t s) {
   const size_t sm = sizeof(SpecXSmem<NN, T>);
   cudaError_t e;
   if ((e = set_smem(k_spec_x<NN, T, ND, PHYS, INC, FLUX>, sm)) != cudaSuccess) return e;
-  k_spec_x<NN, T, ND, PHYS, INC, FLUX><<<(a.nrow + T - 1) / T, Shape<NN>::A * T, sm, s>>>(a);
+  k_spec_x<NN, T, ND, PHYS, INC, FLUX><<<(a.rows + T - 1) / T, Shape<NN>::A * T, sm, s>>>(a);
   return cudaGetLastError();
 }
 template <int NN, int T, int ND, int PHYS>
@@ -35,46 +37,50 @@ cudaError_t spec_x_mode(bool inc, bool flux, const SpecXArgs& a, cudaStream_t s)
   return spec_x_T<NN, T, ND, PHYS, false, true>(a, s);
 }
 
-#define PS_DEFINE_SPEC_LAUNCHERS(NN)                                                                  \
+// A walking grid: as many CTAs as fit the GPU at once, or one per tile.
+template <int NN, int T, typename K>
+cudaError_t spec_grid(K kernel, int threads, size_t sm, long items, int* grid) {
+  static std::atomic<int> known{0};  // per kernel and shape (one instantiation of this function each)
+  int resident = known.load();
+  if (resident == 0) {
+    int per = 0, dev = 0, sms = 0;
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, sm);
+    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    if (per < 1) return cudaErrorInvalidConfiguration;
+    known.store(resident = per * sms);
+  }
+  *grid = (int)(items < resident ? items : resident);
+  return cudaSuccess;
+}
+
+#define PS_DEFINE_SPEC_STRIDED(NN, NAME, ARGS, KERNEL, SMEM, OUTER)                                   \
   template <>                                                                                         \
-  cudaError_t launch_spec_f<NN>(const SpecFArgs& a, int planes, cudaStream_t s) {                     \
-    return dispatch_spec_cols<NN>(a.ncol, planes, [&](auto tw) -> cudaError_t {                       \
+  cudaError_t NAME<NN>(const ARGS& a, cudaStream_t s) {                                               \
+    return dispatch_spec_cols<NN>(a.ncol, OUTER, [&](auto tw) -> cudaError_t {                        \
       constexpr int T = decltype(tw)::value;                                                          \
-      const size_t sm = sizeof(SpecSmem<NN, T>);                                                      \
+      const size_t sm = sizeof(SMEM<NN, T>);                                                                \
       cudaError_t e;                                                                                  \
-      if ((e = set_smem(k_spec_f<NN, T>, sm)) != cudaSuccess) return e;                               \
-      k_spec_f<NN, T><<<dim3((a.ncol + T - 1) / T, planes), Shape<NN>::A * T, sm, s>>>(a);            \
-      return cudaGetLastError();                                                                      \
-    });                                                                                               \
-  }                                                                                                   \
-  template <>                                                                                         \
-  cudaError_t launch_spec_c<NN>(const SpecCArgs& a, int nsol, cudaStream_t s) {                       \
-    return dispatch_spec_cols<NN>(a.ncol, (long)nsol * a.nouter, [&](auto tw) -> cudaError_t {        \
-      constexpr int T = decltype(tw)::value;                                                          \
-      const size_t sm = sizeof(SpecSmem<NN, T>);                                                      \
-      cudaError_t e;                                                                                  \
-      if ((e = set_smem(k_spec_c<NN, T>, sm)) != cudaSuccess) return e;                               \
-      k_spec_c<NN, T><<<dim3((a.ncol + T - 1) / T, nsol * a.nouter), Shape<NN>::A * T, sm, s>>>(a);   \
-      return cudaGetLastError();                                                                      \
-    });                                                                                               \
-  }                                                                                                   \
-  template <>                                                                                         \
-  cudaError_t launch_spec_i<NN>(const SpecIArgs& a, int planes, cudaStream_t s) {                     \
-    return dispatch_spec_cols<NN>(a.ncol, planes, [&](auto tw) -> cudaError_t {                       \
-      constexpr int T = decltype(tw)::value;                                                          \
-      const size_t sm = sizeof(SpecSmem<NN, T>);                                                      \
-      cudaError_t e;                                                                                  \
-      if ((e = set_smem(k_spec_i<NN, T>, sm)) != cudaSuccess) return e;                               \
-      k_spec_i<NN, T><<<dim3((a.ncol + T - 1) / T, planes), Shape<NN>::A * T, sm, s>>>(a);            \
+      int grid;                                                                                       \
+      if ((e = set_smem(KERNEL<NN, T>, sm)) != cudaSuccess) return e;                                 \
+      auto* k = KERNEL<NN, T>;                                                                        \
+      const long items = (long)((a.ncol + T - 1) / T) * (OUTER);                                      \
+      if ((e = spec_grid<NN, T>(k, Shape<NN>::A * T, sm, items, &grid)) != cudaSuccess) return e;     \
+      KERNEL<NN, T><<<grid, Shape<NN>::A * T, sm, s>>>(a);                                            \
       return cudaGetLastError();                                                                      \
     });                                                                                               \
   }
+#define PS_DEFINE_SPEC_LAUNCHERS(NN)                                                                  \
+  PS_DEFINE_SPEC_STRIDED(NN, launch_spec_f, SpecFArgs, k_spec_f, SpecPairSmem, (long)a.planes) \
+  PS_DEFINE_SPEC_STRIDED(NN, launch_spec_c, SpecCArgs, k_spec_c, SpecPairSmem, (long)a.nouter * a.nsolve) \
+  PS_DEFINE_SPEC_STRIDED(NN, launch_spec_i, SpecIArgs, k_spec_i, SpecISmem, (long)a.planes)
 
 // Euler x pass of every length, MHD x pass in a unit of its own
 #define PS_DEFINE_SPEC_X(NN, PHYS)                                                                    \
   template <>                                                                                         \
   cudaError_t launch_spec_x<NN, PHYS>(int nd, bool inc, bool flux, const SpecXArgs& a, cudaStream_t s) { \
-    return dispatch_rows<NN>(a.nrow, [&](auto tw) -> cudaError_t {                                    \
+    return dispatch_rows<NN>(a.rows, [&](auto tw) -> cudaError_t {                                    \
       constexpr int T = decltype(tw)::value;                                                          \
       if (nd == 3) {                                                                                  \
         if constexpr (PHYS == 1 && NN > 256) return cudaErrorInvalidValue; /* 3D MHD: 8..256 */       \

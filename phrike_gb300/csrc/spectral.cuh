@@ -32,6 +32,7 @@
 #pragma once
 #include "euler_passes.cuh"
 #include "mhd_passes.cuh"
+#include "tma.cuh"
 
 namespace ps {
 
@@ -56,7 +57,6 @@ struct SpecXArgs {
   int pitch;          // complex elements per wide row
   long fs, ssU;       // elements per field, per solve
   int rows, rps;      // rows of all solves, of one solve
-  int row0, nrow;     // rows of this launch; D and G hold rows [row0, row0 + nrow)
   AxisOps ax;
   float gamma;
   float rho_min, p_min;
@@ -128,14 +128,12 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_spec_x(SpecXArgs a) {
 
   const int t = threadIdx.x % A;
   const int p = threadIdx.x / A;
-  const int lrow = blockIdx.x * T + p;  // row of the launch
-  const int rend = min(a.row0 + a.nrow, a.rows);
-  const int row = a.row0 + lrow;
-  const int sol = (row < rend ? row : rend - 1) / a.rps;
+  const int row = blockIdx.x * T + p;
+  const int sol = (row < a.rows ? row : a.rows - 1) / a.rps;
   const bool live = a.active == nullptr || a.active[sol] != 0;
-  const bool valid = row < rend && live;
+  const bool valid = row < a.rows && live;
   {  // a CTA whose rows all belong to inactive solves has nothing to do
-    const int r0 = a.row0 + blockIdx.x * T, r1 = min(r0 + T, rend) - 1;
+    const int r0 = blockIdx.x * T, r1 = min(r0 + T, a.rows) - 1;
     bool any = a.active == nullptr;
     for (int s2 = r0 / a.rps; !any && s2 <= r1 / a.rps; ++s2) any = a.active[s2] != 0;
     if (!any) return;
@@ -170,7 +168,7 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_spec_x(SpecXArgs a) {
   };
 
   if constexpr (INC) {
-    const float2* Drow = a.D + (long)lrow * a.pitch;
+    const float2* Drow = a.D + (long)row * a.pitch;
 #pragma unroll 1
     for (int j = 0; j < NJ; ++j) {
       float2 v[B];
@@ -308,8 +306,8 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_spec_x(SpecXArgs a) {
       }
     }
     if (a.speed != nullptr) {
-      const int s0 = (a.row0 + blockIdx.x * T) / a.rps;
-      const int s1 = (min((int)(a.row0 + blockIdx.x * T + T), rend) - 1) / a.rps;
+      const int s0 = (blockIdx.x * T) / a.rps;
+      const int s1 = (min((int)(blockIdx.x * T + T), a.rows) - 1) / a.rps;
       if (s0 == s1) {
         const float m = block_max(smax, S.red);
         if (threadIdx.x == 0) atomic_max_nonneg(a.speed + s0, m);
@@ -368,7 +366,7 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_spec_x(SpecXArgs a) {
       const int dir = job / NJ, j = job % NJ;
       const bool single = ODD && j == NP;
       pf.fwd(v);
-      float2* g = a.G + dir * a.gs + (long)lrow * a.pitch + j * M;
+      float2* g = a.G + dir * a.gs + (long)row * a.pitch + j * M;
       sfor<0, B>([&](auto rc) {
         constexpr int r = decltype(rc)::value;
         if constexpr (spec_keeps<N>(r)) {
@@ -390,28 +388,43 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_spec_x(SpecXArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Strided passes over wide columns: T adjacent columns per CTA, A threads per
-// column.  Points and modes go straight between global memory and registers:
-// a tile row is T * 8 bytes (whole 32-byte sectors), all of a pencil's loads
-// are issued before its transform, and the next pencil's loads overlap it.
+// Strided passes over wide columns: T adjacent columns per tile, A threads per
+// column.  A CTA walks over its share of the tiles; cp.async copies (16 bytes,
+// two columns) bring the next tile's points into shared memory while the
+// present one is transformed, so the transforms do not wait for memory.  A
+// tile row is T * 8 bytes; rows are 64-byte aligned (spec_pitch).
 // ---------------------------------------------------------------------------
-struct SpecFArgs {
-  const float2* G;   // ND wide arrays, planes [plane][N][pitch] of the launch
-  long gs;
-  float2* out;       // A, then B at out + os: [plane of all][M][pitch]
-  long os;
-  int pitch, ncol;
-  int plane0;        // first plane of the launch (G holds planes from plane0)
-  int pps;           // planes per solve
-  AxisOps ax;
-  const int* active;
-};
+__device__ __forceinline__ void cp16(void* dst, const void* src, bool take) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(take ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void cp_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
+}
 
-template <int N, int T>
+// ROWS x T tile at src (row stride as, first column col0) into shared memory;
+// columns from ncol on read as zero.
+template <int ROWS, int T, int THREADS>
+__device__ __forceinline__ void tile_copy(float2* dst, const float2* src, long as, int col0, int ncol) {
+  constexpr int CH = T / 2;
+  for (int i = threadIdx.x; i < ROWS * CH; i += THREADS) {
+    const int r = i / CH, c = 2 * (i % CH);
+    const bool take = col0 + c < ncol;
+    cp16(dst + r * T + c, take ? src + r * as + col0 + c : src, take);
+  }
+}
+
+template <int N, int T, int SLOTS, int ROWS = N>
 struct SpecSmem {
   AxisSmem<N> ax;
   float2 buf[Pencil<N, T, true>::BUF];
+  alignas(16) float2 tile[SLOTS][ROWS * T];
 };
+
+template <int N, int T> using SpecPairSmem = SpecSmem<N, T, 2>;
+template <int N, int T> using SpecISmem = SpecSmem<N, T, 1, spec_modes(N)>;
 
 template <int N, int T>
 constexpr int spec_min_blocks() {
@@ -419,53 +432,95 @@ constexpr int spec_min_blocks() {
 }
 
 template <int N, int T>
+__device__ __forceinline__ void tile_points(float2 (&v)[Shape<N>::B], const float2* tile, int t, int p) {
+#pragma unroll
+  for (int n2 = 0; n2 < Shape<N>::B; ++n2) v[n2] = tile[(t + Shape<N>::A * n2) * T + p];
+}
+
+// 3D y axis, forward: A = P G_x + D G_y and B = P G_z, masked modes dropped.
+struct SpecFArgs {
+  const float2* G;   // 3 wide arrays [plane][N][pitch]
+  long gs;
+  float2* out;       // A, then B at out + os: [plane][M][pitch]
+  long os;
+  int pitch, ncol;
+  int planes, pps;   // planes of all solves, of one solve
+  AxisOps ax;
+  const int* active;
+};
+
+template <int N, int T>
 __global__ void __launch_bounds__(Shape<N>::A * T, spec_min_blocks<N, T>()) k_spec_f(SpecFArgs a) {
   constexpr int A = Shape<N>::A, B = Shape<N>::B, M = spec_modes(N);
   using PF = Pencil<N, T, true>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  auto& S = *reinterpret_cast<SpecSmem<N, T>*>(smem_raw);
+  auto& S = *reinterpret_cast<SpecPairSmem<N, T>*>(smem_raw);
   const int p = threadIdx.x % T, t = threadIdx.x / T;
-  const int col = blockIdx.x * T + p;
-  const int plane = a.plane0 + blockIdx.y;
-  if (a.active != nullptr && a.active[plane / a.pps] == 0) return;
-  const bool valid = col < a.ncol;
   PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
-  const float2* in = a.G + ((long)blockIdx.y * N + t) * a.pitch + col;
-  const long step = (long)A * a.pitch;
-  float2 v0[B], v1[B];
-#pragma unroll
-  for (int n2 = 0; n2 < B; ++n2) v0[n2] = valid ? in[n2 * step] : make_float2(0.0f, 0.0f);
-#pragma unroll
-  for (int n2 = 0; n2 < B; ++n2) v1[n2] = valid ? in[a.gs + n2 * step] : make_float2(0.0f, 0.0f);
+  const int ctiles = (a.ncol + T - 1) / T;
+  const int items = ctiles * a.planes;
+  // first item from w on whose solve is active
+  auto next = [&](int w) {
+    if (a.active != nullptr)
+      while (w < items && a.active[w / ctiles / a.pps] == 0) w += gridDim.x;
+    return w;
+  };
+  auto fetch = [&](int slot, int w, int f) {
+    if (w < items)
+      tile_copy<N, T, A * T>(S.tile[slot], a.G + f * a.gs + (long)(w / ctiles) * N * a.pitch, a.pitch,
+                             (w % ctiles) * T, a.ncol);
+    cp_commit();
+  };
+  int w = next(blockIdx.x);
+  int s = 0;  // slot of the item's first tile
+  fetch(0, w, 0);
+  fetch(1, w, 1);
   load_axis<N>(S.ax, a.ax);
-  __syncthreads();
-  pf.fwd(v0);
-  pf.fwd(v1);
-  float2* out = a.out + (long)plane * M * a.pitch + col;
-  sfor<0, B>([&](auto rc) {
-    constexpr int r = decltype(rc)::value;
-    if constexpr (spec_keeps<N>(r)) {
-      const int k = pf.kidx(r);
-      const int m = spec_col<N>(k);
-      const float P = S.ax.P[k], d = S.ax.d[k];
-      if (valid && m >= 0)
-        out[(long)m * a.pitch] =
-            make_float2(fmaf(P, v0[r].x, -d * v1[r].y), fmaf(P, v0[r].y, d * v1[r].x));
-    }
-  });
-#pragma unroll
-  for (int n2 = 0; n2 < B; ++n2) v0[n2] = valid ? in[2 * a.gs + n2 * step] : make_float2(0.0f, 0.0f);
-  pf.fwd(v0);
-  out += a.os;
-  sfor<0, B>([&](auto rc) {
-    constexpr int r = decltype(rc)::value;
-    if constexpr (spec_keeps<N>(r)) {
-      const int k = pf.kidx(r);
-      const int m = spec_col<N>(k);
-      const float P = S.ax.P[k];
-      if (valid && m >= 0) out[(long)m * a.pitch] = make_float2(P * v0[r].x, P * v0[r].y);
-    }
-  });
+  while (w < items) {
+    const int col = (w % ctiles) * T + p;
+    const bool valid = col < a.ncol;
+    float2* out = a.out + (long)(w / ctiles) * M * a.pitch + col;
+    const int wn = next(w + gridDim.x);
+    float2 v0[B], v1[B];
+    cp_wait<0>();
+    __syncthreads();
+    tile_points<N, T>(v0, S.tile[s], t, p);
+    tile_points<N, T>(v1, S.tile[s ^ 1], t, p);
+    __syncthreads();
+    fetch(s, w, 2);
+    fetch(s ^ 1, wn, 0);
+    pf.fwd(v0);
+    pf.fwd(v1);
+    sfor<0, B>([&](auto rc) {
+      constexpr int r = decltype(rc)::value;
+      if constexpr (spec_keeps<N>(r)) {
+        const int k = pf.kidx(r);
+        const int m = spec_col<N>(k);
+        const float P = S.ax.P[k], d = S.ax.d[k];
+        if (valid && m >= 0)
+          out[(long)m * a.pitch] = make_float2(fmaf(P, v0[r].x, -d * v1[r].y), fmaf(P, v0[r].y, d * v1[r].x));
+      }
+    });
+    cp_wait<1>();
+    __syncthreads();
+    tile_points<N, T>(v0, S.tile[s], t, p);
+    __syncthreads();
+    fetch(s, wn, 1);
+    pf.fwd(v0);
+    out += a.os;
+    sfor<0, B>([&](auto rc) {
+      constexpr int r = decltype(rc)::value;
+      if constexpr (spec_keeps<N>(r)) {
+        const int k = pf.kidx(r);
+        const int m = spec_col<N>(k);
+        const float P = S.ax.P[k];
+        if (valid && m >= 0) out[(long)m * a.pitch] = make_float2(P * v0[r].x, P * v0[r].y);
+      }
+    });
+    w = wn;
+    s ^= 1;
+  }
+  cp_wait<0>();
 }
 
 // Last axis: k = -(P a + D b), RK bookkeeping in spectral space, increment
@@ -473,20 +528,19 @@ __global__ void __launch_bounds__(Shape<N>::A * T, spec_min_blocks<N, T>()) k_sp
 // stages so far; stages 0..2 return wnext k, stage 3 returns the whole
 // increment of the step (rk_update_incr's weights).
 struct SpecCArgs {
-  const float2* a;   // P operand; [outer][N][..] with the strides below
+  const float2* a;   // P operand; [solve][outer][N][..] with the strides below
   const float2* b;   // D operand
   float2* out;       // increment; may alias a
   float2* acc;       // accumulator [solve][M][outer][..] (strides acc_as, acc_os)
   long as, os, ss;   // axis, outer and solve strides (complex elements)
   long acc_as, acc_os, acc_ss;
-  int ncol, nouter;
+  int ncol, nouter, nsolve;
   AxisOps ax;
   int stage;         // 0..3
   int rk2;
   const double* dt_dev;
   double dt;
   const int* active;
-  int sol0;
 };
 
 template <int N, int T>
@@ -494,63 +548,96 @@ __global__ void __launch_bounds__(Shape<N>::A * T, spec_min_blocks<N, T>()) k_sp
   constexpr int A = Shape<N>::A, B = Shape<N>::B;
   using PF = Pencil<N, T, true>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  auto& S = *reinterpret_cast<SpecSmem<N, T>*>(smem_raw);
+  auto& S = *reinterpret_cast<SpecPairSmem<N, T>*>(smem_raw);
   const int p = threadIdx.x % T, t = threadIdx.x / T;
-  const int col = blockIdx.x * T + p;
-  const int sol = a.sol0 + blockIdx.y / a.nouter;
-  const int outer = blockIdx.y % a.nouter;
-  if (a.active != nullptr && a.active[sol] == 0) return;
-  const bool valid = col < a.ncol;
   PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
-  const long base = (long)sol * a.ss + (long)outer * a.os + (long)t * a.as + col;
-  const long step = (long)A * a.as;
-  float2 w[B], z2[B];
-#pragma unroll
-  for (int n2 = 0; n2 < B; ++n2) w[n2] = valid ? a.a[base + n2 * step] : make_float2(0.0f, 0.0f);
-#pragma unroll
-  for (int n2 = 0; n2 < B; ++n2) z2[n2] = valid ? a.b[base + n2 * step] : make_float2(0.0f, 0.0f);
+  const int ctiles = (a.ncol + T - 1) / T;
+  const int items = ctiles * a.nouter * a.nsolve;
+  auto next = [&](int w) {
+    if (a.active != nullptr)
+      while (w < items && a.active[w / ctiles / a.nouter] == 0) w += gridDim.x;
+    return w;
+  };
+  auto base_of = [&](int w) {
+    const int o = w / ctiles;
+    return (long)(o / a.nouter) * a.ss + (long)(o % a.nouter) * a.os;
+  };
+  auto fetch = [&](int w) {
+    if (w < items) {
+      const long b = base_of(w);
+      tile_copy<N, T, A * T>(S.tile[0], a.a + b, a.as, (w % ctiles) * T, a.ncol);
+      tile_copy<N, T, A * T>(S.tile[1], a.b + b, a.as, (w % ctiles) * T, a.ncol);
+    }
+    cp_commit();
+  };
+  int w = next(blockIdx.x);
+  fetch(w);
   load_axis<N>(S.ax, a.ax);
-  const float dt = (a.dt_dev != nullptr) ? (float)a.dt_dev[sol] : (float)a.dt;
-  const RKCoef rk = rk_coef(a.stage, dt, a.rk2);
-  __syncthreads();
-  pf.fwd(w);
-  pf.fwd(z2);
-  float2* acc = a.acc + (long)sol * a.acc_ss + (long)outer * a.acc_os + col;
-  sfor<0, B>([&](auto rc) {
-    constexpr int r = decltype(rc)::value;
-    float2 inc = make_float2(0.0f, 0.0f);
-    if constexpr (spec_keeps<N>(r)) {
-      const int k = pf.kidx(r);
-      const int m = spec_col<N>(k);
-      if (m >= 0) {
-        const float P = -S.ax.P[k], d = -S.ax.d[k];
-        const float2 kk = make_float2(fmaf(P, w[r].x, -d * z2[r].y), fmaf(P, w[r].y, d * z2[r].x));
-        if (a.stage == 3) {
-          const float2 s = valid ? acc[m * a.acc_as] : make_float2(0.0f, 0.0f);
-          inc = make_float2(fmaf(rk.wacc, kk.x, s.x), fmaf(rk.wacc, kk.y, s.y));
-        } else {
-          float2 s = make_float2(0.0f, 0.0f);
-          if (a.stage != 0 && valid) s = acc[m * a.acc_as];
-          if (valid) acc[m * a.acc_as] = make_float2(fmaf(rk.wacc, kk.x, s.x), fmaf(rk.wacc, kk.y, s.y));
-          inc = make_float2(rk.wnext * kk.x, rk.wnext * kk.y);
+  while (w < items) {
+    const int col = (w % ctiles) * T + p;
+    const int outer = w / ctiles % a.nouter, sol = w / ctiles / a.nouter;
+    const bool valid = col < a.ncol;
+    const int wn = next(w + gridDim.x);
+    const float dt = (a.dt_dev != nullptr) ? (float)a.dt_dev[sol] : (float)a.dt;
+    const RKCoef rk = rk_coef(a.stage, dt, a.rk2);
+    float2* acc = a.acc + (long)sol * a.acc_ss + (long)outer * a.acc_os + col;
+    float2 v[B], z2[B];
+    cp_wait<0>();
+    __syncthreads();
+    tile_points<N, T>(v, S.tile[0], t, p);
+    tile_points<N, T>(z2, S.tile[1], t, p);
+    __syncthreads();
+    fetch(wn);
+    if (a.stage != 0 && valid) {  // the accumulator's lines, needed after the transforms
+      sfor<0, B>([&](auto rc) {
+        constexpr int r = decltype(rc)::value;
+        if constexpr (spec_keeps<N>(r)) {
+          const int m = spec_col<N>(pf.kidx(r));
+          if (m >= 0 && p % 16 == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(acc + m * a.acc_as));
+        }
+      });
+    }
+    pf.fwd(v);
+    pf.fwd(z2);
+    sfor<0, B>([&](auto rc) {
+      constexpr int r = decltype(rc)::value;
+      float2 inc = make_float2(0.0f, 0.0f);
+      if constexpr (spec_keeps<N>(r)) {
+        const int k = pf.kidx(r);
+        const int m = spec_col<N>(k);
+        if (m >= 0) {
+          const float P = -S.ax.P[k], d = -S.ax.d[k];
+          const float2 kk = make_float2(fmaf(P, v[r].x, -d * z2[r].y), fmaf(P, v[r].y, d * z2[r].x));
+          if (a.stage == 3) {
+            const float2 q = valid ? acc[m * a.acc_as] : make_float2(0.0f, 0.0f);
+            inc = make_float2(fmaf(rk.wacc, kk.x, q.x), fmaf(rk.wacc, kk.y, q.y));
+          } else {
+            float2 q = make_float2(0.0f, 0.0f);
+            if (a.stage != 0 && valid) q = acc[m * a.acc_as];
+            if (valid) acc[m * a.acc_as] = make_float2(fmaf(rk.wacc, kk.x, q.x), fmaf(rk.wacc, kk.y, q.y));
+            inc = make_float2(rk.wnext * kk.x, rk.wnext * kk.y);
+          }
         }
       }
-    }
-    w[r] = inc;
-  });
-  pf.inv(w);
-  if (valid) {
+      v[r] = inc;
+    });
+    pf.inv(v);
+    if (valid) {
+      float2* out = a.out + base_of(w) + (long)t * a.as + col;
 #pragma unroll
-    for (int n2 = 0; n2 < B; ++n2) a.out[base + n2 * step] = w[n2];
+      for (int n2 = 0; n2 < B; ++n2) out[(long)(A * n2) * a.as] = v[n2];
+    }
+    w = wn;
   }
+  cp_wait<0>();
 }
 
 // 3D: inverse y transform of the increment, [plane][M][pitch] -> wide rows.
 struct SpecIArgs {
   const float2* in;
-  float2* D;         // planes from plane0: [plane][N][pitch]
+  float2* D;          // [plane][N][pitch]
   int pitch, ncol;
-  int plane0, pps;
+  int planes, pps;
   AxisOps ax;
   const int* active;
 };
@@ -560,37 +647,54 @@ __global__ void __launch_bounds__(Shape<N>::A * T, spec_min_blocks<N, T>()) k_sp
   constexpr int A = Shape<N>::A, B = Shape<N>::B, M = spec_modes(N);
   using PF = Pencil<N, T, true>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  auto& S = *reinterpret_cast<SpecSmem<N, T>*>(smem_raw);
+  auto& S = *reinterpret_cast<SpecISmem<N, T>*>(smem_raw);
   const int p = threadIdx.x % T, t = threadIdx.x / T;
-  const int col = blockIdx.x * T + p;
-  const int plane = a.plane0 + blockIdx.y;
-  if (a.active != nullptr && a.active[plane / a.pps] == 0) return;
-  const bool valid = col < a.ncol;
   PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
-  const float2* in = a.in + (long)plane * M * a.pitch + col;
-  float2 v[B];
-  sfor<0, B>([&](auto rc) {
-    constexpr int r = decltype(rc)::value;
-    v[r] = make_float2(0.0f, 0.0f);
-    if constexpr (spec_keeps<N>(r)) {
-      const int m = spec_col<N>(pf.kidx(r));
-      if (valid && m >= 0) v[r] = in[(long)m * a.pitch];
-    }
-  });
+  const int ctiles = (a.ncol + T - 1) / T;
+  const int items = ctiles * a.planes;
+  auto next = [&](int w) {
+    if (a.active != nullptr)
+      while (w < items && a.active[w / ctiles / a.pps] == 0) w += gridDim.x;
+    return w;
+  };
+  auto fetch = [&](int w) {
+    if (w < items)
+      tile_copy<M, T, A * T>(S.tile[0], a.in + (long)(w / ctiles) * M * a.pitch, a.pitch, (w % ctiles) * T, a.ncol);
+    cp_commit();
+  };
+  int w = next(blockIdx.x);
+  fetch(w);
   load_axis<N>(S.ax, a.ax);
-  __syncthreads();
-  pf.inv(v);
-  if (valid) {
-    float2* out = a.D + ((long)blockIdx.y * N + t) * a.pitch + col;
-    const long step = (long)A * a.pitch;
+  while (w < items) {
+    const int col = (w % ctiles) * T + p;
+    const int wn = next(w + gridDim.x);
+    float2 v[B];
+    cp_wait<0>();
+    __syncthreads();
+    sfor<0, B>([&](auto rc) {
+      constexpr int r = decltype(rc)::value;
+      v[r] = make_float2(0.0f, 0.0f);
+      if constexpr (spec_keeps<N>(r)) {
+        const int m = spec_col<N>(pf.kidx(r));
+        if (m >= 0) v[r] = S.tile[0][m * T + p];
+      }
+    });
+    __syncthreads();
+    fetch(wn);
+    pf.inv(v);
+    if (col < a.ncol) {
+      float2* out = a.D + ((long)(w / ctiles) * N + t) * a.pitch + col;
 #pragma unroll
-    for (int n2 = 0; n2 < B; ++n2) out[n2 * step] = v[n2];
+      for (int n2 = 0; n2 < B; ++n2) out[(long)(A * n2) * a.pitch] = v[n2];
+    }
+    w = wn;
   }
+  cp_wait<0>();
 }
 
 template <int N, int PHYS> cudaError_t launch_spec_x(int nd, bool inc, bool flux, const SpecXArgs& a, cudaStream_t s);
-template <int N> cudaError_t launch_spec_f(const SpecFArgs& a, int planes, cudaStream_t s);
-template <int N> cudaError_t launch_spec_c(const SpecCArgs& a, int nsol, cudaStream_t s);
-template <int N> cudaError_t launch_spec_i(const SpecIArgs& a, int planes, cudaStream_t s);
+template <int N> cudaError_t launch_spec_f(const SpecFArgs& a, cudaStream_t s);
+template <int N> cudaError_t launch_spec_c(const SpecCArgs& a, cudaStream_t s);
+template <int N> cudaError_t launch_spec_i(const SpecIArgs& a, cudaStream_t s);
 
 }  // namespace ps
