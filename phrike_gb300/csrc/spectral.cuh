@@ -317,29 +317,31 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_spec_x(SpecXArgs a) {
     }
     const float href = a.gamma * er;
     const float ig1 = 1.0f / g1;
-    // F^dir_c at point n2
-    auto fx = [&](auto dirc, auto cc, int n2) -> float {
-      constexpr int dir = decltype(dirc)::value, c = decltype(cc)::value;
-      if constexpr (PHYS == 1) {
-        const float b2 = q[5][n2] * q[5][n2] + q[6][n2] * q[6][n2] + q[7][n2] * q[7][n2];
-        const float v2 = q[1][n2] * q[1][n2] + q[2][n2] * q[2][n2] + q[3][n2] * q[3][n2];
-        const float ps = g1 * (q[4][n2] - 0.5f * q[0][n2] * v2 - 0.5f * b2) + 0.5f * b2;
-        const float ub = q[1][n2] * q[5][n2] + q[2][n2] * q[6][n2] + q[3][n2] * q[7][n2];
-        return mhd3_flux<dir, c>(q[0][n2], q[1][n2], q[2][n2], q[3][n2], ps, q[4][n2] + ps, ub, q[5][n2], q[6][n2],
-                                 q[7][n2]);
-      } else {
-        const float rho = q[0][n2], ua = q[1 + dir][n2], pr = q[NC - 1][n2];
-        if constexpr (c == 0) return rho * ua;
-        if constexpr (c == NC - 1) {
+    // Euler flux pair j = (F_2j, F_2j+1) along the (runtime) direction dir.
+    // The direction enters by selects, so one body per pair serves the ND
+    // directions (a third of the code: TGV 256^3 x pass 325 -> 321 us, KHI
+    // 512^2 x 16 92 -> 89; the longer MHD bodies ran slower that way, 131 ->
+    // 139 us at 128^3, and take the direction at compile time).
+    auto flux_pair = [&](auto jc, int dir, int n2) -> float2 {
+      constexpr int c = 2 * decltype(jc)::value;
+      const float un = (dir == 0) ? q[1][n2] : (ND == 2 || dir == 1) ? q[2][n2] : q[(ND == 3) ? 3 : 2][n2];
+      const float mn = q[0][n2] * un;
+      auto comp = [&](auto cc) -> float {
+        constexpr int C = decltype(cc)::value;
+        const float pr = q[NC - 1][n2];
+        if constexpr (C == 0) return mn;
+        if constexpr (C == NC - 1) {
           float kin = 0.0f;
 #pragma unroll
           for (int d = 0; d < ND; ++d) kin = fmaf(q[1 + d][n2], q[1 + d][n2], kin);
-          const float Ep = fmaf(pr, ig1, 0.5f * rho * kin);  // E' = E - E_ref
-          return ((Ep + pr) + href) * ua;                    // (E + p) u_dir
+          const float Ep = fmaf(pr, ig1, 0.5f * q[0][n2] * kin);  // E' = E - E_ref
+          return ((Ep + pr) + href) * un;                         // (E + p) u_dir
         }
-        const float rv = rho * ua * q[c][n2];
-        return (c - 1 == dir) ? rv + pr : rv;
-      }
+        return mn * q[C][n2] + ((C - 1 == dir) ? pr : 0.0f);
+      };
+      float2 f = make_float2(comp(std::integral_constant<int, c>{}), 0.0f);
+      if constexpr (c + 1 < NC) f.y = comp(std::integral_constant<int, c + 1>{});
+      return f;
     };
 #pragma unroll 1
     for (int job = 0; job < ND * NJ; ++job) {
@@ -350,20 +352,33 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_spec_x(SpecXArgs a) {
       for (int c = 0; c < NC; ++c)
 #pragma unroll
         for (int n2 = 0; n2 < B; ++n2) asm volatile("" : "+f"(q[c][n2]));
-      float2 v[B];
-      sfor<0, ND * NJ>([&](auto jc) {
-        constexpr int J = decltype(jc)::value;
-        constexpr int dir = J / NJ, c = 2 * (J % NJ);
-        constexpr int c1 = (c + 1 < NC) ? c + 1 : c;
-        if (job == J) {
-#pragma unroll
-          for (int n2 = 0; n2 < B; ++n2) {
-            v[n2].x = fx(std::integral_constant<int, dir>{}, std::integral_constant<int, c>{}, n2);
-            v[n2].y = (c + 1 < NC) ? fx(std::integral_constant<int, dir>{}, std::integral_constant<int, c1>{}, n2) : 0.0f;
-          }
-        }
-      });
       const int dir = job / NJ, j = job % NJ;
+      float2 v[B];
+      if constexpr (PHYS == 1) {
+        sfor<0, ND * NJ>([&](auto jobc) {
+          constexpr int J = decltype(jobc)::value;
+          constexpr int DIR = J / NJ, c = 2 * (J % NJ);
+          if (job == J) {
+#pragma unroll
+            for (int n2 = 0; n2 < B; ++n2) {
+              const float b2 = q[5][n2] * q[5][n2] + q[6][n2] * q[6][n2] + q[7][n2] * q[7][n2];
+              const float v2 = q[1][n2] * q[1][n2] + q[2][n2] * q[2][n2] + q[3][n2] * q[3][n2];
+              const float ps = g1 * (q[4][n2] - 0.5f * q[0][n2] * v2 - 0.5f * b2) + 0.5f * b2;
+              const float ub = q[1][n2] * q[5][n2] + q[2][n2] * q[6][n2] + q[3][n2] * q[7][n2];
+              auto f = [&](auto cc) {
+                return mhd3_flux<DIR, decltype(cc)::value>(q[0][n2], q[1][n2], q[2][n2], q[3][n2], ps, q[4][n2] + ps,
+                                                           ub, q[5][n2], q[6][n2], q[7][n2]);
+              };
+              v[n2] = make_float2(f(std::integral_constant<int, c>{}), f(std::integral_constant<int, c + 1>{}));
+            }
+          }
+        });
+      } else {
+        put(j, [&](auto jc) {
+#pragma unroll
+          for (int n2 = 0; n2 < B; ++n2) v[n2] = flux_pair(jc, dir, n2);
+        });
+      }
       const bool single = ODD && j == NP;
       pf.fwd(v);
       float2* g = a.G + dir * a.gs + (long)row * a.pitch + j * M;
