@@ -7,6 +7,7 @@
 #include <unordered_set>
 
 #include "euler1d.cuh"
+#include "line1d.cuh"
 #include "mhd1d.cuh"
 #include "euler_passes.cuh"
 #include "passes_tma.cuh"
@@ -16,6 +17,8 @@ namespace ps {
 template <int N> cudaError_t launch_xfirst(int nd, const XFirstArgs& a, cudaStream_t s);
 template <int N> cudaError_t launch_op(bool strided, const OpArgs& a, cudaStream_t s);
 template <int N> cudaError_t launch_step1d(const Step1DArgs& a, int nsolve, cudaStream_t s);
+// whole steps without artificial viscosity; tw: W_N^k, natural order
+template <int N> cudaError_t launch_line1d(const Step1DArgs& a, const float2* tw, int nsolve, cudaStream_t s);
 template <int N> cudaError_t launch_ark1d(const Ark1DArgs& a, int nsolve, cudaStream_t s);
 template <int N> cudaError_t launch_mhd1d(const Mhd1DArgs& a, int nsolve, cudaStream_t s);
 
@@ -253,6 +256,14 @@ cudaError_t dispatch_proj_cols(long units, F&& f) {
     return cudaGetLastError();                                                                        \
   }                                                                                                   \
   template <>                                                                                         \
+  cudaError_t launch_line1d<NN>(const Step1DArgs& a, const float2* tw, int nsolve, cudaStream_t s) {  \
+    const size_t sm = sizeof(LineSmem<NN>);                                                           \
+    cudaError_t e;                                                                                    \
+    if ((e = set_smem(k_line1d<NN>, sm)) != cudaSuccess) return e;                                    \
+    k_line1d<NN><<<nsolve, Line<NN>::BLOCK, sm, s>>>(a, tw);                                          \
+    return cudaGetLastError();                                                                        \
+  }                                                                                                   \
+  template <>                                                                                         \
   cudaError_t launch_ark1d<NN>(const Ark1DArgs& a, int nsolve, cudaStream_t s) {                      \
     const size_t sm = sizeof(Step1DSmem<NN>);                                                         \
     cudaError_t e;                                                                                    \
@@ -357,6 +368,14 @@ cudaError_t dispatch_proj_cols(long units, F&& f) {
     cudaError_t e;                                                                                    \
     if ((e = set_smem(k_step1d<NN>, sm)) != cudaSuccess) return e;                                    \
     k_step1d<NN><<<nsolve, Shape<NN>::A, sm, s>>>(a);                                                 \
+    return cudaGetLastError();                                                                        \
+  }                                                                                                   \
+  template <>                                                                                         \
+  cudaError_t launch_line1d<NN>(const Step1DArgs& a, const float2* tw, int nsolve, cudaStream_t s) {  \
+    const size_t sm = sizeof(LineSmem<NN>);                                                           \
+    cudaError_t e;                                                                                    \
+    if ((e = set_smem(k_line1d<NN>, sm)) != cudaSuccess) return e;                                    \
+    k_line1d<NN><<<nsolve, Line<NN>::BLOCK, sm, s>>>(a, tw);                                          \
     return cudaGetLastError();                                                                        \
   }                                                                                                   \
   template <>                                                                                         \

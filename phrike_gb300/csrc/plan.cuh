@@ -25,6 +25,7 @@ struct ps_plan_s {
   float* d[3] = {nullptr, nullptr, nullptr};
   float2* twf[3] = {nullptr, nullptr, nullptr};
   float2* twi[3] = {nullptr, nullptr, nullptr};
+  float2* tw1d = nullptr;  // 1D Euler: W_N^k in natural order (line1d.cuh)
   // scratch, [nsolve][nfields][cells] each
   float* G = nullptr;    // x-pass outputs (2D: 8 fields, 3D: 15)
   float* AB = nullptr;   // 3D y-pass outputs (10 fields)
