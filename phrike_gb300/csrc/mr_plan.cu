@@ -95,12 +95,49 @@ int mr_setup(ps_plan p) {
     ax.tw = p->twf[a];
     ax.P = p->P[a];
     ax.d = p->d[a];
+    SpecAxis& sx = p->sax[a];
+    int sr[16];
+    if (!spec_factor(N, sr, &sx.nst)) return errorf(PS_ERR_UNSUPPORTED, "axis %d: N=%d is not 5-smooth", a, N);
+    spec_layout(sr, sx.nst, &sx.len, sx.st);
+    sx.n = N;
+    sx.km = spec_km(N);
+    for (int s = 0, m = N; s < sx.nst; ++s) {
+      m /= sr[s];
+      sx.radix[s] = sr[s];
+      sx.m[s] = m;
+      sx.inv_m[s] = 1.0f / (float)m;
+      sx.inv_r[s] = 1.0f / (float)sr[s];
+    }
+    std::vector<float2> st(N);
+    spec_twiddles(N, sr, sx.nst, st.data());
+    float2* dst = nullptr;
+    if ((rc = plan_alloc(p, &dst, N)) != PS_OK) return rc;
+    MR_CU(cudaMemcpy(dst, st.data(), N * sizeof(float2), cudaMemcpyHostToDevice), "table upload");
+    sx.tw = dst;
+    sx.P = p->P[a];
+    sx.d = p->d[a];
   }
   return PS_OK;
 }
 
 int mr_apply_op(ps_plan p, int axis, const float* in, float* out, int nf, int deriv, float scale, bool complement,
-                const int* active, long ss_in, cudaStream_t s) {
+                const int* active, long ss_in, bool add_eref, cudaStream_t s) {
+  if (complement && deriv == 0) {
+    MrFilterArgs f{};
+    f.in = in;
+    f.out = out;
+    f.nf = nf;
+    f.fs = p->cells;
+    f.ss_out = p->ss(nf);
+    f.ss_in = (ss_in != 0) ? ss_in : f.ss_out;
+    f.es = 1;
+    for (int a = 0; a < axis; ++a) f.es *= p->n[a];
+    f.npen = p->cells / p->n[axis];
+    f.active = active;
+    f.eadd = add_eref ? p->eref : nullptr;
+    MR_CU(launch_mrs_filter(f, p->sax[axis], p->nsolve, s), "filter pass");
+    return PS_OK;
+  }
   MrOpArgs a{};
   a.in = in;
   a.out = out;
@@ -244,9 +281,9 @@ int mr_steps_1d(ps_plan p, float* U, int nsteps, double dt, const double* d_dt, 
       MR_CU(launch_mr_line(a, p->nsolve, s), "1D stage");
     }
     // filter inside the RK step, then again at the cadence
-    if ((rc = mr_apply_op(p, 0, U, U, 3, 0, 1.0f, true, act, 0, s)) != PS_OK) return rc;
+    if ((rc = mr_apply_op(p, 0, U, U, 3, 0, 1.0f, true, act, 0, false, s)) != PS_OK) return rc;
     if ((p->step_counter % p->desc.filter_interval) == 0 &&
-        (rc = mr_apply_op(p, 0, U, U, 3, 0, 1.0f, true, act, 0, s)) != PS_OK)
+        (rc = mr_apply_op(p, 0, U, U, 3, 0, 1.0f, true, act, 0, false, s)) != PS_OK)
       return rc;
     if (cfl) MR_CU(launch_step_advance(d_t, p->dt, p->speed, p->active, p->steps_done, p->nsolve, s), "advance");
     p->step_counter += 1;

@@ -11,6 +11,7 @@
 
 #include "../../include/phrike_gb300.h"
 #include "mixed_radix.cuh"
+#include "mr_spec.cuh"
 #include "pass_common.cuh"
 
 struct ps_plan_s {
@@ -105,6 +106,9 @@ struct ps_plan_s {
   // Fourier axes of any 5-smooth length (mixed-radix passes, mr_plan.cu)
   bool mr = false;
   ps::MrAxis mrax[3] = {};
+  ps::SpecAxis sax[3] = {};                              // their in-place passes (mr_spec.cu)
+  float2* p2_twf[3] = {nullptr, nullptr, nullptr};       // pencil twiddles of the power-of-two axes of such a grid
+  float2* p2_twi[3] = {nullptr, nullptr, nullptr};
   // point evaluation: 0 auto, 1 exact interpolant, 2 NUFFT (nufft.cu, tables made on first use)
   int tracer_method = 0;
   bool nu_ready = false;
@@ -115,6 +119,9 @@ struct ps_plan_s {
   float2* nu_t2 = nullptr;  // x and y resampled (3D)
 
   ps::AxisOps ax(int a) const { return ps::AxisOps{P[a], d[a], twf[a], twi[a]}; }
+  // axis `a` of the truncated-spectra passes on the register pencils, and its tables
+  bool spec_p2(int a) const { return !mr || p2_twf[a] != nullptr; }
+  ps::AxisOps spec_ax(int a) const { return mr ? ps::AxisOps{P[a], d[a], p2_twf[a], p2_twi[a]} : ax(a); }
   long ss(int nf) const { return (long)nf * cells; }  // solve stride of an nf-field buffer
   int rows() const { return (int)(cells / n[0]); }     // x-pencil rows of one solve
   // parabolic CFL cap of explicit MHD diffusion: cfl_diff / (max(eta, nu)
@@ -209,7 +216,7 @@ int lgl_filter(ps_plan p, const float* f, float* out, int nf, cudaStream_t s);
 bool mr_axis_ok(int n);
 int mr_setup(ps_plan p);
 int mr_apply_op(ps_plan p, int axis, const float* in, float* out, int nf, int deriv, float scale, bool complement,
-                const int* active, long ss_in, cudaStream_t s);
+                const int* active, long ss_in, bool add_eref, cudaStream_t s);
 int mr_xfirst(ps_plan p, const float* U, float* Uw, float* speed, bool shift_in, const int* active, cudaStream_t s);
 int mr_ymid(ps_plan p, const int* active, cudaStream_t s);
 int mr_last(ps_plan p, int stage, const float* Un, float* out, double dt, const double* d_dt, bool filter_last,

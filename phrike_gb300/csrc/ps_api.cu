@@ -89,6 +89,8 @@ bool pow2_axes(const ps_plan_desc* d) {
 // a Fourier grid with some other axis length: the mixed-radix passes
 bool is_mr(const ps_plan_desc* d) { return !is_lgl(d) && !pow2_axes(d); }
 
+bool spec_plan(const ps_plan_desc* d);  // steps run on the truncated-spectra passes
+
 // 1D Euler on power-of-two grids without artificial viscosity runs k_line1d
 // (line1d.cuh) from 16 points (per step, before -> now: 16 points 4.7 -> 4.2
 // us, 256 37 -> 5.4, 1024 71 -> 10.3, 4096 214 -> 72); at 8 points its fused
@@ -334,11 +336,11 @@ ps::StridedGeom geom_z(const ps_plan_s* p) {
 // One-axis operator (deriv: 0 P, 1 D, 2 Laplacian factor L, 3 raw second derivative)
 // on nf fields.  ss_in (axis 0 only): solve stride of `in` when it is a field
 // subset of a wider state (0: the nf-field stride of `out`).  add_eref (axis
-// 0, power-of-two plans): the last field leaves the energy-perturbation form.
+// 0): the last field leaves the energy-perturbation form.
 int apply_op(ps_plan p, int axis, const float* in, float* out, int nf, int deriv, float scale, cudaStream_t s,
              bool complement = false, const int* active = nullptr, long ss_in = 0, bool add_eref = false) {
   ProfScope prof(p, s, PS_KIND_OP, 8.0 * nf * p->cells * p->nsolve);
-  if (p->mr) return ps::mr_apply_op(p, axis, in, out, nf, deriv, scale, complement, active, ss_in, s);
+  if (p->mr) return ps::mr_apply_op(p, axis, in, out, nf, deriv, scale, complement, active, ss_in, add_eref, s);
   cudaError_t e;
   const float kunit = (float)(2.0 * M_PI / p->desc.length[axis]);
   if (axis != 0 && ss_in != 0) return fail(PS_ERR_INVALID, "field-subset input is supported along x only");
@@ -1008,9 +1010,22 @@ int steps_mhd(ps_plan p, float* U, int nsteps, double dt, const double* d_dt, do
 // adaptive stepping, run the real-space passes.
 // ---------------------------------------------------------------------------
 bool spec_plan(const ps_plan_desc* d) {
-  if (d->ndim < 2 || is_lgl(d) || is_mr(d) || !d->dealias || d->av_mode != PS_AV_OFF) return false;
+  if (d->ndim < 2 || is_lgl(d) || !d->dealias || d->av_mode != PS_AV_OFF) return false;
+  const int nd = d->ndim;
+  if (is_mr(d)) {
+    if (!ps::supported_n(d->n[0]) && !ps::mrs_x_fits(nd, d->n[0])) return false;
+    // the wide rows of very short x axes pad past the scratch (spec_bufs)
+    const long cells = (long)d->n[0] * d->n[1] * (nd == 3 ? d->n[2] : 1);
+    const int nc = nd + 2;
+    const long rows = cells / d->n[0];
+    const long wide = 2L * rows * ps::spec_pitch(d->n[0], nc);
+    const long part = wide / d->n[1] * ps::spec_modes(d->n[1]);
+    if (nd * wide > (nd == 3 ? 15 : 8) * cells) return false;
+    if (nd == 3 && (2 * part > 10 * cells || part / d->n[2] * ps::spec_modes(d->n[2]) > 5 * cells)) return false;
+    if (nd == 2 && part > 4 * cells) return false;
+  }
   if (d->equations == PS_EQ_MHD) return d->mhd_resistivity == 0.0 && d->mhd_viscosity == 0.0;
-  for (int a = 0; a < d->ndim; ++a)
+  for (int a = 0; a < nd; ++a)
     if (d->gravity[a] != 0.0) return false;
   return true;
 }
@@ -1070,7 +1085,7 @@ int spec_rows(ps_plan p, const SpecBufs& b, bool inc, bool flux, const float* U,
   a.ssU = p->ss(p->nc);
   a.rps = p->rows();
   a.rows = a.rps * p->nsolve;
-  a.ax = p->ax(0);
+  a.ax = p->spec_ax(0);
   a.gamma = (float)p->desc.gamma;
   a.rho_min = p->mhd ? (float)p->desc.mhd_rho_min : 1e-8f;  // clamp floors (solver.py:467, 876-877)
   a.p_min = p->mhd ? (float)p->desc.mhd_p_min : 1e-10f;
@@ -1088,7 +1103,7 @@ int spec_rows(ps_plan p, const SpecBufs& b, bool inc, bool flux, const float* U,
   f.pitch = b.pitch;
   f.ncol = b.ncol;
   f.pps = p->n[2];
-  f.ax = p->ax(1);
+  f.ax = p->spec_ax(1);
   f.active = act;
   ps::SpecIArgs i{};
   i.in = b.A;
@@ -1096,7 +1111,7 @@ int spec_rows(ps_plan p, const SpecBufs& b, bool inc, bool flux, const float* U,
   i.pitch = b.pitch;
   i.ncol = b.ncol;
   i.pps = p->n[2];
-  i.ax = p->ax(1);
+  i.ax = p->spec_ax(1);
   i.active = act;
   f.planes = i.planes = p->n[2] * p->nsolve;
   const double wide = 8.0 * b.ncol * a.rows;
@@ -1104,13 +1119,14 @@ int spec_rows(ps_plan p, const SpecBufs& b, bool inc, bool flux, const float* U,
   cudaError_t e;
   if (inc && p->nd == 3) {
     ProfScope prof(p, s, PS_KIND_Y, part + wide);
-    e = ps::dispatch_n(p->n[1], [&](auto nn) { return ps::launch_spec_i<decltype(nn)::value>(i, s); });
+    e = !p->spec_p2(1) ? ps::launch_mrs_i(i, p->sax[1], s)
+                       : ps::dispatch_n(p->n[1], [&](auto nn) { return ps::launch_spec_i<decltype(nn)::value>(i, s); });
     if (e != cudaSuccess) return cuda_fail(e, "y inverse pass");
   }
   {
     ProfScope prof(p, s, PS_KIND_X, wide * ((inc ? 1 : 0) + (flux ? p->nd : 0)) +
                                         4.0 * p->cells * p->nsolve * p->nc * (1 + (Uw ? 1 : 0)));
-    e = ps::dispatch_n(p->n[0], [&](auto nn) {
+    e = !p->spec_p2(0) ? ps::launch_mrs_x(p->nd, inc, flux, a, p->sax[0], s) : ps::dispatch_n(p->n[0], [&](auto nn) {
       constexpr int N = decltype(nn)::value;
       return p->mhd ? ps::launch_spec_x<N, 1>(p->nd, inc, flux, a, s) : ps::launch_spec_x<N, 0>(p->nd, inc, flux, a, s);
     });
@@ -1118,7 +1134,8 @@ int spec_rows(ps_plan p, const SpecBufs& b, bool inc, bool flux, const float* U,
   }
   if (flux && p->nd == 3) {
     ProfScope prof(p, s, PS_KIND_Y, 3.0 * wide + 2.0 * part);
-    e = ps::dispatch_n(p->n[1], [&](auto nn) { return ps::launch_spec_f<decltype(nn)::value>(f, s); });
+    e = !p->spec_p2(1) ? ps::launch_mrs_f(f, p->sax[1], s)
+                       : ps::dispatch_n(p->n[1], [&](auto nn) { return ps::launch_spec_f<decltype(nn)::value>(f, s); });
     if (e != cudaSuccess) return cuda_fail(e, "y pass");
   }
   return PS_OK;
@@ -1148,7 +1165,7 @@ int spec_last(ps_plan p, const SpecBufs& b, int stage, double dt, const double* 
   c.acc_as = (long)c.nouter * b.pitch;
   c.acc_os = c.os;
   c.acc_ss = (long)ps::spec_modes(p->n[ax]) * c.nouter * b.pitch;
-  c.ax = p->ax(ax);
+  c.ax = p->spec_ax(ax);
   c.stage = stage;
   c.rk2 = (p->desc.scheme == PS_SCHEME_RK2) ? 1 : 0;
   c.dt_dev = d_dt;
@@ -1157,8 +1174,9 @@ int spec_last(ps_plan p, const SpecBufs& b, int stage, double dt, const double* 
   const double in = 8.0 * b.ncol * p->n[ax] * c.nouter * p->nsolve;
   const double ac = in * ps::spec_modes(p->n[ax]) / p->n[ax];
   ProfScope prof(p, s, PS_KIND_LAST, 3.0 * in + ac * (stage == 0 || stage == 3 ? 1 : 2));
-  cudaError_t e =
-      ps::dispatch_n(p->n[ax], [&](auto nn) { return ps::launch_spec_c<decltype(nn)::value>(c, s); });
+  cudaError_t e = !p->spec_p2(ax)
+                      ? ps::launch_mrs_c(c, p->sax[ax], s)
+                      : ps::dispatch_n(p->n[ax], [&](auto nn) { return ps::launch_spec_c<decltype(nn)::value>(c, s); });
   if (e != cudaSuccess) return cuda_fail(e, "last pass");
   return PS_OK;
 }
@@ -1238,10 +1256,10 @@ int steps_spec(ps_plan p, float* U, int nsteps, double dt, const double* d_dt, d
     if (filt) {
       for (int ax = p->nd - 1; ax >= 1; --ax)
         if ((rc = apply_op(p, ax, U, U, p->nc, 0, 1.0f, s, true, act)) != PS_OK) return rc;
-      if (euler && !last_step) {
+      if (euler && !last_step && p->spec_p2(0)) {  // (the 5-smooth x pass has no fused filter)
         pending_px = true;
       } else {
-        const bool back = euler && !cfl;  // E' -> E in the same pass
+        const bool back = euler && !cfl && last_step;  // E' -> E in the same pass
         if ((rc = apply_op(p, 0, U, U, p->nc, 0, 1.0f, s, true, act, 0, back)) != PS_OK) return rc;
         if (!euler && (rc = project_state(p, U, act, s)) != PS_OK) return rc;
       }
@@ -1502,6 +1520,18 @@ int create(const ps_plan_desc* d, int nsolve, ps_plan* out) {
     if ((rc = ps::lgl_setup(p)) != PS_OK) return cleanup(rc);
   } else if (mr) {
     if ((rc = ps::mr_setup(p)) != PS_OK) return cleanup(rc);
+    for (int a = 0; a < p->nd && p->spec; ++a) {  // its power-of-two axes run on the register pencils
+      if (!ps::supported_n(p->n[a])) continue;
+      const int N = p->n[a];
+      std::vector<float> P, dd;
+      std::vector<float2> twf, twi;
+      build_axis(N, d->length[a], 1, 0, 8, 36.0, P, dd, twf, twi);
+      if ((rc = dalloc(p, &p->p2_twf[a], N)) != PS_OK || (rc = dalloc(p, &p->p2_twi[a], N)) != PS_OK)
+        return cleanup(rc);
+      if (cudaMemcpy(p->p2_twf[a], twf.data(), N * sizeof(float2), cudaMemcpyHostToDevice) != cudaSuccess ||
+          cudaMemcpy(p->p2_twi[a], twi.data(), N * sizeof(float2), cudaMemcpyHostToDevice) != cudaSuccess)
+        return cleanup(cuda_fail(cudaGetLastError(), "table upload"));
+    }
   } else if (p->nd >= 2 && !(p->mhd && p->nd == 3)) {
     if ((rc = make_map(&p->map_G_y, p->G, p, p->mhd ? 16 : (p->nd == 3) ? 15 : 8, 1)) != PS_OK)
       return cleanup(rc);
@@ -1565,9 +1595,11 @@ int ps_batch_scratch_bytes(const ps_plan_desc* d, int nsolve, size_t* bytes) {
   for (int a = 0; a < d->ndim; ++a) tables += (size_t)d->n[a] * (2 * sizeof(float) + 2 * sizeof(float2));
   if (line1d_plan(d)) tables += (size_t)d->n[0] * sizeof(float2);
   if (is_lgl(d)) tables = ps::lgl_scratch_bytes(d, nsolve);
-  if (is_mr(d)) {  // P, d and the twiddles W_N^q per axis
+  if (is_mr(d)) {  // P, d and two twiddle tables per axis
     tables = 0;
-    for (int a = 0; a < d->ndim; ++a) tables += (size_t)d->n[a] * (2 * sizeof(float) + sizeof(float2));
+    for (int a = 0; a < d->ndim; ++a)
+      tables += (size_t)d->n[a] * (2 * sizeof(float) + 2 * sizeof(float2) +
+                                   (spec_plan(d) && ps::supported_n(d->n[a]) ? 2 * sizeof(float2) : 0));
   }
   size_t fields = scratch_fields(d->ndim, d->equations == PS_EQ_MHD);
   if (is_mr(d) && d->ndim == 1) fields += 6;  // stage input and increments

@@ -52,7 +52,13 @@ def check(got, ref, d, mhd):
 
 
 SHAPES2 = [(8, 8), (8, 16), (16, 8), (32, 64), (512, 8), (8, 512), (1024, 16), (16, 1024), (128, 256)]
-SHAPES3 = [(8, 8, 8), (8, 16, 32), (32, 8, 16), (16, 64, 8), (64, 8, 8), (8, 8, 512), (8, 512, 8), (256, 8, 8)]
+# axes of 2^a 3^b 5^c points (csrc/mr_spec.cu): odd, prime powers, the longest,
+# in either place and beside a power of two
+SHAPES2 += [(45, 64), (64, 45), (3, 40), (40, 6), (250, 96), (96, 250), (3645, 8), (8, 3645), (2048, 12), (12, 2048),
+            (4096, 10), (10, 4096), (27, 25), (360, 480), (16, 3125)]
+SHAPES3 = [(15, 16, 27), (16, 15, 8), (8, 27, 20), (30, 8, 16), (12, 10, 9), (6, 5, 4), (81, 8, 10), (8, 125, 9),
+           (10, 9, 1500)]
+SHAPES3 += [(8, 8, 8), (8, 16, 32), (32, 8, 16), (16, 64, 8), (64, 8, 8), (8, 8, 512), (8, 512, 8), (256, 8, 8)]
 
 
 @pytest.mark.parametrize("shape", SHAPES2 + SHAPES3, ids=str)
@@ -101,7 +107,7 @@ def test_mhd_steps(shape, options, interval):
     check(U.double().cpu().numpy(), ref, d, True)
 
 
-@pytest.mark.parametrize("shape", [(16, 8), (64, 64), (256, 32), (8, 16, 8)], ids=str)
+@pytest.mark.parametrize("shape", [(16, 8), (64, 64), (256, 32), (8, 16, 8), (45, 60), (64, 90), (9, 16, 10)], ids=str)
 def test_euler_cfl_batch(shape):
     """Three solves of one plan: one already at its end, one that ends inside
     the chunk, one that runs through it."""
