@@ -78,6 +78,139 @@ LglStageArgs stage_args(ps_plan p, const float* in, int stage, const float* Un, 
 // accumulator and their writes as the stage needs them)
 double field_bytes(const ps_plan_s* p) { return 4.0 * p->cells * p->nsolve; }
 
+// Steps by even and odd parts on the tensor cores: float32 and split-bf16 x3
+// plans with the filter and walls after every step and no gravity (a cadence
+// that skips steps leaves raw wall values in the state, and gravity needs the
+// stage input; those plans and the bare right-hand side keep the kernels above).
+bool eo_plan(const ps_plan_desc* d) {
+  return d->ndim == 2 && (d->gemm_precision == PS_GEMM_FP32 || d->gemm_precision == PS_GEMM_BF16X3) &&
+         d->filter_interval == 1 && d->gravity[0] == 0.0 && d->gravity[1] == 0.0;
+}
+
+struct EoSizes {
+  int hx, hy, kx, ky, ldx;
+  size_t X, Y, mats, C;  // bf16 elements of the operands and matrices, floats of the products
+};
+EoSizes eo_sizes(const ps_plan_desc* d, int nsolve) {
+  EoSizes e{};
+  const int nx = d->n[0], ny = d->n[1], P = kEoParts;
+  e.hx = (nx + 1) / 2;
+  e.hy = (ny + 1) / 2;
+  e.kx = (e.hx + 7) / 8 * 8;
+  e.ky = (e.hy + 7) / 8 * 8;
+  e.ldx = (e.hx + 3) / 4 * 4;
+  e.X = (size_t)P * 2 * nsolve * 4 * ny * e.kx;
+  e.Y = (size_t)P * 2 * nsolve * 4 * nx * e.ky;
+  e.mats = (size_t)P * 2 * ((size_t)e.hx * e.kx + (size_t)e.hy * e.ky) * (d->filter_enabled ? 2 : 1);
+  e.C = (size_t)2 * nsolve * 4 * ((size_t)ny * e.ldx + (size_t)e.hy * nx);
+  return e;
+}
+
+int eo_setup(ps_plan p) {
+  const EoSizes z = eo_sizes(&p->desc, p->nsolve);
+  EoBufs& b = p->eob;
+  int rc;
+  b.x = EoAxis{p->n[0], z.hx, z.kx};
+  b.y = EoAxis{p->n[1], z.hy, z.ky};
+  b.ldx = z.ldx;
+  const int nmax = p->n[0] > p->n[1] ? p->n[0] : p->n[1];
+  b.ntx = eo_n_tile(z.hx > z.hy ? z.hx : z.hy, 4 * (((long)p->nsolve * 4 * nmax + 127) / 128));
+  unsigned short *X = nullptr, *Y = nullptr, *M = nullptr;
+  if ((rc = plan_alloc(p, &X, z.X)) != PS_OK || (rc = plan_alloc(p, &Y, z.Y)) != PS_OK ||
+      (rc = plan_alloc(p, &M, z.mats)) != PS_OK || (rc = plan_alloc(p, &b.CX, z.C)) != PS_OK)
+    return rc;
+  b.X = X;
+  b.Y = Y;
+  b.CY = b.CX + (size_t)2 * p->nsolve * 4 * p->n[1] * z.ldx;
+  LGL_CU(cudaMemset(X, 0, sizeof(unsigned short) * z.X), "operand clear");
+  LGL_CU(cudaMemset(Y, 0, sizeof(unsigned short) * z.Y), "operand clear");
+  LGL_CU(cudaMemset(M, 0, sizeof(unsigned short) * z.mats), "matrix clear");
+  int e = 0;
+  if ((e = encode_eo_map(&b.mX, X, z.hx, p->nsolve * 4 * p->n[1], z.kx, 128)) != 0 ||
+      (e = encode_eo_map(&b.mY, Y, z.hy, p->nsolve * 4 * p->n[0], z.ky, 128)) != 0)
+    return errorf(PS_ERR_CUDA, "tensor map encoding for the even/odd contractions failed (%d)", e);
+  for (int f = 0; f < (p->desc.filter_enabled ? 2 : 1); ++f)
+    for (int a = 0; a < 2; ++a) {
+      const int h = a ? z.hy : z.hx, k = a ? z.ky : z.kx;
+      LGL_CU(launch_eo_matrix(f ? p->F64[a] : p->D64[a], p->n[a], k, f != 0, M, 0), "even/odd matrix");
+      CUtensorMap* m = f ? (a ? &b.mFy : &b.mFx) : (a ? &b.mDy : &b.mDx);
+      if ((e = encode_eo_map(m, M, h, h, k, b.ntx)) != 0)
+        return errorf(PS_ERR_CUDA, "tensor map encoding for the even/odd contractions failed (%d)", e);
+      M += (size_t)kEoParts * 2 * h * k;
+    }
+  LGL_CU(cudaDeviceSynchronize(), "even/odd tables");
+  p->eo = true;
+  return PS_OK;
+}
+
+// One step: operands of U^n, then per stage the contractions and the
+// cell-wise kernel (the last one filters, or writes the state with its walls).
+int step_eo(ps_plan p, float* U, double dt, const double* dtp, bool shift_in, bool shift_out, const int* act,
+            cudaStream_t s) {
+  EoGemmArgs g{};
+  g.b = p->eob;
+  g.nsolve = p->nsolve;
+  g.dirs = 3;
+  g.active = act;
+  g.status = p->status;
+  EoStageArgs a{};
+  a.b = p->eob;
+  a.U = U;
+  a.out = U;
+  a.acc_in = p->acc;
+  a.acc_out = p->Us;
+  a.S = p->G;
+  a.V = p->G + 4 * p->cells * p->nsolve;
+  a.nsolve = p->nsolve;
+  a.dt_dev = dtp;
+  a.dt = dt;
+  a.gamma = (float)p->desc.gamma;
+  a.rho_min = 1e-8f;  // 2D clamp floors (solver.py:489-490)
+  a.p_min = 1e-10f;
+  a.eref = p->eref;
+  a.active = act;
+  a.rk2 = (p->desc.scheme == PS_SCHEME_RK2) ? 1 : 0;
+  a.shift_in = shift_in ? 1 : 0;
+  a.shift_out = shift_out ? 1 : 0;
+  a.wall_acc = p->desc.filter_enabled;
+  // bytes: operands of kEoParts bf16 parts per value (x and y), products in float32
+  const double fb = field_bytes(p), op = 8.0 * fb * kEoParts / 2.0;
+  {
+    ProfScope prof(p, s, PS_KIND_LAST, 4.0 * fb + op);
+    LGL_CU(launch_eo_stage(a, kEoStart, kEoFlux, s), "LGL operands");
+  }
+  for (int st = 0; st < 4; ++st) {
+    if (a.rk2 && (st == 1 || st == 2)) continue;
+    a.stage = st;
+    {
+      ProfScope prof(p, s, PS_KIND_LGL_X, op + 8.0 * fb);
+      LGL_CU(launch_eo_gemm(g, s), "LGL contractions");
+    }
+    if (st < 3) {
+      ProfScope prof(p, s, PS_KIND_LAST, 20.0 * fb + op);
+      LGL_CU(launch_eo_stage(a, kEoStage, kEoFlux, s), "LGL stage");
+      const float* t = a.acc_in;
+      a.acc_in = a.acc_out;
+      a.acc_out = const_cast<float*>(t);
+    }
+  }
+  if (!p->desc.filter_enabled) {
+    ProfScope prof(p, s, PS_KIND_LAST, 20.0 * fb);
+    LGL_CU(launch_eo_stage(a, kEoStage, kEoOut, s), "LGL stage");
+    return PS_OK;
+  }
+  ProfScope prof(p, s, PS_KIND_OP, 24.0 * fb + 2.0 * op);
+  LGL_CU(launch_eo_stage(a, kEoStage, kEoFilterX, s), "LGL stage and filter operand");
+  g.filter = 1;
+  g.dirs = 1;
+  LGL_CU(launch_eo_gemm(g, s), "LGL x filter");
+  LGL_CU(launch_eo_filter_y(a, s), "LGL filter operand");
+  g.dirs = 2;
+  LGL_CU(launch_eo_gemm(g, s), "LGL y filter");
+  LGL_CU(launch_eo_filter_out(a, s), "LGL filtered state");
+  return PS_OK;
+}
+
 // One stage on the tensor cores: split flux planes, the two split-bf16 x3
 // contractions (x: all solves and components stacked as rows; y: one batch
 // entry per solve and component), then the elementwise update.
@@ -300,6 +433,10 @@ size_t lgl_scratch_bytes(const ps_plan_desc* d, int nsolve) {
     b += 4 * (nx * px + ny * py);                             // split D planes
     b += 4 * 4 * (size_t)nsolve * (ny * px + nx * py);       // split flux planes
   }
+  if (eo_plan(d)) {
+    const EoSizes e = eo_sizes(d, nsolve);
+    b += 2 * (e.X + e.Y + e.mats) + 4 * e.C;
+  }
   return b;
 }
 
@@ -385,6 +522,7 @@ int lgl_setup(ps_plan p) {
       return errorf(PS_ERR_CUDA, "tensor map encoding for the split contractions failed (%d)", e);
     LGL_CU(cudaDeviceSynchronize(), "split tables");
   }
+  if (eo_plan(&p->desc) && (rc = eo_setup(p)) != PS_OK) return rc;
   return PS_OK;
 }
 
@@ -461,7 +599,8 @@ int lgl_steps(ps_plan p, float* U, int nsteps, double dt, const double* d_dt, do
   const long ssU = p->ss(4);
   float* E = U + 3 * p->cells;
   LGL_CU(launch_eref_set(E, ssU, p->nsolve, p->eref, s), "energy reference");
-  LGL_CU(launch_energy_shift(E, p->cells, ssU, p->nsolve, p->eref, -1.0f, s), "energy shift");
+  if (cfl || !p->eo)  // fixed even/odd steps subtract E_ref on the first step's loads
+    LGL_CU(launch_energy_shift(E, p->cells, ssU, p->nsolve, p->eref, -1.0f, s), "energy shift");
   if (cfl) LGL_CU(launch_fill_int(p->active, p->nsolve, 1, s), "active reset");
   for (int it = 0; it < nsteps; ++it) {
     const bool due = (p->step_counter % p->desc.filter_interval) == 0;
@@ -472,6 +611,12 @@ int lgl_steps(ps_plan p, float* U, int nsteps, double dt, const double* d_dt, do
              "wave speed");
       LGL_CU(launch_step_control(p->speed, p->desc.cfl, p->hmin(), d_t, d_tend, p->nsolve, p->dt, p->active, s),
              "step control");
+    }
+    if (p->eo) {
+      if ((rc = step_eo(p, U, dt, dtp, !cfl && it == 0, !cfl && it + 1 == nsteps, act, s)) != PS_OK) return rc;
+      if (cfl) LGL_CU(launch_step_advance(d_t, p->dt, p->speed, p->active, p->steps_done, p->nsolve, s), "advance");
+      p->step_counter += 1;
+      continue;
     }
     // The CUDA-core y contraction reads its stage input along whole columns
     // while its epilogue writes the next stage input, so that stage's input
@@ -492,7 +637,8 @@ int lgl_steps(ps_plan p, float* U, int nsteps, double dt, const double* d_dt, do
     if (cfl) LGL_CU(launch_step_advance(d_t, p->dt, p->speed, p->active, p->steps_done, p->nsolve, s), "advance");
     p->step_counter += 1;
   }
-  LGL_CU(launch_energy_shift(E, p->cells, ssU, p->nsolve, p->eref, 1.0f, s), "energy shift");
+  if (cfl || !p->eo)
+    LGL_CU(launch_energy_shift(E, p->cells, ssU, p->nsolve, p->eref, 1.0f, s), "energy shift");
   return PS_OK;
 }
 

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/phrike_gb300.h"
+#include "lgl_eo.cuh"
 #include "mixed_radix.cuh"
 #include "mr_spec.cuh"
 #include "pass_common.cuh"
@@ -102,6 +103,8 @@ struct ps_plan_s {
   void* FYT = nullptr;                    // [2][nsolve*4][nx][pitch_y] transposed y flux
   CUtensorMap map_FX{}, map_Dx{}, map_Dy{}, map_FYT{};
   int nt_x = 0, nt_y = 0;                 // N tiles of the two contractions
+  bool eo = false;                        // steps by even and odd parts (lgl_eo.cu)
+  ps::EoBufs eob{};
 
   // Fourier axes of any 5-smooth length (mixed-radix passes, mr_plan.cu)
   bool mr = false;
