@@ -340,6 +340,8 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_op(OpArgs a) {
   using PF = Pencil<N, T, STRIDED>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto& S = *reinterpret_cast<StridedSmem<N, T, STRIDED>*>(smem_raw);
+  load_axis<N>(S.ax, a.ax);
+  dep_wait();
   int p, t;
   long base_in, base_out, step;
   bool valid;
@@ -364,7 +366,6 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_op(OpArgs a) {
     step = A;
   }
   PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
-  load_axis<N>(S.ax, a.ax);
   __syncthreads();
 #pragma unroll 1
   for (int c = 0; c < a.nf; c += 2) {

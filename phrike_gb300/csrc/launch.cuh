@@ -142,8 +142,7 @@ cudaError_t op_t_T(const CUtensorMap& mIn, const OpTArgs& a, cudaStream_t s) {
   const size_t sm = sizeof(TmaStridedSmem<NN, T, R>);
   cudaError_t e;
   if ((e = set_smem(k_op_t<NN, T, R>, sm)) != cudaSuccess) return e;
-  k_op_t<NN, T, R><<<grid, Shape<NN>::A * T, sm, s>>>(mIn, a);
-  return cudaGetLastError();
+  return launch_dep(k_op_t<NN, T, R>, grid, Shape<NN>::A * T, sm, s, mIn, a);
 }
 
 // Calls f(std::integral_constant<int, T>) for the tile width of a launch.
@@ -228,8 +227,7 @@ cudaError_t dispatch_proj_cols(long units, F&& f) {
     const size_t sm = sizeof(StridedSmem<NN, T, false>);                                              \
     cudaError_t e;                                                                                    \
     if ((e = set_smem(k_op<NN, T, false>, sm)) != cudaSuccess) return e;                              \
-    k_op<NN, T, false><<<grid, Shape<NN>::A * T, sm, s>>>(a);                                         \
-    return cudaGetLastError();                                                                        \
+    return launch_dep(k_op<NN, T, false>, grid, Shape<NN>::A * T, sm, s, a);                          \
   }                                                                                                   \
   template <>                                                                                         \
   cudaError_t launch_ymid3_t<NN>(const CUtensorMap& mG, const YMidTArgs& a, cudaStream_t s) {         \
@@ -260,8 +258,7 @@ cudaError_t dispatch_proj_cols(long units, F&& f) {
     const size_t sm = sizeof(LineSmem<NN>);                                                           \
     cudaError_t e;                                                                                    \
     if ((e = set_smem(k_line1d<NN>, sm)) != cudaSuccess) return e;                                    \
-    k_line1d<NN><<<nsolve, Line<NN>::BLOCK, sm, s>>>(a, tw);                                          \
-    return cudaGetLastError();                                                                        \
+    return launch_dep(k_line1d<NN>, nsolve, Line<NN>::BLOCK, sm, s, a, tw);                           \
   }                                                                                                   \
   template <>                                                                                         \
   cudaError_t launch_ark1d<NN>(const Ark1DArgs& a, int nsolve, cudaStream_t s) {                      \
@@ -315,8 +312,7 @@ cudaError_t dispatch_proj_cols(long units, F&& f) {
       if ((e = set_smem(k_proj_xf<NN, T>, sm)) != cudaSuccess) return e;                              \
       const int tiles = (a.ny * a.nsolve + T - 1) / T;                                                \
       const int fgroups = (tiles < 2 * 148) ? 2 : 1; /* Bx and By in separate CTAs */                 \
-      k_proj_xf<NN, T><<<dim3(tiles, fgroups), Shape<NN>::A * T, sm, s>>>(a);                         \
-      return cudaGetLastError();                                                                      \
+      return launch_dep(k_proj_xf<NN, T>, dim3(tiles, fgroups), Shape<NN>::A * T, sm, s, a);          \
     });                                                                                               \
   }                                                                                                   \
   template <>                                                                                         \
@@ -326,8 +322,7 @@ cudaError_t dispatch_proj_cols(long units, F&& f) {
       const size_t sm = sizeof(ProjYSmem<NN, T>);                                                     \
       cudaError_t e;                                                                                  \
       if ((e = set_smem(k_proj_y<NN, T>, sm)) != cudaSuccess) return e;                               \
-      k_proj_y<NN, T><<<dim3((a.hx + T - 1) / T, a.nsolve), Shape<NN>::A * T, sm, s>>>(a);            \
-      return cudaGetLastError();                                                                      \
+      return launch_dep(k_proj_y<NN, T>, dim3((a.hx + T - 1) / T, a.nsolve), Shape<NN>::A * T, sm, s, a); \
     });                                                                                               \
   }                                                                                                   \
   template <>                                                                                         \
@@ -337,8 +332,7 @@ cudaError_t dispatch_proj_cols(long units, F&& f) {
       const size_t sm = sizeof(MhdXSmem<NN, T>);                                                      \
       cudaError_t e;                                                                                  \
       if ((e = set_smem(k_proj_xi<NN, T>, sm)) != cudaSuccess) return e;                              \
-      k_proj_xi<NN, T><<<(a.ny * a.nsolve + T - 1) / T, Shape<NN>::A * T, sm, s>>>(a);                \
-      return cudaGetLastError();                                                                      \
+      return launch_dep(k_proj_xi<NN, T>, (a.ny * a.nsolve + T - 1) / T, Shape<NN>::A * T, sm, s, a); \
     });                                                                                               \
   }
 
@@ -359,8 +353,7 @@ cudaError_t dispatch_proj_cols(long units, F&& f) {
     const size_t sm = sizeof(StridedSmem<NN, T, false>);                                              \
     cudaError_t e;                                                                                    \
     if ((e = set_smem(k_op<NN, T, false>, sm)) != cudaSuccess) return e;                              \
-    k_op<NN, T, false><<<grid, Shape<NN>::A * T, sm, s>>>(a);                                         \
-    return cudaGetLastError();                                                                        \
+    return launch_dep(k_op<NN, T, false>, grid, Shape<NN>::A * T, sm, s, a);                          \
   }                                                                                                   \
   template <>                                                                                         \
   cudaError_t launch_step1d<NN>(const Step1DArgs& a, int nsolve, cudaStream_t s) {                    \
@@ -375,8 +368,7 @@ cudaError_t dispatch_proj_cols(long units, F&& f) {
     const size_t sm = sizeof(LineSmem<NN>);                                                           \
     cudaError_t e;                                                                                    \
     if ((e = set_smem(k_line1d<NN>, sm)) != cudaSuccess) return e;                                    \
-    k_line1d<NN><<<nsolve, Line<NN>::BLOCK, sm, s>>>(a, tw);                                          \
-    return cudaGetLastError();                                                                        \
+    return launch_dep(k_line1d<NN>, nsolve, Line<NN>::BLOCK, sm, s, a, tw);                           \
   }                                                                                                   \
   template <>                                                                                         \
   cudaError_t launch_ark1d<NN>(const Ark1DArgs& a, int nsolve, cudaStream_t s) {                      \

@@ -156,17 +156,11 @@ __global__ void __launch_bounds__(128, 1)
   const int M = g.nsolve * 4 * line, N = ax.h;
   const int m0 = blockIdx.y * 128, n0 = blockIdx.x * NT;
   if (m0 >= M || n0 >= N) return;
-  if (g.active != nullptr) {  // tiles whose rows all belong to inactive solves
-    bool any = false;
-    for (int z = m0 / (4 * line); !any && z <= (min(m0 + 128, M) - 1) / (4 * line); ++z) any = g.active[z] != 0;
-    if (!any) return;
-  }
   const CUtensorMap* mA = ydir ? &mAy : &mAx;
   const CUtensorMap* mB = ydir ? &mBy : &mBx;
   const uint32_t raw = smem_addr(umma_smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   unsigned char* sbase = umma_smem_raw + (base - raw);
-  const int nk = (ax.h + 63) / 64;
   if (tid == 0) {
     for (int s = 0; s < ST; ++s) {
       mbar_init(&full[s], 1);
@@ -183,11 +177,16 @@ __global__ void __launch_bounds__(128, 1)
     tmem_alloc(&tmem_base, COLS);
     tmem_relinquish();
   }
+  dep_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base;
   volatile int* vabort = &abort_flag;
+  // a tile whose rows all belong to inactive solves loads and stores nothing
+  bool any = g.active == nullptr;
+  for (int z = m0 / (4 * line); !any && z <= (min(m0 + 128, M) - 1) / (4 * line); ++z) any = g.active[z] != 0;
+  const int nk = any ? (ax.h + 63) / 64 : 0;
 
   if (tid == 0) {  // producer
     int kb = 0;
@@ -264,7 +263,7 @@ __global__ void __launch_bounds__(128, 1)
   if (!ok) atomicOr(g.status, kStatusTmaTimeout);
   tc_fence_after();
   const int all_ok = __syncthreads_and(ok ? 1 : 0);  // CTA-uniform: TMEM loads are warp-collective
-  const bool valid = all_ok && (*vabort == 0);
+  const bool valid = all_ok && (*vabort == 0) && nk > 0;
   const int m = m0 + warp * 32 + lane;
   if (valid) {
     float* row;    // element n at row[n * step]
@@ -326,8 +325,8 @@ cudaError_t eo_gemm_t(const EoGemmArgs& a, cudaStream_t s) {
   const int hx = x ? b.x.h : 0, hy = y ? b.y.h : 0;
   const int rows = rx > ry ? rx : ry, h = hx > hy ? hx : hy;
   const dim3 grid((h + NT - 1) / NT, (rows + 127) / 128, (x && y) ? 4 : 2);
-  k_eo_gemm<NT><<<grid, 128, bytes, s>>>(b.mX, a.filter ? b.mFx : b.mDx, b.mY, a.filter ? b.mFy : b.mDy, a);
-  return cudaGetLastError();
+  return launch_dep(k_eo_gemm<NT>, grid, 128, bytes, s, b.mX, a.filter ? b.mFx : b.mDx, b.mY,
+                    a.filter ? b.mFy : b.mDy, a);
 }
 }  // namespace
 
@@ -343,8 +342,6 @@ cudaError_t launch_eo_gemm(const EoGemmArgs& a, cudaStream_t s) {
 namespace {
 constexpr int TI = 32, TJ = 8;
 
-// NC: U is not written by the launch (read-only loads may pass the stores)
-template <bool NC>
 struct EoCell {
   const EoStageArgs& a;
   const int sol;
@@ -368,7 +365,7 @@ struct EoCell {
     inside(J, I, Jp, Ip);
     const float* p = a.U + so + (long)Jp * nx + Ip;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) u[c] = NC ? __ldg(p + c * cells) : p[c * cells];
+    for (int c = 0; c < 4; ++c) u[c] = p[c * cells];
     u[3] -= eshift;
     if (Ip != I) u[1] = 0.0f;
     if (Jp != J) u[2] = 0.0f;
@@ -383,36 +380,38 @@ struct EoCell {
       const float* cx = a.b.CX + ((long)(sol * 4 + c) * ny + J) * a.b.ldx + i;
       const float* cy = a.b.CY + ((long)(sol * 4 + c) * a.b.y.h + j) * nx + I;
       // even operand -> difference of the mirror pair, odd operand -> sum
-      k[c] = -((0.5f * __ldg(cx + px) + sx * __ldg(cx)) + (0.5f * __ldg(cy + py) + sy * __ldg(cy)));
+      k[c] = -((0.5f * cx[px] + sx * cx[0]) + (0.5f * cy[py] + sy * cy[0]));
     }
   }
-  // stage update of one point (own products, U^n with walls, increments)
-  __device__ __forceinline__ void stage(int J, int I, bool own, float (&u)[4]) const {
-    float k[4], ac[4];
+  // stage update of one point (own products, U^n with walls, increments); ac
+  // leaves with the stage's contribution and is stored by the caller, after
+  // the loads of its other points
+  __device__ __forceinline__ void stage(int J, int I, float (&u)[4], float (&ac)[4]) const {
+    float k[4];
     un(J, I, u);
     slope(J, I, k);
     const long o = so + (long)J * nx + I;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) ac[c] = (a.stage >= 1) ? __ldg(a.acc_in + o + c * cells) : 0.0f;
+    for (int c = 0; c < 4; ++c) ac[c] = (a.stage >= 1) ? a.acc_in[o + c * cells] : 0.0f;
 #pragma unroll
     for (int c = 0; c < 4; ++c) u[c] = rk_update_incr(a.stage, rk, k[c], u[c], ac[c]);
-    if (own && a.stage != 3) {
-#pragma unroll
-      for (int c = 0; c < 4; ++c) a.acc_out[o + c * cells] = ac[c];
-    }
     clamp_state<2>(u, a.gamma, a.rho_min, pmin_shift);
   }
   // the increments alone of a wall point (stages 0..2)
-  __device__ __forceinline__ void wall_increment(int J, int I) const {
+  __device__ __forceinline__ void wall_increment(int J, int I, float (&ac)[4]) const {
     float k[4];
     slope(J, I, k);
     const long o = so + (long)J * nx + I;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      float ac = (a.stage >= 1) ? __ldg(a.acc_in + o + c * cells) : 0.0f;
-      rk_update_incr(a.stage, rk, k[c], 0.0f, ac);
-      a.acc_out[o + c * cells] = ac;
+      ac[c] = (a.stage >= 1) ? a.acc_in[o + c * cells] : 0.0f;
+      rk_update_incr(a.stage, rk, k[c], 0.0f, ac[c]);
     }
+  }
+  __device__ __forceinline__ void keep(int J, int I, const float (&ac)[4]) const {
+    const long o = so + (long)J * nx + I;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) a.acc_out[o + c * cells] = ac[c];
   }
 };
 
@@ -452,8 +451,7 @@ __device__ __forceinline__ void put_y(const EoStageArgs& a, int sol, const float
 }
 
 // stores the point's new state and the wall points that copy it
-template <bool NC>
-__device__ __forceinline__ void put_state(const EoStageArgs& a, const EoCell<NC>& cell, int J, int I, const float (&u)[4]) {
+__device__ __forceinline__ void put_state(const EoStageArgs& a, const EoCell& cell, int J, int I, const float (&u)[4]) {
   if (J == 0 || I == 0 || J == cell.ny - 1 || I == cell.nx - 1) return;
   const float e = u[3] + (a.shift_out ? cell.er : 0.0f);
   auto put = [&](int j, int i) {
@@ -473,9 +471,10 @@ template <int FROM, int TO>
 __global__ void __launch_bounds__(TI * TJ, 2) k_eo_stage(EoStageArgs a) {
   __shared__ float sm[TO == kEoFlux ? 16 * TI * (TJ + 1) : 1];
   const int sol = blockIdx.z;
+  dep_wait();
   if (a.active != nullptr && a.active[sol] == 0) return;
   const float dt = (a.dt_dev != nullptr) ? (float)a.dt_dev[sol] : (float)a.dt;
-  const EoCell<TO != kEoOut> cell(a, sol, dt);
+  const EoCell cell(a, sol, dt);
   const int nx = cell.nx, ny = cell.ny, hx = a.b.x.h, hy = a.b.y.h;
   const int il = threadIdx.x % TI, jl = threadIdx.x / TI;
   const int i0 = blockIdx.x * TI, j0 = blockIdx.y * TJ;
@@ -483,7 +482,7 @@ __global__ void __launch_bounds__(TI * TJ, 2) k_eo_stage(EoStageArgs a) {
   const bool in = i < hx && j < hy;
   const int im = nx - 1 - i, jm = ny - 1 - j;
   const bool ci = im == i, cj = jm == j;  // centre line / row: its own mirror
-  float u[4][4] = {};  // points (j, i), (j, im), (jm, i), (jm, im)
+  float u[4][4] = {}, ac[4][4];  // points (j, i), (j, im), (jm, i), (jm, im)
 #pragma unroll
   for (int p = 0; p < 4; ++p) {
     const int J = (p & 2) ? jm : j, I = (p & 1) ? im : i;
@@ -493,7 +492,6 @@ __global__ void __launch_bounds__(TI * TJ, 2) k_eo_stage(EoStageArgs a) {
     } else if (FROM == kEoStart) {
       cell.un(J, I, u[p]);
     } else {
-      const bool dup = ((p & 1) && ci) || ((p & 2) && cj);
       // a launch that writes the state skips the walls: their U^n may be in the making
       const bool wall = i == 0 || j == 0;
       if (TO == kEoOut && wall) continue;
@@ -502,15 +500,22 @@ __global__ void __launch_bounds__(TI * TJ, 2) k_eo_stage(EoStageArgs a) {
         // increments are kept only for the filter, which sees the raw walls
         int Jp, Ip;
         cell.inside(J, I, Jp, Ip);
-        cell.stage(Jp, Ip, !dup && !wall, u[p]);
+        cell.stage(Jp, Ip, u[p], ac[p]);
         if (wall) {
           if (Ip != I) u[p][1] = 0.0f;
           if (Jp != J) u[p][2] = 0.0f;
-          if (a.wall_acc && !dup) cell.wall_increment(J, I);
+          if (a.wall_acc) cell.wall_increment(J, I, ac[p]);
         }
       } else {
-        cell.stage(J, I, !dup, u[p]);
+        cell.stage(J, I, u[p], ac[p]);
       }
+    }
+  }
+  if constexpr (FROM == kEoStage && TO == kEoFlux) {
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      const bool dup = ((p & 1) && ci) || ((p & 2) && cj);
+      if (in && !dup && (a.wall_acc || (i > 0 && j > 0))) cell.keep((p & 2) ? jm : j, (p & 1) ? im : i, ac[p]);
     }
   }
   if constexpr (TO == kEoOut) {
@@ -533,7 +538,8 @@ __global__ void __launch_bounds__(TI * TJ, 2) k_eo_stage(EoStageArgs a) {
       const int J = q ? jm : j;
       if (!in || (q && cj)) break;
       float f0[4];
-      cell.stage(J, 0, false, f0);
+      float f1[4];
+      cell.stage(J, 0, f0, f1);
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const float f = q ? u[2][c] : u[0][c], fm = q ? u[3][c] : u[1][c];
@@ -591,13 +597,14 @@ __device__ __forceinline__ void x_filtered(const EoStageArgs& a, int sol, int J,
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     const float* cx = a.b.CX + ((long)(sol * 4 + c) * ny + J) * a.b.ldx + i;
-    v[c] = __ldg(a.S + ((long)sol * 4 + c) * cells + (long)J * nx + I) - (0.5f * __ldg(cx) + sx * __ldg(cx + px));
+    v[c] = a.S[((long)sol * 4 + c) * cells + (long)J * nx + I] - (0.5f * cx[0] + sx * cx[px]);
   }
 }
 
 __global__ void __launch_bounds__(TI * TJ) k_eo_filter_y(EoStageArgs a) {
   __shared__ float sm[16 * TI * (TJ + 1)];
   const int sol = blockIdx.z;
+  dep_wait();
   if (a.active != nullptr && a.active[sol] == 0) return;
   const int nx = a.b.x.n, ny = a.b.y.n, hx = a.b.x.h, hy = a.b.y.h;
   const int il = threadIdx.x % TI, jl = threadIdx.x / TI;
@@ -634,8 +641,9 @@ __global__ void __launch_bounds__(TI * TJ) k_eo_filter_y(EoStageArgs a) {
 
 __global__ void __launch_bounds__(TI * TJ) k_eo_filter_out(EoStageArgs a) {
   const int sol = blockIdx.z;
+  dep_wait();
   if (a.active != nullptr && a.active[sol] == 0) return;
-  const EoCell<false> cell(a, sol, 0.0f);
+  const EoCell cell(a, sol, 0.0f);
   const int nx = cell.nx, ny = cell.ny, hy = a.b.y.h;
   const int I = blockIdx.x * TI + threadIdx.x % TI, J = blockIdx.y * TJ + threadIdx.x / TI;
   if (I >= nx || J >= ny) return;
@@ -646,7 +654,7 @@ __global__ void __launch_bounds__(TI * TJ) k_eo_filter_out(EoStageArgs a) {
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     const float* cy = a.b.CY + ((long)(sol * 4 + c) * hy + j) * nx + I;
-    u[c] = __ldg(a.V + cell.so + c * cell.cells + (long)J * nx + I) - (0.5f * __ldg(cy) + sy * __ldg(cy + py));
+    u[c] = a.V[cell.so + c * cell.cells + (long)J * nx + I] - (0.5f * cy[0] + sy * cy[py]);
   }
   put_state(a, cell, J, I, u);
 }
@@ -656,12 +664,11 @@ dim3 eo_grid(const EoStageArgs& a) {
 }
 cudaError_t eo_stage_any(const EoStageArgs& a, int from, int to, cudaStream_t s) {
   const dim3 g = eo_grid(a);
-  if (from == kEoStart && to == kEoFlux) k_eo_stage<kEoStart, kEoFlux><<<g, TI * TJ, 0, s>>>(a);
-  else if (from == kEoStage && to == kEoFlux) k_eo_stage<kEoStage, kEoFlux><<<g, TI * TJ, 0, s>>>(a);
-  else if (from == kEoStage && to == kEoFilterX) k_eo_stage<kEoStage, kEoFilterX><<<g, TI * TJ, 0, s>>>(a);
-  else if (from == kEoStage && to == kEoOut) k_eo_stage<kEoStage, kEoOut><<<g, TI * TJ, 0, s>>>(a);
-  else return cudaErrorInvalidValue;
-  return cudaGetLastError();
+  if (from == kEoStart && to == kEoFlux) return launch_dep(k_eo_stage<kEoStart, kEoFlux>, g, TI * TJ, 0, s, a);
+  if (from == kEoStage && to == kEoFlux) return launch_dep(k_eo_stage<kEoStage, kEoFlux>, g, TI * TJ, 0, s, a);
+  if (from == kEoStage && to == kEoFilterX) return launch_dep(k_eo_stage<kEoStage, kEoFilterX>, g, TI * TJ, 0, s, a);
+  if (from == kEoStage && to == kEoOut) return launch_dep(k_eo_stage<kEoStage, kEoOut>, g, TI * TJ, 0, s, a);
+  return cudaErrorInvalidValue;
 }
 }  // namespace
 
@@ -669,12 +676,10 @@ cudaError_t launch_eo_stage(const EoStageArgs& a, int from, int to, cudaStream_t
   return eo_stage_any(a, from, to, s);
 }
 cudaError_t launch_eo_filter_y(const EoStageArgs& a, cudaStream_t s) {
-  k_eo_filter_y<<<eo_grid(a), TI * TJ, 0, s>>>(a);
-  return cudaGetLastError();
+  return launch_dep(k_eo_filter_y, eo_grid(a), TI * TJ, 0, s, a);
 }
 cudaError_t launch_eo_filter_out(const EoStageArgs& a, cudaStream_t s) {
-  k_eo_filter_out<<<dim3((a.b.x.n + TI - 1) / TI, (a.b.y.n + TJ - 1) / TJ, a.nsolve), TI * TJ, 0, s>>>(a);
-  return cudaGetLastError();
+  return launch_dep(k_eo_filter_out, dim3((a.b.x.n + TI - 1) / TI, (a.b.y.n + TJ - 1) / TJ, a.nsolve), TI * TJ, 0, s, a);
 }
 
 }  // namespace ps

@@ -225,8 +225,14 @@ __global__ void __launch_bounds__(Line<N>::BLOCK) k_line1d(Step1DArgs a, const f
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto& S = *reinterpret_cast<LineSmem<N>*>(smem_raw);
   const int sol = blockIdx.x;
-  if (a.active != nullptr && a.active[sol] == 0) return;
   const int tid = threadIdx.x;
+  LineFft<N> ft{S, tid, tid < TH};
+  if (!Ln::HELP || tid < TH) ft.setup(tw, a.ax);
+  if constexpr (Ln::TW_SMEM) {
+    for (int k = tid; k < N; k += blockDim.x) S.tw[k] = tw[k];
+  }
+  dep_wait();
+  if (a.active != nullptr && a.active[sol] == 0) return;
   const bool cfl = a.t != nullptr;
   float* U = a.U + (long)sol * a.solve_stride;
   const float er = U[2 * N];  // E_ref; U is written only after the last step
@@ -249,9 +255,6 @@ __global__ void __launch_bounds__(Line<N>::BLOCK) k_line1d(Step1DArgs a, const f
   if (cfl && (Ln::HELP ? tid == TH : tid == 0)) {
     tl = a.t[sol];
     te = a.tend[sol];
-  }
-  if constexpr (Ln::TW_SMEM) {
-    for (int k = tid; k < N; k += blockDim.x) S.tw[k] = tw[k];
   }
   // er is read by every thread before any writes U
   __syncthreads();
@@ -278,8 +281,6 @@ __global__ void __launch_bounds__(Line<N>::BLOCK) k_line1d(Step1DArgs a, const f
     return;
   }
 
-  LineFft<N> ft{S, tid, tid < TH};
-  ft.setup(tw, a.ax);
   const bool own = tid < TH;
   const float pmin_shift = a.p_min - g1 * er;
   const float href = a.gamma * er;

@@ -163,6 +163,8 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_proj3_xf(Proj3Args a) {
   using PF = Pencil<N, T, false>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto& S = *reinterpret_cast<MhdXSmem<N, T>*>(smem_raw);
+  load_axis<N>(S.ax, a.ax);
+  dep_wait();
   const int t = threadIdx.x % A, p = threadIdx.x / A;
   const int rps = a.ny * a.nz;
   const int rows = rps * a.nsolve;
@@ -171,7 +173,6 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_proj3_xf(Proj3Args a) {
   const int r = row % rps;
   const bool valid = row < rows && (a.active == nullptr || a.active[sol] != 0);
   PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
-  load_axis<N>(S.ax, a.ax);
   __syncthreads();
 #pragma unroll 1
   for (int f = 0; f < 3; ++f) {
@@ -199,6 +200,8 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_proj3_y(Proj3Args a) {
   using PF = Pencil<N, T, true>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto& S = *reinterpret_cast<ProjYSmem<N, T>*>(smem_raw);
+  load_axis<N>(S.ax, a.ax);
+  dep_wait();
   const int p = threadIdx.x % T, t = threadIdx.x / T;
   const int kx = blockIdx.x * T + p;
   const int plane = blockIdx.y;  // (sol * 3 + f) * nz + z
@@ -206,7 +209,6 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_proj3_y(Proj3Args a) {
   if (a.active != nullptr && a.active[sol] == 0) return;
   const bool valid = kx < a.hx;
   PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
-  load_axis<N>(S.ax, a.ax);
   __syncthreads();
   float2* col = a.H + (long)plane * N * a.hx + kx;
   float2 v[B];
@@ -237,6 +239,8 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_proj3_z(Proj3Args a) {
   using PF = Pencil<N, T, true>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto& S = *reinterpret_cast<ProjYSmem<N, T>*>(smem_raw);
+  load_axis<N>(S.ax, a.ax);
+  dep_wait();
   const int p = threadIdx.x % T, t = threadIdx.x / T;
   const int colid = blockIdx.x * T + p;  // ky * hx + kx
   const int sol = blockIdx.y;
@@ -244,7 +248,6 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_proj3_z(Proj3Args a) {
   const long plane = (long)a.ny * a.hx;
   const bool valid = colid < plane;
   PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
-  load_axis<N>(S.ax, a.ax);
   __syncthreads();
   const long fstride = (long)N * plane;
   float2* c0 = a.H + (long)sol * 3 * fstride + colid;
@@ -304,6 +307,8 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_proj3_xi(Proj3Args a) {
   using PF = Pencil<N, T, false>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto& S = *reinterpret_cast<MhdXSmem<N, T>*>(smem_raw);
+  load_axis<N>(S.ax, a.ax);
+  dep_wait();
   const int t = threadIdx.x % A, p = threadIdx.x / A;
   const int rps = a.ny * a.nz;
   const int rows = rps * a.nsolve;
@@ -312,7 +317,6 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_proj3_xi(Proj3Args a) {
   const int r = row % rps;
   const bool valid = row < rows && (a.active == nullptr || a.active[sol] != 0);
   PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
-  load_axis<N>(S.ax, a.ax);
   __syncthreads();
   const float2* h0 = a.H + (((long)sol * 3 + 0) * rps + r) * a.hx;
   const float2* h1 = h0 + (long)rps * a.hx;
@@ -412,8 +416,7 @@ cudaError_t launch_proj3_xf(int n, const Proj3Args& a, cudaStream_t s) {
     cudaError_t e = set_smem(k_proj3_xf<NN, T>, sm);
     if (e != cudaSuccess) return e;
     const int rows = a.ny * a.nz * a.nsolve;
-    k_proj3_xf<NN, T><<<(rows + T - 1) / T, Shape<NN>::A * T, sm, s>>>(a);
-    return cudaGetLastError();
+    return launch_dep(k_proj3_xf<NN, T>, (rows + T - 1) / T, Shape<NN>::A * T, sm, s, a);
   });
 }
 
@@ -425,10 +428,10 @@ cudaError_t launch_proj3_y(int n, bool inverse, const Proj3Args& a, cudaStream_t
     cudaError_t e;
     if (inverse) {
       if ((e = set_smem(k_proj3_y<NN, T, true>, sm)) != cudaSuccess) return e;
-      k_proj3_y<NN, T, true><<<grid, Shape<NN>::A * T, sm, s>>>(a);
+      return launch_dep(k_proj3_y<NN, T, true>, grid, Shape<NN>::A * T, sm, s, a);
     } else {
       if ((e = set_smem(k_proj3_y<NN, T, false>, sm)) != cudaSuccess) return e;
-      k_proj3_y<NN, T, false><<<grid, Shape<NN>::A * T, sm, s>>>(a);
+      return launch_dep(k_proj3_y<NN, T, false>, grid, Shape<NN>::A * T, sm, s, a);
     }
     return cudaGetLastError();
   });
@@ -441,8 +444,7 @@ cudaError_t launch_proj3_z(int n, const Proj3Args& a, cudaStream_t s) {
     cudaError_t e = set_smem(k_proj3_z<NN, T>, sm);
     if (e != cudaSuccess) return e;
     const dim3 grid((a.ny * a.hx + T - 1) / T, a.nsolve);
-    k_proj3_z<NN, T><<<grid, Shape<NN>::A * T, sm, s>>>(a);
-    return cudaGetLastError();
+    return launch_dep(k_proj3_z<NN, T>, grid, Shape<NN>::A * T, sm, s, a);
   });
 }
 
@@ -453,8 +455,7 @@ cudaError_t launch_proj3_xi(int n, const Proj3Args& a, cudaStream_t s) {
     cudaError_t e = set_smem(k_proj3_xi<NN, T>, sm);
     if (e != cudaSuccess) return e;
     const int rows = a.ny * a.nz * a.nsolve;
-    k_proj3_xi<NN, T><<<(rows + T - 1) / T, Shape<NN>::A * T, sm, s>>>(a);
-    return cudaGetLastError();
+    return launch_dep(k_proj3_xi<NN, T>, (rows + T - 1) / T, Shape<NN>::A * T, sm, s, a);
   });
 }
 

@@ -223,6 +223,8 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_proj_xf(ProjArgs a) {
   using PF = Pencil<N, T, false>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto& S = *reinterpret_cast<MhdXSmem<N, T>*>(smem_raw);
+  load_axis<N>(S.ax, a.ax);
+  dep_wait();
   const int t = threadIdx.x % A, p = threadIdx.x / A;
   const int rows = a.ny * a.nsolve;
   const int row = blockIdx.x * T + p;
@@ -230,7 +232,6 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_proj_xf(ProjArgs a) {
   const int j = row % a.ny;
   const bool valid = row < rows && (a.active == nullptr || a.active[sol] != 0);
   PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
-  load_axis<N>(S.ax, a.ax);
   __syncthreads();
   // Bx and By: both in each CTA, or one per CTA row of a two-row grid
 #pragma unroll 1
@@ -264,13 +265,14 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_proj_y(ProjArgs a) {
   using PF = Pencil<N, T, true>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto& S = *reinterpret_cast<ProjYSmem<N, T>*>(smem_raw);
+  load_axis<N>(S.ax, a.ax);
+  dep_wait();
   const int p = threadIdx.x % T, t = threadIdx.x / T;
   const int kx = blockIdx.x * T + p;
   const int sol = blockIdx.y;
   if (a.active != nullptr && a.active[sol] == 0) return;
   const bool valid = kx < a.hx;
   PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
-  load_axis<N>(S.ax, a.ax);
   __syncthreads();
   float2* hx_ = a.H + ((long)sol * 2 + 0) * a.ny * a.hx + kx;
   float2* hy_ = a.H + ((long)sol * 2 + 1) * a.ny * a.hx + kx;
@@ -322,6 +324,8 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_proj_xi(ProjArgs a) {
   using PF = Pencil<N, T, false>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto& S = *reinterpret_cast<MhdXSmem<N, T>*>(smem_raw);
+  load_axis<N>(S.ax, a.ax);
+  dep_wait();
   const int t = threadIdx.x % A, p = threadIdx.x / A;
   const int rows = a.ny * a.nsolve;
   const int row = blockIdx.x * T + p;
@@ -329,7 +333,6 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_proj_xi(ProjArgs a) {
   const int j = row % a.ny;
   const bool valid = row < rows && (a.active == nullptr || a.active[sol] != 0);
   PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
-  load_axis<N>(S.ax, a.ax);
   __syncthreads();
   const float2* hx_ = a.H + (((long)sol * 2 + 0) * a.ny + j) * a.hx;
   const float2* hy_ = a.H + (((long)sol * 2 + 1) * a.ny + j) * a.hx;

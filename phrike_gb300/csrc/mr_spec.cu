@@ -223,11 +223,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_mrs_x(SpecXArgs a, SpecAxis ax,
   float2* buf = sm + 2 * n;                                                // [nsig][pg][stride]
   float* prim = reinterpret_cast<float*>(buf + (long)nsig * pg * stride);  // 3D fluxes: [NC][pg][n]
   const int row0 = blockIdx.x * pg;
-  // rows of a CTA belong to one solve (rps is a multiple of pg, or pg = 1)
-  const int sol = row0 / a.rps;
-  if (a.active != nullptr && a.active[sol] == 0) return;
   const Tables tb = load_tables(sm, ax);
   cp_commit();
+  dep_wait();
+  // rows of a CTA belong to one solve (rps is a multiple of pg, or pg = 1)
+  const int sol = row0 / a.rps;
+  if (a.active != nullptr && a.active[sol] == 0) {
+    cp_wait<0>();
+    return;
+  }
   const float inv_n = 1.0f / (float)n;
   const float er = a.eref[sol];
   const float eshift = a.shift_in ? er : 0.0f;
@@ -394,12 +398,16 @@ __global__ void __launch_bounds__(MAXT, 1) k_mrs_f(SpecFArgs a, SpecAxis ax, int
   const int stride = ax.len << lt;
   float2* buf = sm;
   const int plane = blockIdx.y, col0 = blockIdx.x * T;
-  if (a.active != nullptr && a.active[plane / a.pps] == 0) return;
+  const Tables tb = load_tables(buf + 2 * stride, ax);
+  dep_wait();
+  if (a.active != nullptr && a.active[plane / a.pps] == 0) {
+    cp_wait<0>();
+    return;
+  }
   const float2* in = a.G + (long)plane * n * a.pitch;
   auto same = [&](int i) { return elem_of_point(ax, i); };
   tile_in(buf, lt, n, in, a.pitch, col0, a.ncol, same);
   tile_in(buf + stride, lt, n, in + a.gs, a.pitch, col0, a.ncol, same);
-  const Tables tb = load_tables(buf + 2 * stride, ax);
   cp_commit();
   cp_wait<0>();
   forward<false>(Lay{buf, stride, 2, lt}, ax, tb.tw);
@@ -435,12 +443,16 @@ __global__ void __launch_bounds__(MAXT, 1) k_mrs_c(SpecCArgs a, SpecAxis ax, int
   const int stride = ax.len << lt;
   float2* buf = sm;
   const int outer = blockIdx.y % a.nouter, sol = blockIdx.y / a.nouter, col0 = blockIdx.x * T;
-  if (a.active != nullptr && a.active[sol] == 0) return;
+  const Tables tb = load_tables(buf + 2 * stride, ax);
+  dep_wait();
+  if (a.active != nullptr && a.active[sol] == 0) {
+    cp_wait<0>();
+    return;
+  }
   const long base = (long)sol * a.ss + (long)outer * a.os;
   auto same = [&](int i) { return elem_of_point(ax, i); };
   tile_in(buf, lt, n, a.a + base, a.as, col0, a.ncol, same);
   tile_in(buf + stride, lt, n, a.b + base, a.as, col0, a.ncol, same);
-  const Tables tb = load_tables(buf + 2 * stride, ax);
   cp_commit();
   const float dt = (a.dt_dev != nullptr) ? (float)a.dt_dev[sol] : (float)a.dt;
   const RKCoef rk = rk_coef(a.stage, dt, a.rk2);
@@ -494,10 +506,14 @@ __global__ void __launch_bounds__(MAXT, 1) k_mrs_i(SpecIArgs a, SpecAxis ax, int
   const int T = 1 << lt, n = ax.n, M = 2 * ax.km + 1;
   float2* buf = sm;
   const int plane = blockIdx.y, col0 = blockIdx.x * T;
-  if (a.active != nullptr && a.active[plane / a.pps] == 0) return;
+  const Tables tb = load_tables(buf + (ax.len << lt), ax);
+  dep_wait();
+  if (a.active != nullptr && a.active[plane / a.pps] == 0) {
+    cp_wait<0>();
+    return;
+  }
   tile_in(buf, lt, M, a.in + (long)plane * M * a.pitch, a.pitch, col0, a.ncol,
           [&](int m) { return elem_of_mode(ax, mode_of(ax, m)); });
-  const Tables tb = load_tables(buf + (ax.len << lt), ax);
   cp_commit();
   for (int e = threadIdx.x; e < (n - M) << lt; e += blockDim.x)  // masked modes
     buf[(elem_of_mode(ax, ax.km + 1 + (e >> lt)) << lt) + (e & (T - 1))] = make_float2(0.0f, 0.0f);
@@ -521,8 +537,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_mrs_filter(MrFilterArgs a, Spec
   const int stride = ROWS ? ax.len : ax.len << lt;
   float2* buf = sm + 2 * n;
   const int sol = blockIdx.y;
-  if (a.active != nullptr && a.active[sol] == 0) return;
   const Tables tb = load_tables(sm, ax);
+  dep_wait();
+  if (a.active != nullptr && a.active[sol] == 0) {
+    cp_wait<0>();
+    return;
+  }
   const long j0 = (long)blockIdx.x * T;  // first pencil
   const float inv_n = 1.0f / (float)n;
   const int fa = 2 * blockIdx.z;         // field pair of this CTA
@@ -712,8 +732,7 @@ cudaError_t mrs_x(const SpecXArgs& a, const SpecAxis& ax, cudaStream_t s) {
   const size_t sm = x_bytes(ND, ax.n, ax.len, pg, FLUX);
   cudaError_t e;
   if ((e = set_smem(k_mrs_x<ND, INC, FLUX>, kSmemMax)) != cudaSuccess) return e;
-  k_mrs_x<ND, INC, FLUX><<<a.rows / pg, threads_for((long)nsig * pg * (ax.n / rmax)), sm, s>>>(a, ax, pg);
-  return cudaGetLastError();
+  return launch_dep(k_mrs_x<ND, INC, FLUX>, a.rows / pg, threads_for((long)nsig * pg * (ax.n / rmax)), sm, s, a, ax, pg);
 }
 }  // namespace
 
@@ -738,12 +757,10 @@ cudaError_t launch_mrs_x(int nd, bool inc, bool flux, const SpecXArgs& a, const 
     cudaError_t e;                                                                             \
     if (threads > kThreads) {                                                                  \
       if ((e = set_smem(KERNEL<kWide>, kSmemMax)) != cudaSuccess) return e;                    \
-      KERNEL<kWide><<<grid, threads, sm, s>>>(a, ax, lt);                                      \
-    } else {                                                                                   \
-      if ((e = set_smem(KERNEL<kThreads>, kSmemMax)) != cudaSuccess) return e;                 \
-      KERNEL<kThreads><<<grid, threads, sm, s>>>(a, ax, lt);                                   \
+      return launch_dep(KERNEL<kWide>, grid, threads, sm, s, a, ax, lt);                       \
     }                                                                                          \
-    return cudaGetLastError();                                                                 \
+    if ((e = set_smem(KERNEL<kThreads>, kSmemMax)) != cudaSuccess) return e;                   \
+    return launch_dep(KERNEL<kThreads>, grid, threads, sm, s, a, ax, lt);                      \
   }
 PS_MRS_STRIDED(launch_mrs_f, SpecFArgs, k_mrs_f, 2, a.planes)
 PS_MRS_STRIDED(launch_mrs_c, SpecCArgs, k_mrs_c, 2, a.nouter * a.nsolve)
@@ -762,15 +779,13 @@ cudaError_t launch_mrs_filter(const MrFilterArgs& a, const SpecAxis& ax, int nso
       ++lt;
     sm = bytes(lt);
     if ((e = set_smem(k_mrs_filter<true>, kSmemMax)) != cudaSuccess) return e;
-    k_mrs_filter<true><<<dim3((unsigned)((a.npen + (1 << lt) - 1) >> lt), nsolve, pairs),
-                         threads_for((long)(ax.n / rmax) << lt), sm, s>>>(a, ax, lt);
-  } else {
-    lt = strided_lt(ax, 1, a.npen, (long)pairs * nsolve, &sm);
-    if ((e = set_smem(k_mrs_filter<false>, kSmemMax)) != cudaSuccess) return e;
-    k_mrs_filter<false><<<dim3((unsigned)((a.npen + (1 << lt) - 1) >> lt), nsolve, pairs),
-                          threads_for((long)(ax.n / rmax) << lt), sm, s>>>(a, ax, lt);
+    return launch_dep(k_mrs_filter<true>, dim3((unsigned)((a.npen + (1 << lt) - 1) >> lt), nsolve, pairs),
+                      threads_for((long)(ax.n / rmax) << lt), sm, s, a, ax, lt);
   }
-  return cudaGetLastError();
+  lt = strided_lt(ax, 1, a.npen, (long)pairs * nsolve, &sm);
+  if ((e = set_smem(k_mrs_filter<false>, kSmemMax)) != cudaSuccess) return e;
+  return launch_dep(k_mrs_filter<false>, dim3((unsigned)((a.npen + (1 << lt) - 1) >> lt), nsolve, pairs),
+                    threads_for((long)(ax.n / rmax) << lt), sm, s, a, ax, lt);
 }
 
 }  // namespace ps

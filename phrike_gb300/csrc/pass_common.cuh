@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "dep.cuh"
 #include "fft_pencil.cuh"
 
 namespace ps {

@@ -655,6 +655,8 @@ __global__ void __launch_bounds__(Shape<N>::A * T, tma_min_blocks<N, T>())
   const int col = blockIdx.x * T + p;
   const int sol = blockIdx.y / a.g.nouter;
   const int outer = blockIdx.y % a.g.nouter;
+  load_axis<N>(S.ax, a.ax);
+  dep_wait();
   if (a.active != nullptr && a.active[sol] == 0) return;
   const bool valid = col < a.g.ncol;
   PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
@@ -663,7 +665,6 @@ __global__ void __launch_bounds__(Shape<N>::A * T, tma_min_blocks<N, T>())
     for (int f = 0; f < a.nf; ++f) S.ring.sched[f] = f;
     S.ring.ntiles = a.nf;
   }
-  load_axis<N>(S.ax, a.ax);
   __syncthreads();
   const MapSet maps{&mIn, &mIn, &mIn};
   RingCursor<N, T, R> rc{S.ring, maps, TileIssue{a.axis, (int)(blockIdx.x * T), outer, sol * a.nf, 0, 0},

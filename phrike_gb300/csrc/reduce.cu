@@ -198,12 +198,14 @@ __global__ void k_flux1d(const float* __restrict__ U, long n, float gamma, float
 
 // E_ref of the energy-perturbation form: the energy of each solve's first cell.
 __global__ void k_eref_set(const float* E, long ss, int nsolve, float* eref) {
+  dep_wait();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s < nsolve) eref[s] = E[(long)s * ss];
 }
 
 // E <- E + sign * E_ref[solve] (sign -1: to perturbation form, +1: back)
 __global__ void k_energy_shift(float* E, long n, long ss, const float* eref, float sign) {
+  dep_wait();
   const float s = sign * eref[blockIdx.y];
   E += (long)blockIdx.y * ss;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) E[i] += s;
@@ -213,6 +215,7 @@ __global__ void k_energy_shift(float* E, long n, long ss, const float* eref, flo
 // active = t < t_end - 1e-12; dt = active ? min(cfl h / speed, t_end - t) : 0.
 __global__ void k_step_control(const float* speed, double cfl, double hmin, const double* t, const double* tend,
                                int nsolve, double* dt, int* active, double dt_cap) {
+  dep_wait();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nsolve) return;
   const bool on = t[s] < tend[s] - 1e-12;
@@ -228,6 +231,7 @@ __global__ void k_step_control(const float* speed, double cfl, double hmin, cons
 // the speed maxima for the next step.
 __global__ void k_step_advance(double* t, const double* dt, float* speed, const int* active, int* steps,
                                int nsolve) {
+  dep_wait();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nsolve) return;
   t[s] += dt[s];
@@ -236,38 +240,34 @@ __global__ void k_step_advance(double* t, const double* dt, float* speed, const 
 }
 
 __global__ void k_fill_int(int* a, int n, int v) {
+  dep_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) a[i] = v;
 }
 
 cudaError_t launch_fill_int(int* a, int n, int v, cudaStream_t s) {
-  k_fill_int<<<(n + 127) / 128, 128, 0, s>>>(a, n, v);
-  return cudaGetLastError();
+  return launch_dep(k_fill_int, (n + 127) / 128, 128, 0, s, a, n, v);
 }
 
 cudaError_t launch_eref_set(const float* E, long ss, int nsolve, float* eref, cudaStream_t s) {
-  k_eref_set<<<(nsolve + 127) / 128, 128, 0, s>>>(E, ss, nsolve, eref);
-  return cudaGetLastError();
+  return launch_dep(k_eref_set, (nsolve + 127) / 128, 128, 0, s, E, ss, nsolve, eref);
 }
 
 cudaError_t launch_energy_shift(float* E, long n, long ss, int nsolve, const float* eref, float sign,
                                 cudaStream_t s) {
   const long want = (n + 255) / 256;
   const int blocks = (int)(want < 1024 ? want : 1024);
-  k_energy_shift<<<dim3(blocks, nsolve), 256, 0, s>>>(E, n, ss, eref, sign);
-  return cudaGetLastError();
+  return launch_dep(k_energy_shift, dim3(blocks, nsolve), 256, 0, s, E, n, ss, eref, sign);
 }
 
 cudaError_t launch_step_control(const float* speed, double cfl, double hmin, const double* t, const double* tend,
                                 int nsolve, double* dt, int* active, cudaStream_t s, double dt_cap) {
-  k_step_control<<<(nsolve + 127) / 128, 128, 0, s>>>(speed, cfl, hmin, t, tend, nsolve, dt, active, dt_cap);
-  return cudaGetLastError();
+  return launch_dep(k_step_control, (nsolve + 127) / 128, 128, 0, s, speed, cfl, hmin, t, tend, nsolve, dt, active, dt_cap);
 }
 
 cudaError_t launch_step_advance(double* t, const double* dt, float* speed, const int* active, int* steps,
                                 int nsolve, cudaStream_t s) {
-  k_step_advance<<<(nsolve + 127) / 128, 128, 0, s>>>(t, dt, speed, active, steps, nsolve);
-  return cudaGetLastError();
+  return launch_dep(k_step_advance, (nsolve + 127) / 128, 128, 0, s, t, dt, speed, active, steps, nsolve);
 }
 
 static int reduce_blocks(long cells, int nsolve) {

@@ -27,8 +27,7 @@ cudaError_t spec_x_T(const SpecXArgs& a, cudaStream_t s) {
   const size_t sm = sizeof(SpecXSmem<NN, T>);
   cudaError_t e;
   if ((e = set_smem(k_spec_x<NN, T, ND, PHYS, INC, FLUX>, sm)) != cudaSuccess) return e;
-  k_spec_x<NN, T, ND, PHYS, INC, FLUX><<<(a.rows + T - 1) / T, Shape<NN>::A * T, sm, s>>>(a);
-  return cudaGetLastError();
+  return launch_dep(k_spec_x<NN, T, ND, PHYS, INC, FLUX>, (a.rows + T - 1) / T, Shape<NN>::A * T, sm, s, a);
 }
 template <int NN, int T, int ND, int PHYS>
 cudaError_t spec_x_mode(bool inc, bool flux, const SpecXArgs& a, cudaStream_t s) {
@@ -67,8 +66,7 @@ cudaError_t spec_grid(K kernel, int threads, size_t sm, long items, int* grid) {
       auto* k = KERNEL<NN, T>;                                                                        \
       const long items = (long)((a.ncol + T - 1) / T) * (OUTER);                                      \
       if ((e = spec_grid<NN, T>(k, Shape<NN>::A * T, sm, items, &grid)) != cudaSuccess) return e;     \
-      KERNEL<NN, T><<<grid, Shape<NN>::A * T, sm, s>>>(a);                                            \
-      return cudaGetLastError();                                                                      \
+      return launch_dep(k, grid, Shape<NN>::A * T, sm, s, a);                                         \
     });                                                                                               \
   }
 #define PS_DEFINE_SPEC_LAUNCHERS(NN)                                                                  \

@@ -126,6 +126,8 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_spec_x(SpecXArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto& S = *reinterpret_cast<SpecXSmem<N, T>*>(smem_raw);
 
+  load_axis<N>(S.ax, a.ax);
+  dep_wait();
   const int t = threadIdx.x % A;
   const int p = threadIdx.x / A;
   const int row = blockIdx.x * T + p;
@@ -139,7 +141,6 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_spec_x(SpecXArgs a) {
     if (!any) return;
   }
   PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
-  load_axis<N>(S.ax, a.ax);
   const long rbase = (long)sol * a.ssU + (long)(row % a.rps) * N + t;
   const float er = (PHYS == 0) ? a.eref[sol] : 0.0f;
   const float eshift = a.shift_in ? er : 0.0f;
@@ -470,6 +471,8 @@ __global__ void __launch_bounds__(Shape<N>::A * T, spec_min_blocks<N, T>()) k_sp
   using PF = Pencil<N, T, true>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto& S = *reinterpret_cast<SpecPairSmem<N, T>*>(smem_raw);
+  load_axis<N>(S.ax, a.ax);
+  dep_wait();
   const int p = threadIdx.x % T, t = threadIdx.x / T;
   PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
   const int ctiles = (a.ncol + T - 1) / T;
@@ -490,7 +493,6 @@ __global__ void __launch_bounds__(Shape<N>::A * T, spec_min_blocks<N, T>()) k_sp
   int s = 0;  // slot of the item's first tile
   fetch(0, w, 0);
   fetch(1, w, 1);
-  load_axis<N>(S.ax, a.ax);
   while (w < items) {
     const int col = (w % ctiles) * T + p;
     const bool valid = col < a.ncol;
@@ -564,6 +566,8 @@ __global__ void __launch_bounds__(Shape<N>::A * T, spec_min_blocks<N, T>()) k_sp
   using PF = Pencil<N, T, true>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto& S = *reinterpret_cast<SpecPairSmem<N, T>*>(smem_raw);
+  load_axis<N>(S.ax, a.ax);
+  dep_wait();
   const int p = threadIdx.x % T, t = threadIdx.x / T;
   PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
   const int ctiles = (a.ncol + T - 1) / T;
@@ -587,7 +591,6 @@ __global__ void __launch_bounds__(Shape<N>::A * T, spec_min_blocks<N, T>()) k_sp
   };
   int w = next(blockIdx.x);
   fetch(w);
-  load_axis<N>(S.ax, a.ax);
   while (w < items) {
     const int col = (w % ctiles) * T + p;
     const int outer = w / ctiles % a.nouter, sol = w / ctiles / a.nouter;
@@ -663,6 +666,8 @@ __global__ void __launch_bounds__(Shape<N>::A * T, spec_min_blocks<N, T>()) k_sp
   using PF = Pencil<N, T, true>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto& S = *reinterpret_cast<SpecISmem<N, T>*>(smem_raw);
+  load_axis<N>(S.ax, a.ax);
+  dep_wait();
   const int p = threadIdx.x % T, t = threadIdx.x / T;
   PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
   const int ctiles = (a.ncol + T - 1) / T;
@@ -679,7 +684,6 @@ __global__ void __launch_bounds__(Shape<N>::A * T, spec_min_blocks<N, T>()) k_sp
   };
   int w = next(blockIdx.x);
   fetch(w);
-  load_axis<N>(S.ax, a.ax);
   while (w < items) {
     const int col = (w % ctiles) * T + p;
     const int wn = next(w + gridDim.x);
