@@ -36,6 +36,21 @@ cudaError_t spec_x_mode(bool inc, bool flux, const SpecXArgs& a, cudaStream_t s)
   return spec_x_T<NN, T, ND, PHYS, false, true>(a, s);
 }
 
+template <int NN, int ND, int PHYS, bool INC, bool FLUX>
+cudaError_t spec_xs(const SpecXArgs& a, cudaStream_t s) {
+  constexpr int T = 32 / Shape<NN>::A, NG = SpecXsGroups<ND, PHYS>::value, NC = (PHYS == 1) ? 8 : ND + 2;
+  const size_t sm = sizeof(SpecXsSmem<NN, T, NC, NG>);
+  cudaError_t e;
+  if ((e = set_smem(k_spec_xs<NN, ND, PHYS, INC, FLUX>, sm)) != cudaSuccess) return e;
+  return launch_dep(k_spec_xs<NN, ND, PHYS, INC, FLUX>, (a.rows + T - 1) / T, 32 * NG, sm, s, a);
+}
+template <int NN, int ND, int PHYS>
+cudaError_t spec_xs_mode(bool inc, bool flux, const SpecXArgs& a, cudaStream_t s) {
+  if (inc && flux) return spec_xs<NN, ND, PHYS, true, true>(a, s);
+  if (inc) return spec_xs<NN, ND, PHYS, true, false>(a, s);
+  return spec_xs<NN, ND, PHYS, false, true>(a, s);
+}
+
 // A walking grid: as many CTAs as fit the GPU at once, or one per tile.
 template <int NN, int T, typename K>
 cudaError_t spec_grid(K kernel, int threads, size_t sm, long items, int* grid) {
@@ -74,10 +89,24 @@ cudaError_t spec_grid(K kernel, int threads, size_t sm, long items, int* grid) {
   PS_DEFINE_SPEC_STRIDED(NN, launch_spec_c, SpecCArgs, k_spec_c, SpecPairSmem, (long)a.nouter * a.nsolve) \
   PS_DEFINE_SPEC_STRIDED(NN, launch_spec_i, SpecIArgs, k_spec_i, SpecISmem, (long)a.planes)
 
+// Rows of k_spec_x fill 32 / A pencils per warp; up to eight such warps per SM
+// their chains of 6 to 12 transforms do not overlap enough, and the row's jobs
+// go to several warps (k_spec_xs).  Step times, k_spec_x against k_spec_xs:
+// KHI 128^2 84.1 -> 65.7 us (32 warps), Orszag-Tang 512^2 262 -> 217 us (512),
+// Taylor-Green 64^3 100.0 -> 98.1 us (1024); past the line k_spec_x is the
+// better one: 3D MHD 128^3 1212 against 1222 us (4096), KHI 512^2 x 16 (three
+// CFL steps) 2300 against 2448 us (8192).
+constexpr long kSpecXsWarps = 8 * 152;
+
 // Euler x pass of every length, MHD x pass in a unit of its own
 #define PS_DEFINE_SPEC_X(NN, PHYS)                                                                    \
   template <>                                                                                         \
   cudaError_t launch_spec_x<NN, PHYS>(int nd, bool inc, bool flux, const SpecXArgs& a, cudaStream_t s) { \
+    if constexpr (Shape<NN>::A <= 32)                                                                 \
+      if ((long)a.rows * Shape<NN>::A <= 32 * kSpecXsWarps)  {                                        \
+        if (nd == 2) return spec_xs_mode<NN, 2, PHYS>(inc, flux, a, s);                               \
+        if constexpr (PHYS == 0 || NN <= 256) return spec_xs_mode<NN, 3, PHYS>(inc, flux, a, s);      \
+      }                                                                                               \
     return dispatch_rows<NN>(a.rows, [&](auto tw) -> cudaError_t {                                    \
       constexpr int T = decltype(tw)::value;                                                          \
       if (nd == 3) {                                                                                  \
