@@ -488,6 +488,22 @@ __global__ void __launch_bounds__(32 * SpecXsGroups<ND, PHYS>::value) k_spec_xs(
   const float pref = g1 * er;
   constexpr int CE = (PHYS == 1) ? 4 : NC - 1;
   auto slot = [&](int c, int n2) -> float& { return S.q[c][n2 * 32 + lane]; };
+  // this thread's points in the middle part are n2 = grp + NG i; the stage
+  // projection's change of U^n there is loaded ahead of the transforms
+  constexpr int NPT = (B + NG - 1) / NG;
+  [[maybe_unused]] float dB[NPT][3];
+  if constexpr (INC && PHYS == 1) {
+#pragma unroll
+    for (int i = 0; i < NPT; ++i)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const int n2 = grp + NG * i;
+        const long o = (long)(row % a.rps) * N + t + A * n2;  // within a field
+        dB[i][c] = (a.Bp != nullptr && valid && n2 < B && c < a.nproj)
+                       ? a.Bp[((long)sol * a.nproj + c) * a.fs + o] - a.U[(5 + c) * a.fs + rbase + A * n2]
+                       : 0.0f;
+      }
+  }
   __syncthreads();
 
   // the group's component pairs: U^n (plus the increment, or filtered along x)
@@ -555,8 +571,10 @@ __global__ void __launch_bounds__(32 * SpecXsGroups<ND, PHYS>::value) k_spec_xs(
 
   // points n2 = grp, grp + NG, ..: clamp, new state, primitives
   float smax = 0.0f;
-#pragma unroll 1
-  for (int n2 = grp; n2 < B; n2 += NG) {
+#pragma unroll
+  for (int i = 0; i < NPT; ++i) {
+    const int n2 = grp + NG * i;
+    if (n2 >= B) break;
     float u[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) u[c] = slot(c, n2);
@@ -567,8 +585,7 @@ __global__ void __launch_bounds__(32 * SpecXsGroups<ND, PHYS>::value) k_spec_xs(
 #pragma unroll
           for (int c = 5; c < 8; ++c) {
             if (c - 5 >= a.nproj) break;
-            const long o = (long)(row % a.rps) * N + t + A * n2;  // within a field
-            const float b = u[c] + (a.Bp[((long)sol * a.nproj + c - 5) * a.fs + o] - a.U[c * a.fs + rbase + A * n2]);
+            const float b = u[c] + dB[i][c - 5];
             u[4] += 0.5f * (b * b - u[c] * u[c]);
             u[c] = b;
           }
@@ -818,21 +835,35 @@ __global__ void __launch_bounds__(Shape<N>::A * T, spec_min_blocks<N, T>()) k_sp
     pf.fwd(z2);
     sfor<0, B>([&](auto rc) {
       constexpr int r = decltype(rc)::value;
-      float2 inc = make_float2(0.0f, 0.0f);
       if constexpr (spec_keeps<N>(r)) {
         const int k = pf.kidx(r);
-        const int m = spec_col<N>(k);
+        const float P = -S.ax.P[k], d = -S.ax.d[k];
+        v[r] = make_float2(fmaf(P, v[r].x, -d * z2[r].y), fmaf(P, v[r].y, d * z2[r].x));
+      }
+    });
+    // all of the accumulator's points in flight before the first is used: with
+    // each load behind the previous point's store the thread waited for up to
+    // B cache round trips in turn
+    float2 (&q)[B] = z2;
+    sfor<0, B>([&](auto rc) {
+      constexpr int r = decltype(rc)::value;
+      if constexpr (spec_keeps<N>(r)) {
+        const int m = spec_col<N>(pf.kidx(r));
+        q[r] = (a.stage != 0 && valid && m >= 0) ? acc[m * a.acc_as] : make_float2(0.0f, 0.0f);
+      }
+    });
+    sfor<0, B>([&](auto rc) {
+      constexpr int r = decltype(rc)::value;
+      float2 inc = make_float2(0.0f, 0.0f);
+      if constexpr (spec_keeps<N>(r)) {
+        const int m = spec_col<N>(pf.kidx(r));
         if (m >= 0) {
-          const float P = -S.ax.P[k], d = -S.ax.d[k];
-          const float2 kk = make_float2(fmaf(P, v[r].x, -d * z2[r].y), fmaf(P, v[r].y, d * z2[r].x));
+          q[r] = make_float2(fmaf(rk.wacc, v[r].x, q[r].x), fmaf(rk.wacc, v[r].y, q[r].y));
           if (a.stage == 3) {
-            const float2 q = valid ? acc[m * a.acc_as] : make_float2(0.0f, 0.0f);
-            inc = make_float2(fmaf(rk.wacc, kk.x, q.x), fmaf(rk.wacc, kk.y, q.y));
+            inc = q[r];
           } else {
-            float2 q = make_float2(0.0f, 0.0f);
-            if (a.stage != 0 && valid) q = acc[m * a.acc_as];
-            if (valid) acc[m * a.acc_as] = make_float2(fmaf(rk.wacc, kk.x, q.x), fmaf(rk.wacc, kk.y, q.y));
-            inc = make_float2(rk.wnext * kk.x, rk.wnext * kk.y);
+            if (valid) acc[m * a.acc_as] = q[r];
+            inc = make_float2(rk.wnext * v[r].x, rk.wnext * v[r].y);
           }
         }
       }
