@@ -367,8 +367,9 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_op(OpArgs a) {
   }
   PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
   __syncthreads();
+  // blockIdx.y: share of the field pairs (op_pair_groups)
 #pragma unroll 1
-  for (int c = 0; c < a.nf; c += 2) {
+  for (int c = 2 * blockIdx.y; c < a.nf; c += 2 * gridDim.y) {
     const bool two = c + 1 < a.nf;
     float2 w[B], w0[B];
     load_pair<N>(w, a.in + c * a.fs, two ? a.in + (c + 1) * a.fs : nullptr, base_in, step, valid);

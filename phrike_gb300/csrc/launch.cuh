@@ -135,10 +135,22 @@ cudaError_t last_t_T(int nd, const CUtensorMap& mAB, const CUtensorMap& mU, cons
   return cudaGetLastError();
 }
 
+// Groups the field pairs of an operator pass are split into: a CTA per pair up
+// to four tiles per SM, where the pairs' chain of transforms is what the pass
+// takes.  Steps, whole tiles -> split: KHI 128^2 55.1 -> 51.6 us (filter passes
+// of 8 and 32 CTAs), Taylor-Green 64^3 95.9 -> 92.8 us (256); no gain at 1024
+// (3D MHD 128^3: 1196 us unsplit, 1203 split).
+constexpr long kOpSplitTiles = 4 * 152;
+inline int op_pair_groups(long tiles, int nf) {
+  const int pairs = (nf + 1) / 2;
+  return (tiles >= kOpSplitTiles) ? 1 : (pairs < 32 ? pairs : 32);
+}
+
 template <int NN, int T>
 cudaError_t op_t_T(const CUtensorMap& mIn, const OpTArgs& a, cudaStream_t s) {
   constexpr int R = TmaTile<NN>::R;
-  const dim3 grid((a.g.ncol + T - 1) / T, a.g.nouter * a.nsolve);
+  dim3 grid((a.g.ncol + T - 1) / T, a.g.nouter * a.nsolve);
+  grid.z = op_pair_groups((long)grid.x * grid.y, a.nf);
   const size_t sm = sizeof(TmaStridedSmem<NN, T, R>);
   cudaError_t e;
   if ((e = set_smem(k_op_t<NN, T, R>, sm)) != cudaSuccess) return e;
@@ -222,12 +234,14 @@ cudaError_t dispatch_proj_cols(long units, F&& f) {
   template <>                                                                                         \
   cudaError_t launch_op<NN>(bool strided, const OpArgs& a, cudaStream_t s) {                          \
     if (strided) return cudaErrorInvalidValue; /* strided axes use launch_op_t */                     \
-    constexpr int T = Tile<NN>::TC;                                                                   \
-    const dim3 grid((a.rows + T - 1) / T);                                                            \
-    const size_t sm = sizeof(StridedSmem<NN, T, false>);                                              \
-    cudaError_t e;                                                                                    \
-    if ((e = set_smem(k_op<NN, T, false>, sm)) != cudaSuccess) return e;                              \
-    return launch_dep(k_op<NN, T, false>, grid, Shape<NN>::A * T, sm, s, a);                          \
+    return dispatch_rows<NN>(a.rows, [&](auto tw) -> cudaError_t {                                    \
+      constexpr int T = decltype(tw)::value;                                                          \
+      const int tiles = (a.rows + T - 1) / T;                                                         \
+      const size_t sm = sizeof(StridedSmem<NN, T, false>);                                            \
+      cudaError_t e;                                                                                  \
+      if ((e = set_smem(k_op<NN, T, false>, sm)) != cudaSuccess) return e;                            \
+      return launch_dep(k_op<NN, T, false>, dim3(tiles, op_pair_groups(tiles, a.nf)), Shape<NN>::A * T, sm, s, a); \
+    });                                                                                               \
   }                                                                                                   \
   template <>                                                                                         \
   cudaError_t launch_ymid3_t<NN>(const CUtensorMap& mG, const YMidTArgs& a, cudaStream_t s) {         \

@@ -353,20 +353,21 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_proj_xi(ProjArgs a) {
     }
     z[r] = make_float2(X.x - Y.y, X.y + Y.x);  // X + i Y
   }
+  float* bx = a.Bx + (long)sol * a.ss + (long)j * N;
+  float* by = a.By + (long)sol * a.ss + (long)j * N;
+  float* e = (a.E != nullptr) ? a.E + (long)sol * a.ss + (long)j * N : nullptr;
+  float ox[B], oy[B], oe[B];  // old B and E, in flight during the transform
+#pragma unroll
+  for (int n2 = 0; n2 < B; ++n2) {
+    const int i = t + A * n2;
+    const bool take = valid && e != nullptr;
+    ox[n2] = take ? bx[i] : 0.0f;
+    oy[n2] = take ? by[i] : 0.0f;
+    oe[n2] = take ? e[i] : 0.0f;
+  }
   pf.inv(z);
   if (valid) {
-    float* bx = a.Bx + (long)sol * a.ss + (long)j * N;
-    float* by = a.By + (long)sol * a.ss + (long)j * N;
-    float* e = (a.E != nullptr) ? a.E + (long)sol * a.ss + (long)j * N : nullptr;
-    if (e != nullptr) {  // every old B and E of the row loaded before the first store
-      float ox[B], oy[B], oe[B];
-#pragma unroll
-      for (int n2 = 0; n2 < B; ++n2) {
-        const int i = t + A * n2;
-        ox[n2] = bx[i];
-        oy[n2] = by[i];
-        oe[n2] = e[i];
-      }
+    if (e != nullptr) {
 #pragma unroll
       for (int n2 = 0; n2 < B; ++n2)
         e[t + A * n2] = oe[n2] + 0.5f * ((z[n2].x * z[n2].x + z[n2].y * z[n2].y) - (ox[n2] * ox[n2] + oy[n2] * oy[n2]));

@@ -661,9 +661,14 @@ __global__ void __launch_bounds__(Shape<N>::A * T, tma_min_blocks<N, T>())
   const bool valid = col < a.g.ncol;
   PF pf{p, t, S.buf, S.ax.twf, S.ax.twi};
   ring_init(S.ring);
+  // blockIdx.z: share of the field pairs (op_pair_groups)
   if (threadIdx.x == 0) {
-    for (int f = 0; f < a.nf; ++f) S.ring.sched[f] = f;
-    S.ring.ntiles = a.nf;
+    int n = 0;
+    for (int f = 2 * blockIdx.z; f < a.nf; f += 2 * gridDim.z) {
+      S.ring.sched[n++] = f;
+      if (f + 1 < a.nf) S.ring.sched[n++] = f + 1;
+    }
+    S.ring.ntiles = n;
   }
   __syncthreads();
   const MapSet maps{&mIn, &mIn, &mIn};
@@ -675,7 +680,7 @@ __global__ void __launch_bounds__(Shape<N>::A * T, tma_min_blocks<N, T>())
   const bool comp = a.complement && !a.deriv;
   int ti = 0;
 #pragma unroll 1
-  for (int c = 0; c < a.nf; c += 2) {
+  for (int c = 2 * blockIdx.z; c < a.nf; c += 2 * gridDim.z) {
     const bool two = c + 1 < a.nf;
     float2 w[B], w0[B];
     tile_pair<N, T>(w, rc.wait(ti), two ? rc.wait(ti + 1) : nullptr, t, p);
