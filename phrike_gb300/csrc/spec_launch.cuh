@@ -22,35 +22,6 @@ cudaError_t dispatch_spec_cols(int ncol, long outer, F&& f) {
   return f(std::integral_constant<int, TMIN>{});
 }
 
-template <int NN, int T, int ND, int PHYS, bool INC, bool FLUX>
-cudaError_t spec_x_T(const SpecXArgs& a, cudaStream_t s) {
-  const size_t sm = sizeof(SpecXSmem<NN, T>);
-  cudaError_t e;
-  if ((e = set_smem(k_spec_x<NN, T, ND, PHYS, INC, FLUX>, sm)) != cudaSuccess) return e;
-  return launch_dep(k_spec_x<NN, T, ND, PHYS, INC, FLUX>, (a.rows + T - 1) / T, Shape<NN>::A * T, sm, s, a);
-}
-template <int NN, int T, int ND, int PHYS>
-cudaError_t spec_x_mode(bool inc, bool flux, const SpecXArgs& a, cudaStream_t s) {
-  if (inc && flux) return spec_x_T<NN, T, ND, PHYS, true, true>(a, s);
-  if (inc) return spec_x_T<NN, T, ND, PHYS, true, false>(a, s);
-  return spec_x_T<NN, T, ND, PHYS, false, true>(a, s);
-}
-
-template <int NN, int ND, int PHYS, bool INC, bool FLUX>
-cudaError_t spec_xs(const SpecXArgs& a, cudaStream_t s) {
-  constexpr int T = 32 / Shape<NN>::A, NG = SpecXsGroups<ND, PHYS>::value, NC = (PHYS == 1) ? 8 : ND + 2;
-  const size_t sm = sizeof(SpecXsSmem<NN, T, NC, NG>);
-  cudaError_t e;
-  if ((e = set_smem(k_spec_xs<NN, ND, PHYS, INC, FLUX>, sm)) != cudaSuccess) return e;
-  return launch_dep(k_spec_xs<NN, ND, PHYS, INC, FLUX>, (a.rows + T - 1) / T, 32 * NG, sm, s, a);
-}
-template <int NN, int ND, int PHYS>
-cudaError_t spec_xs_mode(bool inc, bool flux, const SpecXArgs& a, cudaStream_t s) {
-  if (inc && flux) return spec_xs<NN, ND, PHYS, true, true>(a, s);
-  if (inc) return spec_xs<NN, ND, PHYS, true, false>(a, s);
-  return spec_xs<NN, ND, PHYS, false, true>(a, s);
-}
-
 // A walking grid: as many CTAs as fit the GPU at once, or one per tile.
 template <int NN, int T, typename K>
 cudaError_t spec_grid(K kernel, int threads, size_t sm, long items, int* grid) {
@@ -67,6 +38,40 @@ cudaError_t spec_grid(K kernel, int threads, size_t sm, long items, int* grid) {
   }
   *grid = (int)(items < resident ? items : resident);
   return cudaSuccess;
+}
+
+template <int NN, int T, int ND, int PHYS, bool INC, bool FLUX>
+cudaError_t spec_x_T(const SpecXArgs& a, cudaStream_t s) {
+  const size_t sm = sizeof(SpecXSmem<NN, T>);
+  cudaError_t e;
+  if ((e = set_smem(k_spec_x<NN, T, ND, PHYS, INC, FLUX>, sm)) != cudaSuccess) return e;
+  return launch_dep(k_spec_x<NN, T, ND, PHYS, INC, FLUX>, (a.rows + T - 1) / T, Shape<NN>::A * T, sm, s, a);
+}
+template <int NN, int T, int ND, int PHYS>
+cudaError_t spec_x_mode(bool inc, bool flux, const SpecXArgs& a, cudaStream_t s) {
+  if (inc && flux) return spec_x_T<NN, T, ND, PHYS, true, true>(a, s);
+  if (inc) return spec_x_T<NN, T, ND, PHYS, true, false>(a, s);
+  return spec_x_T<NN, T, ND, PHYS, false, true>(a, s);
+}
+
+template <int NN, int ND, int PHYS, bool INC, bool FLUX>
+cudaError_t spec_xs(const SpecXArgs& a, cudaStream_t s) {
+  constexpr int T = 32 / Shape<NN>::A, NG = (ND == 3 && PHYS == 0) ? 3 : 4, NC = (PHYS == 1) ? 8 : ND + 2;
+  const size_t sm = sizeof(SpecXsSmem<NN, T, NC, NG>);
+  auto* k = k_spec_xs<NN, ND, PHYS, NG, INC, FLUX>;
+  cudaError_t e;
+  int grid = (a.rows + T - 1) / T;
+  if ((e = set_smem(k, sm)) != cudaSuccess) return e;
+  if (PHYS == 1 &&  // these kernels walk over their tiles
+      (e = spec_grid<NN, (PHYS * 4 + ND) * 4 + INC * 2 + FLUX>(k, 32 * NG, sm, grid, &grid)) != cudaSuccess)
+    return e;
+  return launch_dep(k, grid, 32 * NG, sm, s, a);
+}
+template <int NN, int ND, int PHYS>
+cudaError_t spec_xs_mode(bool inc, bool flux, const SpecXArgs& a, cudaStream_t s) {
+  if (inc && flux) return spec_xs<NN, ND, PHYS, true, true>(a, s);
+  if (inc) return spec_xs<NN, ND, PHYS, true, false>(a, s);
+  return spec_xs<NN, ND, PHYS, false, true>(a, s);
 }
 
 #define PS_DEFINE_SPEC_STRIDED(NN, NAME, ARGS, KERNEL, SMEM, OUTER)                                   \
@@ -89,32 +94,36 @@ cudaError_t spec_grid(K kernel, int threads, size_t sm, long items, int* grid) {
   PS_DEFINE_SPEC_STRIDED(NN, launch_spec_c, SpecCArgs, k_spec_c, SpecPairSmem, (long)a.nouter * a.nsolve) \
   PS_DEFINE_SPEC_STRIDED(NN, launch_spec_i, SpecIArgs, k_spec_i, SpecISmem, (long)a.planes)
 
-// Rows of k_spec_x fill 32 / A pencils per warp; up to eight such warps per SM
-// their chains of 6 to 12 transforms do not overlap enough, and the row's jobs
-// go to several warps (k_spec_xs).  Step times, k_spec_x against k_spec_xs:
-// KHI 128^2 84.1 -> 65.7 us (32 warps), Orszag-Tang 512^2 262 -> 217 us (512),
-// Taylor-Green 64^3 100.0 -> 98.1 us (1024); past the line k_spec_x is the
-// better one: 3D MHD 128^3 1212 against 1222 us (4096), KHI 512^2 x 16 (three
-// CFL steps) 2300 against 2448 us (8192).
+// Euler rows of k_spec_x fill 32 / A pencils per warp; up to eight such warps
+// per SM their chains of 6 to 12 transforms do not overlap enough, and the jobs
+// of a row go to several warps (k_spec_xs).  Step times, k_spec_x against
+// k_spec_xs: KHI 128^2 84.1 -> 65.7 us (32 warps), Taylor-Green 64^3 94.9 ->
+// 92.8 us (1024); past the line k_spec_x is the better one: KHI 512^2 x 16,
+// three CFL steps, 2300 against 2448 us (8192).  MHD rows up to 512 points
+// always take k_spec_xs: Orszag-Tang 512^2 249 -> 183 us (512 warps), 3D MHD
+// 128^3 1184 -> 1056 us (4096).
 constexpr long kSpecXsWarps = 8 * 152;
 
 // Euler x pass of every length, MHD x pass in a unit of its own
 #define PS_DEFINE_SPEC_X(NN, PHYS)                                                                    \
   template <>                                                                                         \
   cudaError_t launch_spec_x<NN, PHYS>(int nd, bool inc, bool flux, const SpecXArgs& a, cudaStream_t s) { \
-    if constexpr (Shape<NN>::A <= 32)                                                                 \
-      if ((long)a.rows * Shape<NN>::A <= 32 * kSpecXsWarps)  {                                        \
-        if (nd == 2) return spec_xs_mode<NN, 2, PHYS>(inc, flux, a, s);                               \
-        if constexpr (PHYS == 0 || NN <= 256) return spec_xs_mode<NN, 3, PHYS>(inc, flux, a, s);      \
-      }                                                                                               \
-    return dispatch_rows<NN>(a.rows, [&](auto tw) -> cudaError_t {                                    \
-      constexpr int T = decltype(tw)::value;                                                          \
-      if (nd == 3) {                                                                                  \
-        if constexpr (PHYS == 1 && NN > 256) return cudaErrorInvalidValue; /* 3D MHD: 8..256 */       \
-        else return spec_x_mode<NN, T, 3, PHYS>(inc, flux, a, s);                                     \
-      }                                                                                               \
-      return spec_x_mode<NN, T, 2, PHYS>(inc, flux, a, s);                                            \
-    });                                                                                               \
+    constexpr bool few = Shape<NN>::A <= 32; /* a warp holds a pencil */                              \
+    if constexpr (few && PHYS == 1) {                                                                 \
+      if (nd == 2) return spec_xs_mode<NN, 2, 1>(inc, flux, a, s);                                    \
+      if constexpr (NN <= 256) return spec_xs_mode<NN, 3, 1>(inc, flux, a, s); /* 3D MHD: 8..256 */   \
+      return cudaErrorInvalidValue;                                                                   \
+    } else {                                                                                          \
+      if constexpr (few)                                                                              \
+        if ((long)a.rows * Shape<NN>::A <= 32 * kSpecXsWarps)                                         \
+          return nd == 2 ? spec_xs_mode<NN, 2, 0>(inc, flux, a, s) : spec_xs_mode<NN, 3, 0>(inc, flux, a, s); \
+      return dispatch_rows<NN>(a.rows, [&](auto tw) -> cudaError_t {                                  \
+        constexpr int T = decltype(tw)::value;                                                        \
+        if (nd == 2) return spec_x_mode<NN, T, 2, PHYS>(inc, flux, a, s);                             \
+        if constexpr (PHYS == 0) return spec_x_mode<NN, T, 3, PHYS>(inc, flux, a, s);                 \
+        else return cudaErrorInvalidValue;                                                            \
+      });                                                                                             \
+    }                                                                                                 \
   }
 
 }  // namespace ps

@@ -143,10 +143,11 @@ __device__ __forceinline__ float spec_primitive(float (&u)[NC], float gamma, flo
   }
 }
 
-// Largest speed of the CTA's T rows into their solves' slots (all threads)
-__device__ __forceinline__ void spec_speed(const SpecXArgs& a, float smax, bool valid, int sol, int T, float* red) {
-  const int s0 = (blockIdx.x * T) / a.rps;
-  const int s1 = (min((int)(blockIdx.x * T + T), a.rows) - 1) / a.rps;
+// Largest speed of a tile's T rows into their solves' slots (all threads)
+__device__ __forceinline__ void spec_speed(const SpecXArgs& a, float smax, bool valid, int sol, int tile, int T,
+                                           float* red) {
+  const int s0 = (tile * T) / a.rps;
+  const int s1 = (min(tile * T + T, a.rows) - 1) / a.rps;
   if (s0 == s1) {
     const float m = block_max(smax, red);
     if (threadIdx.x == 0) atomic_max_nonneg(a.speed + s0, m);
@@ -155,13 +156,15 @@ __device__ __forceinline__ void spec_speed(const SpecXArgs& a, float smax, bool 
   }
 }
 
-// Flux jobs first, first + step, .. of a row whose primitives are q: fluxes of
-// a component pair along one direction, forward transform, D_x or P_x, store.
-template <int N, int T, int ND, int PHYS, int NC, typename PF>
+// Flux jobs first, first + step, .. of a row whose primitives are q(c, n2):
+// fluxes of a component pair along one direction, forward transform, D_x or
+// P_x, store.  opaque() keeps the compiler from carrying flux terms over the
+// jobs.
+template <int N, int T, int ND, int PHYS, typename PF, typename Q, typename O>
 __device__ __forceinline__ void spec_fluxes(const SpecXArgs& a, const PF& pf, const AxisSmem<N>& ax,
-                                            float (&q)[NC][Shape<N>::B], float er, int row, bool valid, int first,
-                                            int step) {
+                                            Q&& q, O&& opaque, float er, int row, bool valid, int first, int step) {
   constexpr int B = Shape<N>::B;
+  constexpr int NC = (PHYS == 1) ? 8 : ND + 2;
   constexpr int NP = NC / 2;
   constexpr bool ODD = (NC % 2) != 0;
   constexpr int NJ = NP + (ODD ? 1 : 0);
@@ -181,20 +184,20 @@ __device__ __forceinline__ void spec_fluxes(const SpecXArgs& a, const PF& pf, co
   // 139 us at 128^3, and take the direction at compile time).
   auto flux_pair = [&](auto jc, int dir, int n2) -> float2 {
     constexpr int c = 2 * decltype(jc)::value;
-    const float un = (dir == 0) ? q[1][n2] : (ND == 2 || dir == 1) ? q[2][n2] : q[(ND == 3) ? 3 : 2][n2];
-    const float mn = q[0][n2] * un;
+    const float un = (dir == 0) ? q(1, n2) : (ND == 2 || dir == 1) ? q(2, n2) : q((ND == 3) ? 3 : 2, n2);
+    const float mn = q(0, n2) * un;
     auto comp = [&](auto cc) -> float {
       constexpr int C = decltype(cc)::value;
-      const float pr = q[NC - 1][n2];
+      const float pr = q(NC - 1, n2);
       if constexpr (C == 0) return mn;
       if constexpr (C == NC - 1) {
         float kin = 0.0f;
 #pragma unroll
-        for (int d = 0; d < ND; ++d) kin = fmaf(q[1 + d][n2], q[1 + d][n2], kin);
-        const float Ep = fmaf(pr, ig1, 0.5f * q[0][n2] * kin);  // E' = E - E_ref
+        for (int d = 0; d < ND; ++d) kin = fmaf(q(1 + d, n2), q(1 + d, n2), kin);
+        const float Ep = fmaf(pr, ig1, 0.5f * q(0, n2) * kin);  // E' = E - E_ref
         return ((Ep + pr) + href) * un;                         // (E + p) u_dir
       }
-      return mn * q[C][n2] + ((C - 1 == dir) ? pr : 0.0f);
+      return mn * q(C, n2) + ((C - 1 == dir) ? pr : 0.0f);
     };
     float2 f = make_float2(comp(std::integral_constant<int, c>{}), 0.0f);
     if constexpr (c + 1 < NC) f.y = comp(std::integral_constant<int, c + 1>{});
@@ -202,13 +205,7 @@ __device__ __forceinline__ void spec_fluxes(const SpecXArgs& a, const PF& pf, co
   };
 #pragma unroll 1
   for (int job = first; job < ND * NJ; job += step) {
-    // the state's registers are opaque per job: without this the compiler
-    // keeps flux terms shared by several jobs live across the loop (16
-    // registers each) and spills
-#pragma unroll
-    for (int c = 0; c < NC; ++c)
-#pragma unroll
-      for (int n2 = 0; n2 < B; ++n2) asm volatile("" : "+f"(q[c][n2]));
+    opaque();
     const int dir = job / NJ, j = job % NJ;
     float2 v[B];
     if constexpr (PHYS == 1) {
@@ -218,13 +215,13 @@ __device__ __forceinline__ void spec_fluxes(const SpecXArgs& a, const PF& pf, co
         if (job == J) {
 #pragma unroll
           for (int n2 = 0; n2 < B; ++n2) {
-            const float b2 = q[5][n2] * q[5][n2] + q[6][n2] * q[6][n2] + q[7][n2] * q[7][n2];
-            const float v2 = q[1][n2] * q[1][n2] + q[2][n2] * q[2][n2] + q[3][n2] * q[3][n2];
-            const float ps = g1 * (q[4][n2] - 0.5f * q[0][n2] * v2 - 0.5f * b2) + 0.5f * b2;
-            const float ub = q[1][n2] * q[5][n2] + q[2][n2] * q[6][n2] + q[3][n2] * q[7][n2];
+            const float b2 = q(5, n2) * q(5, n2) + q(6, n2) * q(6, n2) + q(7, n2) * q(7, n2);
+            const float v2 = q(1, n2) * q(1, n2) + q(2, n2) * q(2, n2) + q(3, n2) * q(3, n2);
+            const float ps = g1 * (q(4, n2) - 0.5f * q(0, n2) * v2 - 0.5f * b2) + 0.5f * b2;
+            const float ub = q(1, n2) * q(5, n2) + q(2, n2) * q(6, n2) + q(3, n2) * q(7, n2);
             auto f = [&](auto cc) {
-              return mhd3_flux<DIR, decltype(cc)::value>(q[0][n2], q[1][n2], q[2][n2], q[3][n2], ps, q[4][n2] + ps,
-                                                         ub, q[5][n2], q[6][n2], q[7][n2]);
+              return mhd3_flux<DIR, decltype(cc)::value>(q(0, n2), q(1, n2), q(2, n2), q(3, n2), ps, q(4, n2) + ps,
+                                                         ub, q(5, n2), q(6, n2), q(7, n2));
             };
             v[n2] = make_float2(f(std::integral_constant<int, c>{}), f(std::integral_constant<int, c + 1>{}));
           }
@@ -432,19 +429,29 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_spec_x(SpecXArgs a) {
 #pragma unroll
       for (int c = 0; c < NC; ++c) q[c][n2] = u[c];
     }
-    if (a.speed != nullptr) spec_speed(a, smax, valid, sol, T, S.red);
-    spec_fluxes<N, T, ND, PHYS>(a, pf, S.ax, q, er, row, valid, 0, 1);
+    if (a.speed != nullptr) spec_speed(a, smax, valid, sol, blockIdx.x, T, S.red);
+    // the state's registers are opaque per job: without this the compiler
+    // keeps flux terms shared by several jobs live across the loop (16
+    // registers each) and spills
+    auto opaque = [&]() {
+#pragma unroll
+      for (int c = 0; c < NC; ++c)
+#pragma unroll
+        for (int n2 = 0; n2 < B; ++n2) asm volatile("" : "+f"(q[c][n2]));
+    };
+    spec_fluxes<N, T, ND, PHYS>(a, pf, S.ax, [&](int c, int n2) { return q[c][n2]; }, opaque, er, row, valid, 0, 1);
   }
 }
 
-// x rows of grids with few pencils: one warp per pencil group and job group.
-// k_spec_x walks a row through all its transforms in one warp (12 at 2D MHD),
-// which leaves most of the GPU idle when the rows are few: a 512^2 solve has
-// 512 warps for 152 SMs.  Here NG job groups share the rows of a CTA: each
-// takes its component pairs through the inverse transform, the state meets in
-// shared memory, the points are dealt over all threads for the clamp and the
-// primitives, and each group takes its share of the flux transforms.  The
-// arithmetic per value is that of k_spec_x.
+// x rows of MHD and of Euler grids with few pencils: a warp per pencil group
+// and job group.  k_spec_x takes a row through all its transforms in one warp.
+// That leaves most of the GPU idle when the rows are few (128 rows of 128
+// points are 32 warps for 152 SMs, each with a chain of 6 transforms), and the
+// 128 registers of an MHD state leave two CTAs per SM.  Here NG job groups
+// share the rows of a CTA: each takes its component pairs through the inverse
+// transform, the state meets in shared memory, the points are dealt over all
+// threads for the clamp and the primitives, and each group takes its share of
+// the flux transforms.  The arithmetic per value is that of k_spec_x.
 template <int N, int T, int NC, int NG>
 struct SpecXsSmem {
   AxisSmem<N> ax;
@@ -453,16 +460,13 @@ struct SpecXsSmem {
   float red[32];
 };
 
-template <int ND, int PHYS> struct SpecXsGroups { static constexpr int value = (ND == 3 && PHYS == 0) ? 3 : 4; };
-
-template <int N, int ND, int PHYS, bool INC, bool FLUX>
-__global__ void __launch_bounds__(32 * SpecXsGroups<ND, PHYS>::value) k_spec_xs(SpecXArgs a) {
+template <int N, int ND, int PHYS, int NG, bool INC, bool FLUX>
+__global__ void __launch_bounds__(32 * NG, (PHYS == 1) ? 4 : 0) k_spec_xs(SpecXArgs a) {
   constexpr int NC = (PHYS == 1) ? 8 : ND + 2;
   constexpr int NP = NC / 2;
   constexpr bool ODD = (NC % 2) != 0;
   constexpr int NJ = NP + (ODD ? 1 : 0);
   constexpr int A = Shape<N>::A, B = Shape<N>::B, T = 32 / A;
-  constexpr int NG = SpecXsGroups<ND, PHYS>::value;
   constexpr int KM = spec_km(N), M = spec_modes(N);
   using PF = Pencil<N, T, false>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -471,151 +475,174 @@ __global__ void __launch_bounds__(32 * SpecXsGroups<ND, PHYS>::value) k_spec_xs(
   dep_wait();
   const int grp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int t = lane % A, p = lane / A;
-  const int row = blockIdx.x * T + p;
-  const int sol = (row < a.rows ? row : a.rows - 1) / a.rps;
-  const bool valid = row < a.rows && (a.active == nullptr || a.active[sol] != 0);
-  {
-    const int r0 = blockIdx.x * T, r1 = min(r0 + T, a.rows) - 1;
-    bool any = a.active == nullptr;
-    for (int s2 = r0 / a.rps; !any && s2 <= r1 / a.rps; ++s2) any = a.active[s2] != 0;
-    if (!any) return;
-  }
   PF pf{p, t, S.buf[grp], S.ax.twf, S.ax.twi};
-  const long rbase = (long)sol * a.ssU + (long)(row % a.rps) * N + t;
-  const float er = (PHYS == 0) ? a.eref[sol] : 0.0f;
-  const float eshift = a.shift_in ? er : 0.0f;
-  const float g1 = a.gamma - 1.0f;
-  const float pref = g1 * er;
-  constexpr int CE = (PHYS == 1) ? 4 : NC - 1;
-  auto slot = [&](int c, int n2) -> float& { return S.q[c][n2 * 32 + lane]; };
-  // this thread's points in the middle part are n2 = grp + NG i; the stage
-  // projection's change of U^n there is loaded ahead of the transforms
-  constexpr int NPT = (B + NG - 1) / NG;
-  [[maybe_unused]] float dB[NPT][3];
-  if constexpr (INC && PHYS == 1) {
+  auto tile_rows = [&](int tile) {
+    const int row = tile * T + p;
+    const int sol = (row < a.rows ? row : a.rows - 1) / a.rps;
+    const bool valid = row < a.rows && (a.active == nullptr || a.active[sol] != 0);
+    if (a.active != nullptr) {
+      bool any = false;
+      for (int s2 = tile * T / a.rps; !any && s2 <= (min(tile * T + T, a.rows) - 1) / a.rps; ++s2)
+        any = a.active[s2] != 0;
+      if (!any) return;
+    }
+    const long rbase = (long)sol * a.ssU + (long)(row % a.rps) * N + t;
+    const float er = (PHYS == 0) ? a.eref[sol] : 0.0f;
+    const float eshift = a.shift_in ? er : 0.0f;
+    const float g1 = a.gamma - 1.0f;
+    const float pref = g1 * er;
+    constexpr int CE = (PHYS == 1) ? 4 : NC - 1;
+    auto slot = [&](int c, int n2) -> float& { return S.q[c][n2 * 32 + lane]; };
+    // this thread's points in the middle part are n2 = grp + NG i; the stage
+    // projection's change of U^n there is loaded ahead of the transforms
+    constexpr int NPT = (B + NG - 1) / NG;
+    [[maybe_unused]] float dB[NPT][3];
+    if constexpr (INC && PHYS == 1) {
 #pragma unroll
-    for (int i = 0; i < NPT; ++i)
+      for (int i = 0; i < NPT; ++i)
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const int n2 = grp + NG * i;
-        const long o = (long)(row % a.rps) * N + t + A * n2;  // within a field
-        dB[i][c] = (a.Bp != nullptr && valid && n2 < B && c < a.nproj)
-                       ? a.Bp[((long)sol * a.nproj + c) * a.fs + o] - a.U[(5 + c) * a.fs + rbase + A * n2]
-                       : 0.0f;
-      }
-  }
-  __syncthreads();
+        for (int c = 0; c < 3; ++c) {
+          const int n2 = grp + NG * i;
+          const long o = (long)(row % a.rps) * N + t + A * n2;  // within a field
+          dB[i][c] = (a.Bp != nullptr && valid && n2 < B && c < a.nproj)
+                         ? a.Bp[((long)sol * a.nproj + c) * a.fs + o] - a.U[(5 + c) * a.fs + rbase + A * n2]
+                         : 0.0f;
+        }
+    }
+    __syncthreads();  // the tables; the state's last readers
 
-  // the group's component pairs: U^n (plus the increment, or filtered along x)
+    // the group's component pairs: U^n (plus the increment, or filtered along x)
 #pragma unroll 1
-  for (int j = grp; j < NJ; j += NG) {
-    const bool single = ODD && j == NP;
-    const int c0 = 2 * j, c1 = single ? c0 : c0 + 1;
-    float2 u[B], v[B];
-#pragma unroll
-    for (int n2 = 0; n2 < B; ++n2) {
-      u[n2].x = valid ? a.U[c0 * a.fs + rbase + A * n2] : (c0 == 0 ? 1.0f : 0.0f);
-      u[n2].y = (valid && !single) ? a.U[c1 * a.fs + rbase + A * n2] : 0.0f;
-      if (PHYS == 0 && valid) {
-        if (c0 == CE) u[n2].x -= eshift;
-        else if (c1 == CE) u[n2].y -= eshift;
-      }
-    }
-    if constexpr (INC) {
-      const float2* d = a.D + (long)row * a.pitch + j * M;
-      sfor<0, B>([&](auto rc) {
-        constexpr int r = decltype(rc)::value;
-        v[r] = make_float2(0.0f, 0.0f);
-        if constexpr (spec_keeps<N>(r)) {
-          const int k = pf.kidx(r);
-          int m = spec_col<N>(k);
-          if (ODD && single && m > KM) m = N - k;  // half spectra: X(-k) = conj X(k)
-          if (valid && m >= 0) v[r] = d[m];
-          if (ODD && single && k > KM) v[r].y = -v[r].y;
-        }
-      });
-      pf.inv(v);
+    for (int j = grp; j < NJ; j += NG) {
+      const bool single = ODD && j == NP;
+      const int c0 = 2 * j, c1 = single ? c0 : c0 + 1;
+      float2 u[B], v[B];
 #pragma unroll
       for (int n2 = 0; n2 < B; ++n2) {
-        u[n2].x += v[n2].x;
-        u[n2].y += v[n2].y;
-      }
-    } else if (a.px) {
-#pragma unroll
-      for (int n2 = 0; n2 < B; ++n2) v[n2] = u[n2];
-      pf.fwd(v);
-#pragma unroll
-      for (int r = 0; r < B; ++r) {
-        const float s = (1.0f / N) - S.ax.P[pf.kidx(r)];
-        v[r].x *= s;
-        v[r].y *= s;
-      }
-      pf.inv(v);
-#pragma unroll
-      for (int n2 = 0; n2 < B; ++n2) {
-        u[n2].x -= v[n2].x;
-        u[n2].y -= v[n2].y;
-        if (valid) {
-          a.Uw[c0 * a.fs + rbase + A * n2] = u[n2].x;
-          if (!single) a.Uw[c1 * a.fs + rbase + A * n2] = u[n2].y;
+        u[n2].x = valid ? a.U[c0 * a.fs + rbase + A * n2] : (c0 == 0 ? 1.0f : 0.0f);
+        u[n2].y = (valid && !single) ? a.U[c1 * a.fs + rbase + A * n2] : 0.0f;
+        if (PHYS == 0 && valid) {
+          if (c0 == CE) u[n2].x -= eshift;
+          else if (c1 == CE) u[n2].y -= eshift;
         }
       }
-    }
+      if constexpr (INC) {
+        const float2* d = a.D + (long)row * a.pitch + j * M;
+        sfor<0, B>([&](auto rc) {
+          constexpr int r = decltype(rc)::value;
+          v[r] = make_float2(0.0f, 0.0f);
+          if constexpr (spec_keeps<N>(r)) {
+            const int k = pf.kidx(r);
+            int m = spec_col<N>(k);
+            if (ODD && single && m > KM) m = N - k;  // half spectra: X(-k) = conj X(k)
+            if (valid && m >= 0) v[r] = d[m];
+            if (ODD && single && k > KM) v[r].y = -v[r].y;
+          }
+        });
+        pf.inv(v);
 #pragma unroll
-    for (int n2 = 0; n2 < B; ++n2) {
-      slot(c0, n2) = u[n2].x;
-      if (!single) slot(c1, n2) = u[n2].y;
-    }
-  }
-  __syncthreads();
-
-  // points n2 = grp, grp + NG, ..: clamp, new state, primitives
-  float smax = 0.0f;
+        for (int n2 = 0; n2 < B; ++n2) {
+          u[n2].x += v[n2].x;
+          u[n2].y += v[n2].y;
+        }
+      } else if (a.px) {
 #pragma unroll
-  for (int i = 0; i < NPT; ++i) {
-    const int n2 = grp + NG * i;
-    if (n2 >= B) break;
-    float u[NC];
+        for (int n2 = 0; n2 < B; ++n2) v[n2] = u[n2];
+        pf.fwd(v);
 #pragma unroll
-    for (int c = 0; c < NC; ++c) u[c] = slot(c, n2);
-    if constexpr (INC) {
-      if constexpr (PHYS == 1) {
-        clamp_mhd(u, a.gamma, a.rho_min, a.p_min);
-        if (a.Bp != nullptr && valid) {
+        for (int r = 0; r < B; ++r) {
+          const float s = (1.0f / N) - S.ax.P[pf.kidx(r)];
+          v[r].x *= s;
+          v[r].y *= s;
+        }
+        pf.inv(v);
 #pragma unroll
-          for (int c = 5; c < 8; ++c) {
-            if (c - 5 >= a.nproj) break;
-            const float b = u[c] + dB[i][c - 5];
-            u[4] += 0.5f * (b * b - u[c] * u[c]);
-            u[c] = b;
+        for (int n2 = 0; n2 < B; ++n2) {
+          u[n2].x -= v[n2].x;
+          u[n2].y -= v[n2].y;
+          if (valid) {
+            a.Uw[c0 * a.fs + rbase + A * n2] = u[n2].x;
+            if (!single) a.Uw[c1 * a.fs + rbase + A * n2] = u[n2].y;
           }
         }
-      } else if constexpr (ND == 2) {
-        const float pmin_shift = a.p_min - pref;
-        clamp_state<ND>(u, a.gamma, a.rho_min, pmin_shift);
       }
-      if (a.Uw != nullptr && valid) {
-        const float so = (PHYS == 0 && a.shift_out) ? er : 0.0f;
 #pragma unroll
-        for (int c = 0; c < NC; ++c)
-          a.Uw[c * a.fs + rbase + A * n2] = (PHYS == 0 && c == CE) ? u[c] + so : u[c];
+      for (int n2 = 0; n2 < B; ++n2) {
+        slot(c0, n2) = u[n2].x;
+        if (!single) slot(c1, n2) = u[n2].y;
+      }
+    }
+    __syncthreads();
+
+    // points n2 = grp, grp + NG, ..: clamp, new state, primitives
+    float smax = 0.0f;
+#pragma unroll
+    for (int i = 0; i < NPT; ++i) {
+      const int n2 = grp + NG * i;
+      if (n2 >= B) break;
+      float u[NC];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) u[c] = slot(c, n2);
+      if constexpr (INC) {
+        if constexpr (PHYS == 1) {
+          clamp_mhd(u, a.gamma, a.rho_min, a.p_min);
+          if (a.Bp != nullptr && valid) {
+#pragma unroll
+            for (int c = 5; c < 8; ++c) {
+              if (c - 5 >= a.nproj) break;
+              const float b = u[c] + dB[i][c - 5];
+              u[4] += 0.5f * (b * b - u[c] * u[c]);
+              u[c] = b;
+            }
+          }
+        } else if constexpr (ND == 2) {
+          const float pmin_shift = a.p_min - pref;
+          clamp_state<ND>(u, a.gamma, a.rho_min, pmin_shift);
+        }
+        if (a.Uw != nullptr && valid) {
+          const float so = (PHYS == 0 && a.shift_out) ? er : 0.0f;
+#pragma unroll
+          for (int c = 0; c < NC; ++c)
+            a.Uw[c * a.fs + rbase + A * n2] = (PHYS == 0 && c == CE) ? u[c] + so : u[c];
+        }
+      }
+      if constexpr (FLUX) {
+        smax = fmaxf(smax, spec_primitive<ND, PHYS>(u, a.gamma, g1, pref, a.speed != nullptr && valid));
+#pragma unroll
+        for (int c = 0; c < NC; ++c) slot(c, n2) = u[c];
       }
     }
     if constexpr (FLUX) {
-      smax = fmaxf(smax, spec_primitive<ND, PHYS>(u, a.gamma, g1, pref, a.speed != nullptr && valid));
+      if (a.speed != nullptr) spec_speed(a, smax, valid, sol, tile, T, S.red);
+      __syncthreads();
+      if constexpr (PHYS == 1) {
+        // points come from shared memory per job: the whole state in registers
+        // (128 of them) leaves half the warps in flight.  Orszag-Tang 512^2 step
+        // 200 -> 183 us; the 16 to 80 registers of the Euler states stay
+        spec_fluxes<N, T, ND, PHYS>(a, pf, S.ax, slot, [] { asm volatile("" ::: "memory"); }, er, row, valid, grp, NG);
+      } else {
+        float q[NC][B];
 #pragma unroll
-      for (int c = 0; c < NC; ++c) slot(c, n2) = u[c];
+        for (int c = 0; c < NC; ++c)
+#pragma unroll
+          for (int n2 = 0; n2 < B; ++n2) q[c][n2] = slot(c, n2);
+        auto opaque = [&] {  // as in k_spec_x
+#pragma unroll
+          for (int c = 0; c < NC; ++c)
+#pragma unroll
+            for (int n2 = 0; n2 < B; ++n2) asm volatile("" : "+f"(q[c][n2]));
+        };
+        spec_fluxes<N, T, ND, PHYS>(a, pf, S.ax, [&](int c, int n2) { return q[c][n2]; }, opaque, er, row, valid, grp, NG);
+      }
     }
-  }
-  if constexpr (FLUX) {
-    if (a.speed != nullptr) spec_speed(a, smax, valid, sol, T, S.red);
-    __syncthreads();
-    float q[NC][B];
-#pragma unroll
-    for (int c = 0; c < NC; ++c)
-#pragma unroll
-      for (int n2 = 0; n2 < B; ++n2) q[c][n2] = slot(c, n2);
-    spec_fluxes<N, T, ND, PHYS>(a, pf, S.ax, q, er, row, valid, grp, NG);
+  };
+  if constexpr (PHYS == 1) {
+    // a CTA walks over its tiles, the tables loaded once; the loop costs the
+    // Euler kernels 10 to 30 registers (Taylor-Green 64^3 92.8 -> 99 us)
+#pragma unroll 1
+    for (int tile = blockIdx.x; tile < (a.rows + T - 1) / T; tile += gridDim.x) tile_rows(tile);
+  } else {
+    tile_rows(blockIdx.x);
   }
 }
 

@@ -1,8 +1,9 @@
-"""The x rows of the truncated-spectra steps run in one warp per row group or,
-when the rows are few, in several warps that share them (k_spec_x and
-k_spec_xs, csrc/spectral.cuh).  A large batch takes the first kernel and each
-of its solves alone the second; both run the same operations per value, so
-their states differ by rounding only.
+"""The x rows of the truncated-spectra steps run in one warp per row group
+(k_spec_x, csrc/spectral.cuh) or in several warps that share them (k_spec_xs:
+MHD, and Euler where the rows are few).  A large Euler batch takes the first
+kernel and each of its solves alone the second; the CTAs of a large MHD batch
+walk over several tiles of rows, those of one solve take one tile each.  All
+run the same operations per value, so their states differ by rounding only.
 
 Bound: both are within 8e-6 of exact arithmetic over these steps (16 stages of
 8 eps), and they share all but the contraction of products and sums, so half of
