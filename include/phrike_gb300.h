@@ -187,6 +187,12 @@ int ps_run_steps(ps_plan plan, float* U, int nsteps, double dt, const double* d_
  * happen): advance in chunks and read d_t between chunks.  Replaces the
  * while-loop of SpectralSolver*.run (solver.py:384-417, 773-800, 1480-1505). */
 int ps_run_cfl(ps_plan plan, float* U, int nsteps, double* d_t, const double* d_tend, void* stream);
+/* ps_run_cfl with one t_end for all solves that also stops a solve before a
+ * step that would start at or past t_out (t + 1e-12 >= t_out).  For the plans of which
+ * ps_plan_can_pause returns 1 (2D/3D Fourier grids with the 2/3 mask, no
+ * gravity, artificial viscosity or MHD diffusion); PS_ERR_UNSUPPORTED else. */
+int ps_run_cfl_until(ps_plan plan, float* U, int nsteps, double* d_t, double t_end, double t_out, void* stream);
+int ps_plan_can_pause(ps_plan plan);
 
 /* Adaptive embedded Runge-Kutta (adaptive.py:23-437).  Methods: */
 #define PS_ARK_RK23 0 /* Bogacki-Shampine 3(2)                                   */

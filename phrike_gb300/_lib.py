@@ -100,6 +100,8 @@ _SIGNATURES = [
     ("ps_plan_nsolve", C.c_int, [C.c_void_p]),
     ("ps_plan_steps_done", C.c_int, [C.c_void_p, C.POINTER(C.c_int)]),
     ("ps_run_cfl", C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]),
+    ("ps_run_cfl_until", C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_double, C.c_double, C.c_void_p]),
+    ("ps_plan_can_pause", C.c_int, [C.c_void_p]),
     ("ps_adaptive_desc_init", None, [C.POINTER(AdaptiveDesc)]),
     ("ps_run_adaptive", C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.POINTER(AdaptiveDesc), C.c_void_p, C.c_void_p,
                                   C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),

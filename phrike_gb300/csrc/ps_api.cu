@@ -1188,7 +1188,7 @@ int spec_last(ps_plan p, const SpecBufs& b, int stage, double dt, const double* 
 // every later increment lies inside it too (its spectra are stored truncated,
 // and 3D has no clamp), and the projection of a sum of such fields is the sum.
 int steps_spec(ps_plan p, float* U, int nsteps, double dt, const double* d_dt, double* d_t, const double* d_tend,
-               cudaStream_t s) {
+               cudaStream_t s, ps::StepLimits lim = {}) {
   int rc;
   const SpecBufs b = spec_bufs(p);
   const bool cfl = d_t != nullptr;
@@ -1233,7 +1233,7 @@ int steps_spec(ps_plan p, float* U, int nsteps, double dt, const double* d_dt, d
     pending_px = false;
     if (cfl)
       PS_CU(ps::launch_step_control(p->speed, p->desc.cfl, p->hmin(), d_t, d_tend, p->nsolve, p->dt, p->active, s,
-                                    p->dt_diff()),
+                                    p->dt_diff(), lim),
             "step control");
     const bool use_bp = substages && it == 0;
     for (int stage = 0; stage < 4; ++stage) {
@@ -1735,6 +1735,16 @@ int ps_run_cfl(ps_plan p, float* U, int nsteps, double* d_t, const double* d_ten
   if (p->mhd) return steps_mhd(p, U, nsteps, 0.0, nullptr, d_t, d_tend, s);
   if (p->nd == 1) return step_1d(p, U, nsteps, 0.0, nullptr, d_t, d_tend, s);
   return steps_nd(p, U, nsteps, 0.0, nullptr, d_t, d_tend, s);
+}
+
+int ps_plan_can_pause(ps_plan p) { return (p && p->spec) ? 1 : 0; }
+
+int ps_run_cfl_until(ps_plan p, float* U, int nsteps, double* d_t, double t_end, double t_out, void* stream) {
+  if (!p || !U || !d_t) return fail(PS_ERR_INVALID, "null argument");
+  if (nsteps < 0) return fail(PS_ERR_INVALID, "nsteps must be >= 0");
+  if (!p->spec) return fail(PS_ERR_UNSUPPORTED, "this plan's CFL runs take no pause time");
+  if (nsteps == 0) return PS_OK;
+  return steps_spec(p, U, nsteps, 0.0, nullptr, d_t, nullptr, (cudaStream_t)stream, ps::StepLimits{t_end, t_out});
 }
 
 void ps_adaptive_desc_init(ps_adaptive_desc* ad) {

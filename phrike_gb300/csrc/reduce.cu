@@ -214,15 +214,16 @@ __global__ void k_energy_shift(float* E, long n, long ss, const float* eref, flo
 // Per-solve CFL step control before a step (solver.py:386-389, 235-240):
 // active = t < t_end - 1e-12; dt = active ? min(cfl h / speed, t_end - t) : 0.
 __global__ void k_step_control(const float* speed, double cfl, double hmin, const double* t, const double* tend,
-                               int nsolve, double* dt, int* active, double dt_cap) {
+                               int nsolve, double* dt, int* active, double dt_cap, StepLimits lim) {
   dep_wait();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nsolve) return;
-  const bool on = t[s] < tend[s] - 1e-12;
+  const double te = (tend != nullptr) ? tend[s] : lim.t_end;
+  const bool on = t[s] < te - 1e-12 && (tend != nullptr || t[s] + 1e-12 < lim.t_out);
   const double sp = (double)speed[s];
   double d = (sp <= 0.0) ? 1e-6 : cfl * hmin / sp;
   if (sp > 0.0 && dt_cap > 0.0) d = fmin(d, dt_cap);  // parabolic limit of explicit diffusion
-  d = fmin(d, tend[s] - t[s]);
+  d = fmin(d, te - t[s]);
   dt[s] = on ? d : 0.0;
   active[s] = on ? 1 : 0;
 }
@@ -261,8 +262,10 @@ cudaError_t launch_energy_shift(float* E, long n, long ss, int nsolve, const flo
 }
 
 cudaError_t launch_step_control(const float* speed, double cfl, double hmin, const double* t, const double* tend,
-                                int nsolve, double* dt, int* active, cudaStream_t s, double dt_cap) {
-  return launch_dep(k_step_control, (nsolve + 127) / 128, 128, 0, s, speed, cfl, hmin, t, tend, nsolve, dt, active, dt_cap);
+                                int nsolve, double* dt, int* active, cudaStream_t s, double dt_cap,
+                                StepLimits lim) {
+  return launch_dep(k_step_control, (nsolve + 127) / 128, 128, 0, s, speed, cfl, hmin, t, tend, nsolve, dt, active, dt_cap,
+                    lim);
 }
 
 cudaError_t launch_step_advance(double* t, const double* dt, float* speed, const int* active, int* steps,
@@ -291,7 +294,8 @@ cudaError_t launch_conserved(int nd, const float* U, long cells, long ss, int ns
                              cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(out, 0, sizeof(double) * (nd + 2) * nsolve, s);
   if (e != cudaSuccess) return e;
-  const dim3 grid(reduce_blocks(cells, nsolve), nsolve);
+  // four cells per thread: the blocks' float64 atomics queue on nd + 2 words
+  const dim3 grid(reduce_blocks((cells + 3) / 4, nsolve), nsolve);
   if (nd == 1) k_conserved<1><<<grid, 256, 0, s>>>(U, cells, ss, gamma, out);
   else if (nd == 2) k_conserved<2><<<grid, 256, 0, s>>>(U, cells, ss, gamma, out);
   else k_conserved<3><<<grid, 256, 0, s>>>(U, cells, ss, gamma, out);

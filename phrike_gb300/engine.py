@@ -267,6 +267,21 @@ class Plan:
                                         _stream(self.device)))
         return U
 
+    def can_pause(self) -> bool:
+        """Whether run_cfl_until_ takes this plan."""
+        return bool(self._lib.ps_plan_can_pause(self._handle))
+
+    def run_cfl_until_(self, U: torch.Tensor, nsteps: int, t: torch.Tensor, t_end: float,
+                       t_out: float) -> torch.Tensor:
+        """run_cfl_ with one ``t_end`` that also stops a solve before a step
+        that would start at or past ``t_out``."""
+        self._check_state(U)
+        if t.dtype != torch.float64 or t.device != self.device or t.numel() != self.nsolve:
+            raise RuntimeError("t must be a float64 device tensor with one entry per solve")
+        _lib.check(self._lib.ps_run_cfl_until(self._handle, _ptr(U), int(nsteps), _ptr(t), float(t_end), float(t_out),
+                                              _stream(self.device)))
+        return U
+
     @staticmethod
     def adaptive_desc(adaptive_config: Optional[dict] = None) -> "_lib.AdaptiveDesc":
         """ps_adaptive_desc from the reference's adaptive_config keys
