@@ -143,6 +143,14 @@ __device__ __forceinline__ float spec_primitive(float (&u)[NC], float gamma, flo
   }
 }
 
+// total pressure and u . B of MHD primitives (rho, u, E, B)
+__device__ __forceinline__ void mhd_derived(const float (&u)[8], float g1, float& ps, float& ub) {
+  const float b2 = u[5] * u[5] + u[6] * u[6] + u[7] * u[7];
+  const float v2 = u[1] * u[1] + u[2] * u[2] + u[3] * u[3];
+  ps = g1 * (u[4] - 0.5f * u[0] * v2 - 0.5f * b2) + 0.5f * b2;
+  ub = u[1] * u[5] + u[2] * u[6] + u[3] * u[7];
+}
+
 // Largest speed of a tile's T rows into their solves' slots (all threads)
 __device__ __forceinline__ void spec_speed(const SpecXArgs& a, float smax, bool valid, int sol, int tile, int T,
                                            float* red) {
@@ -159,8 +167,9 @@ __device__ __forceinline__ void spec_speed(const SpecXArgs& a, float smax, bool 
 // Flux jobs first, first + step, .. of a row whose primitives are q(c, n2):
 // fluxes of a component pair along one direction, forward transform, D_x or
 // P_x, store.  opaque() keeps the compiler from carrying flux terms over the
-// jobs.
-template <int N, int T, int ND, int PHYS, typename PF, typename Q, typename O>
+// jobs.  DERIVED (MHD): q(4) is E plus the total pressure, q(8) the total
+// pressure and q(9) u . B, so that the jobs do not each take them again.
+template <int N, int T, int ND, int PHYS, bool DERIVED, typename PF, typename Q, typename O>
 __device__ __forceinline__ void spec_fluxes(const SpecXArgs& a, const PF& pf, const AxisSmem<N>& ax,
                                             Q&& q, O&& opaque, float er, int row, bool valid, int first, int step) {
   constexpr int B = Shape<N>::B;
@@ -215,13 +224,21 @@ __device__ __forceinline__ void spec_fluxes(const SpecXArgs& a, const PF& pf, co
         if (job == J) {
 #pragma unroll
           for (int n2 = 0; n2 < B; ++n2) {
-            const float b2 = q(5, n2) * q(5, n2) + q(6, n2) * q(6, n2) + q(7, n2) * q(7, n2);
-            const float v2 = q(1, n2) * q(1, n2) + q(2, n2) * q(2, n2) + q(3, n2) * q(3, n2);
-            const float ps = g1 * (q(4, n2) - 0.5f * q(0, n2) * v2 - 0.5f * b2) + 0.5f * b2;
-            const float ub = q(1, n2) * q(5, n2) + q(2, n2) * q(6, n2) + q(3, n2) * q(7, n2);
+            float ps, ub, eps;
+            if constexpr (DERIVED) {
+              eps = q(4, n2);
+              ps = q(8, n2);
+              ub = q(9, n2);
+            } else {
+              float u[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) u[i] = q(i, n2);
+              mhd_derived(u, g1, ps, ub);
+              eps = u[4] + ps;
+            }
             auto f = [&](auto cc) {
-              return mhd3_flux<DIR, decltype(cc)::value>(q(0, n2), q(1, n2), q(2, n2), q(3, n2), ps, q(4, n2) + ps,
-                                                         ub, q(5, n2), q(6, n2), q(7, n2));
+              return mhd3_flux<DIR, decltype(cc)::value>(q(0, n2), q(1, n2), q(2, n2), q(3, n2), ps, eps, ub, q(5, n2),
+                                                         q(6, n2), q(7, n2));
             };
             v[n2] = make_float2(f(std::integral_constant<int, c>{}), f(std::integral_constant<int, c + 1>{}));
           }
@@ -439,7 +456,8 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_spec_x(SpecXArgs a) {
 #pragma unroll
         for (int n2 = 0; n2 < B; ++n2) asm volatile("" : "+f"(q[c][n2]));
     };
-    spec_fluxes<N, T, ND, PHYS>(a, pf, S.ax, [&](int c, int n2) { return q[c][n2]; }, opaque, er, row, valid, 0, 1);
+    spec_fluxes<N, T, ND, PHYS, false>(a, pf, S.ax, [&](int c, int n2) { return q[c][n2]; }, opaque, er, row, valid, 0,
+                                       1);
   }
 }
 
@@ -456,7 +474,7 @@ template <int N, int T, int NC, int NG>
 struct SpecXsSmem {
   AxisSmem<N> ax;
   float2 buf[NG][Pencil<N, T, false>::BUF];
-  float q[NC][T * N];  // [component][n2][thread of the group]
+  float q[(NC == 8) ? 10 : NC][T * N];  // [component (and MHD's derived values)][n2][thread of the group]
   float red[32];
 };
 
@@ -608,6 +626,13 @@ __global__ void __launch_bounds__(32 * NG, (PHYS == 1) ? 4 : 0) k_spec_xs(SpecXA
       }
       if constexpr (FLUX) {
         smax = fmaxf(smax, spec_primitive<ND, PHYS>(u, a.gamma, g1, pref, a.speed != nullptr && valid));
+        if constexpr (PHYS == 1) {
+          float ps, ub;
+          mhd_derived(u, g1, ps, ub);
+          u[4] += ps;
+          slot(8, n2) = ps;
+          slot(9, n2) = ub;
+        }
 #pragma unroll
         for (int c = 0; c < NC; ++c) slot(c, n2) = u[c];
       }
@@ -619,7 +644,7 @@ __global__ void __launch_bounds__(32 * NG, (PHYS == 1) ? 4 : 0) k_spec_xs(SpecXA
         // points come from shared memory per job: the whole state in registers
         // (128 of them) leaves half the warps in flight.  Orszag-Tang 512^2 step
         // 200 -> 183 us; the 16 to 80 registers of the Euler states stay
-        spec_fluxes<N, T, ND, PHYS>(a, pf, S.ax, slot, [] { asm volatile("" ::: "memory"); }, er, row, valid, grp, NG);
+        spec_fluxes<N, T, ND, PHYS, true>(a, pf, S.ax, slot, [] { asm volatile("" ::: "memory"); }, er, row, valid, grp, NG);
       } else {
         float q[NC][B];
 #pragma unroll
@@ -632,7 +657,7 @@ __global__ void __launch_bounds__(32 * NG, (PHYS == 1) ? 4 : 0) k_spec_xs(SpecXA
 #pragma unroll
             for (int n2 = 0; n2 < B; ++n2) asm volatile("" : "+f"(q[c][n2]));
         };
-        spec_fluxes<N, T, ND, PHYS>(a, pf, S.ax, [&](int c, int n2) { return q[c][n2]; }, opaque, er, row, valid, grp, NG);
+        spec_fluxes<N, T, ND, PHYS, false>(a, pf, S.ax, [&](int c, int n2) { return q[c][n2]; }, opaque, er, row, valid, grp, NG);
       }
     }
   };
