@@ -45,7 +45,7 @@ def workload_config(n: int, world: int) -> dict:
         "grid": [n, n, n],
         "state_dtype": "float32",
         "dealias": "2/3",
-        "filter": "off (mask-only end-of-step filter applied every step)",
+        "filter": "off (mask-only end-of-step filter; the increments stay inside the mask)",
         "cells_per_step": n ** 3,
         "l2_policy": "inputs larger than L2 (state + pass intermediates ~2.7 GB >> 129 MB)",
         "parallelism": f"replicas x{world}" if world > 1 else "single solve",
@@ -61,11 +61,11 @@ def hbm_peak():
 
 
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of the
-# pass kernels of a TGV 256^3 RK4 step, averaged over the step's launches,
-# from ncu captures of the bench command (x pass at 256^3; y and last pass
-# at 128^3, reads scaled by the 8x cell count, writes at their algorithmic
-# size, which every write reaches at 256^3).
-NCU_TRAFFIC_TGV256 = {"x_pass": 1.366e9, "y_pass": 1.678e9, "last_pass": 1.762e9}
+# pass kernels of a TGV 256^3 RK4 step, averaged over the step's launches, from
+# an ncu capture of one step (profiles/truncated_spectra.md).  The step's fourth
+# x launch ends one step and begins the next: a stage's 1.173e9 and the state it
+# also writes (0.281e9 as captured on the last launch of a run), 1.454e9.
+NCU_TRAFFIC_TGV256 = {"x_pass": 1.243e9, "y_pass": 0.630e9, "last_pass": 0.575e9}
 
 
 def traffic_per_launch(kind: str, n: int):

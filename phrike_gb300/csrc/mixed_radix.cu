@@ -101,8 +101,7 @@ __global__ void __launch_bounds__(kMrThreads, kMrMinBlocks) k_mr_op(MrOpArgs a) 
     });
     mr_fft(mr_sig, pitch, nsig * pg, ax, false);
     mr_spectra(mr_sig, a.g, nsig, [&](int, int k, float2& w) {
-      if (a.complement) w = cscale(w, complement_factor(a.ax, k));
-      else w = mr_symbol(w, k, a.g.n, a.deriv, a.scale, a.kunit, a.ax.P, a.ax.d);
+      w = mr_symbol(w, k, a.g.n, a.deriv, a.scale, a.kunit, a.ax.P, a.ax.d);
     });
     mr_fft(mr_sig, pitch, nsig * pg, ax, true);
     mr_each(a.g, pb, [&](int q, int i, long off) {
@@ -111,15 +110,8 @@ __global__ void __launch_bounds__(kMrThreads, kMrMinBlocks) k_mr_op(MrOpArgs a) 
         const int fa = f0 + 2 * s, fb = fa + 1;
         const float2 w = mr_sig[(s * pg + q) * pitch + i];
         const long oa = fa * a.fs + off, ob = fb * a.fs + off;
-        if (a.complement) {
-          const float va = in[oa] - w.x;
-          const float vb = (fb < a.nf) ? in[ob] - w.y : 0.0f;
-          out[oa] = va;
-          if (fb < a.nf) out[ob] = vb;
-        } else {
-          out[oa] = w.x;
-          if (fb < a.nf) out[ob] = w.y;
-        }
+        out[oa] = w.x;
+        if (fb < a.nf) out[ob] = w.y;
       }
     });
     __syncthreads();

@@ -16,8 +16,8 @@
 // field layouts, operator tables and stage arithmetic), so the step loops,
 // adaptive stepping and the operator entry points run on either:
 //   op    : out = op(in) along one axis, pairs of real fields packed into one
-//           complex transform (op: P, D, L, raw second derivative, or the
-//           complementary filter in - IFFT((1/N - P) FFT in))
+//           complex transform (op: P, D, L or raw second derivative; the
+//           complementary filters run in mr_spec.cu)
 //   x     : optional fused filter P_x of the state, CFL speed, flux of the
 //           state, G = [D_x F^x, P_x F^y (, P_x F^z)]
 //   y3    : 3D middle axis: AB = [P_y G + D_y H^y, P_y H^z]
@@ -79,7 +79,6 @@ struct MrOpArgs {
   MrGeom g;
   int deriv;  // 0 P, 1 D, 2 L, 3 raw second derivative (op_symbol)
   float scale, kunit;
-  int complement;
   const int* active;
 };
 

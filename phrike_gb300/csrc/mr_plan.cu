@@ -150,7 +150,6 @@ int mr_apply_op(ps_plan p, int axis, const float* in, float* out, int nf, int de
   a.deriv = deriv;
   a.scale = scale;
   a.kunit = (float)(2.0 * M_PI / p->desc.length[axis]);
-  a.complement = complement ? 1 : 0;
   a.active = active;
   MR_CU(launch_mr_op(a, p->nsolve, s), "operator pass");
   return PS_OK;

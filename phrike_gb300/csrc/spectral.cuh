@@ -19,8 +19,12 @@
 // per cell instead of 75 and runs 22 complex pencil transforms per cell
 // instead of 37; a 3D MHD stage moves 77 words instead of 230 (and needs no
 // projection per stage, see steps_spec).  Measured per step against those
-// passes: Taylor-Green 256^3 4.95 -> 3.88 ms, KHI 512^2 x 16 1.06 -> 0.96 ms,
-// Orszag-Tang 512^2 0.456 -> 0.319 ms, 3D MHD 128^3 2.29 -> 1.41 ms.
+// passes, with what the kernels below gained since: Taylor-Green 256^3 (mask
+// filter) 4.95 -> 3.23 ms, KHI 512^2 x 16 1.06 -> 0.72 ms, Orszag-Tang 512^2
+// 0.456 -> 0.180 ms, 3D MHD 128^3 2.29 -> 0.98 ms.  Traffic bounds the y and z
+// passes (Taylor-Green 256^3: y forward 173 us at 5.7 TB/s, last 128 us, y
+// inverse 66 us) and instruction issue the x pass (349 us for 1.24 GB, 12
+// transforms per row at 12 warps per SM).
 //
 // Two real fields travel as one complex field: every operator maps real
 // fields to real fields, so it acts on f + i g as on f and g, and no pass but
