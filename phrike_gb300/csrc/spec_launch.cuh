@@ -98,11 +98,11 @@ cudaError_t spec_xs_mode(bool inc, bool flux, const SpecXArgs& a, cudaStream_t s
 // per SM their chains of 6 to 12 transforms do not overlap enough, and the jobs
 // of a row go to several warps (k_spec_xs).  Step times, k_spec_x against
 // k_spec_xs: KHI 128^2 84.1 -> 65.7 us (32 warps), Taylor-Green 64^3 94.9 ->
-// 92.8 us (1024), batches at 6.7 warps per SM between 52 -> 46 us (64^2 x 64) and
-// 90 -> 92 us (256^2 x 8); at 10 to 27 warps per SM k_spec_xs takes 1% to 13%
-// longer (256^2 x 32 237 against 267 us) but at 512^2 x 4 (208 against 199 us).  MHD rows up to 512 points
-// always take k_spec_xs: Orszag-Tang 512^2 249 -> 183 us (512 warps), 3D MHD
-// 128^3 1184 -> 1056 us (4096).
+// 92.8 us (1024), batches at 6.7 warps per SM between 52 -> 46 us (64^2 x 64)
+// and 90 -> 92 us (256^2 x 8); at 10 to 27 warps per SM k_spec_xs takes 1% to
+// 13% longer (256^2 x 32 237 against 267 us) but at 512^2 x 4 (208 against
+// 199 us).  MHD rows up to 512 points always take k_spec_xs: Orszag-Tang 512^2
+// 249 -> 183 us (512 warps), 3D MHD 128^3 1184 -> 1056 us (4096).
 constexpr long kSpecXsWarps = 8 * 152;
 
 // Euler x pass of every length, MHD x pass in a unit of its own
