@@ -781,12 +781,14 @@ int xfirst_mhd(ps_plan p, const float* U, float* speed, cudaStream_t s, const in
 
 // Helmholtz projection of (Bx, By) in place (solve stride ss); E (nullable)
 // updated with the thermal pressure held fixed.
-int project(ps_plan p, float* Bx, float* By, float* E, long ss, const int* active, cudaStream_t s) {
+// With from, the field read is from's (Bx, By one field apart, solve stride ss_from).
+int project(ps_plan p, float* Bx, float* By, float* E, long ss, const int* active, cudaStream_t s,
+            float* from = nullptr, long ss_from = 0) {
   ps::ProjArgs a{};
-  a.Bx = Bx;
-  a.By = By;
+  a.Bx = from ? from : Bx;  // the forward pass only reads them
+  a.By = from ? from + p->cells : By;
   a.E = E;
-  a.ss = ss;
+  a.ss = from ? ss_from : ss;
   a.H = p->H;
   a.nx = p->n[0];
   a.ny = p->n[1];
@@ -804,6 +806,9 @@ int project(ps_plan p, float* Bx, float* By, float* E, long ss, const int* activ
   e = ps::dispatch_n(p->n[1], [&](auto nc) { return ps::launch_proj_y<decltype(nc)::value>(a, s); });
   if (e != cudaSuccess) return cuda_fail(e, "projection y");
   a.ax = p->ax(0);
+  a.Bx = Bx;
+  a.By = By;
+  a.ss = ss;
   e = ps::dispatch_n(p->n[0], [&](auto nc) { return ps::launch_proj_xi<decltype(nc)::value>(a, s); });
   if (e != cudaSuccess) return cuda_fail(e, "projection x inverse");
   return PS_OK;
@@ -811,14 +816,14 @@ int project(ps_plan p, float* Bx, float* By, float* E, long ss, const int* activ
 
 // 3D Helmholtz projection of (Bx, By, Bz) in place (solve stride ss); E
 // (nullable) updated at fixed thermal pressure (grid.py:1649-1684,
-// solver.py:966-986)
-int project3(ps_plan p, float* Bx, float* By, float* Bz, float* E, long ss, const int* active, cudaStream_t s) {
+// solver.py:966-986); from as in project
+int project3(ps_plan p, float* Bx, float* By, float* Bz, float* E, long ss, const int* active, cudaStream_t s,
+             float* from = nullptr, long ss_from = 0) {
   ps::Proj3Args a{};
-  a.B[0] = Bx;
-  a.B[1] = By;
-  a.B[2] = Bz;
+  float* const out[3] = {Bx, By, Bz};
+  for (int c = 0; c < 3; ++c) a.B[c] = from ? from + c * p->cells : out[c];
   a.E = E;
-  a.ss = ss;
+  a.ss = from ? ss_from : ss;
   a.H = p->H;
   a.nx = p->n[0];
   a.ny = p->n[1];
@@ -841,6 +846,8 @@ int project3(ps_plan p, float* Bx, float* By, float* Bz, float* E, long ss, cons
   a.ax = p->ax(1);
   if ((e = ps::launch_proj3_y(p->n[1], true, a, s)) != cudaSuccess) return cuda_fail(e, "3D projection y inverse");
   a.ax = p->ax(0);
+  for (int c = 0; c < 3; ++c) a.B[c] = out[c];
+  a.ss = ss;
   if ((e = ps::launch_proj3_xi(p->n[0], a, s)) != cudaSuccess) return cuda_fail(e, "3D projection x inverse");
   return PS_OK;
 }
@@ -1213,11 +1220,10 @@ int steps_spec(ps_plan p, float* U, int nsteps, double dt, const double* d_dt, d
   if (substages) {
     // the projection of the stage states replaces U^n's B by its projection;
     // later steps start from a projected state
-    const size_t w = (size_t)p->nd * p->cells * sizeof(float);
-    PS_CU(cudaMemcpy2DAsync(b.Bp, w, U + 5 * p->cells, ssU * sizeof(float), w, p->nsolve, cudaMemcpyDeviceToDevice, s),
-          "B copy");
-    rc = (p->nd == 3) ? project3(p, b.Bp, b.Bp + p->cells, b.Bp + 2 * p->cells, nullptr, 3 * p->cells, act, s)
-                      : project(p, b.Bp, b.Bp + p->cells, nullptr, 2 * p->cells, act, s);
+    float* B = U + 5 * p->cells;
+    rc = (p->nd == 3)
+             ? project3(p, b.Bp, b.Bp + p->cells, b.Bp + 2 * p->cells, nullptr, 3 * p->cells, act, s, B, ssU)
+             : project(p, b.Bp, b.Bp + p->cells, nullptr, 2 * p->cells, act, s, B, ssU);
     if (rc != PS_OK) return rc;
   }
   bool pending_px = false, begun = false;
