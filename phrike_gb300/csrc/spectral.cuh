@@ -22,7 +22,7 @@
 // passes, with what the kernels below gained since: Taylor-Green 256^3 (mask
 // filter) 4.95 -> 3.23 ms, KHI 512^2 x 16 1.06 -> 0.72 ms, Orszag-Tang 512^2
 // 0.456 -> 0.180 ms, 3D MHD 128^3 2.29 -> 0.98 ms.  Traffic bounds the y and z
-// passes (Taylor-Green 256^3: y forward 173 us at 5.7 TB/s, last 128 us, y
+// passes (Taylor-Green 256^3: y forward 173 us at 5.4 TB/s, last 128 us, y
 // inverse 66 us) and instruction issue the x pass (349 us for 1.24 GB, 12
 // transforms per row at 12 warps per SM).
 //
