@@ -102,7 +102,8 @@ cudaError_t spec_xs_mode(bool inc, bool flux, const SpecXArgs& a, cudaStream_t s
 // and 90 -> 92 us (256^2 x 8); at 10 to 27 warps per SM k_spec_xs takes 1% to
 // 13% longer (256^2 x 32 237 against 267 us) but at 512^2 x 4 (208 against
 // 199 us).  MHD rows up to 512 points always take k_spec_xs: Orszag-Tang 512^2
-// 249 -> 183 us (512 warps), 3D MHD 128^3 1184 -> 1056 us (4096).
+// 249 -> 183 us (512 warps), 3D MHD 128^3 1184 -> 1056 us (4096).  A batch may
+// take the other kernel than one of its solves alone: both give the same bits.
 constexpr long kSpecXsWarps = 8 * 152;
 
 // Euler x pass of every length, MHD x pass in a unit of its own

@@ -115,7 +115,11 @@ __device__ __forceinline__ float mhd3_flux(float rho, float ux, float uy, float 
 }
 
 // Conservative to primitive at one point (rho, u, p' for Euler; B and E stay
-// for MHD); returns the wave speed of the point, or 0 if not asked for.
+// for MHD); returns the wave speed of the point, or 0 if not asked for.  The
+// Euler products that meet a sum here and in the fluxes are rounded as
+// written: left to the compiler, the two kernels of the x rows contracted them
+// differently (wave speeds at 8 points per row), and a solve must give the
+// same bits alone and in a batch.
 template <int ND, int PHYS, int NC>
 __device__ __forceinline__ float spec_primitive(float (&u)[NC], float gamma, float g1, float pref, bool speed) {
   constexpr int NV = (PHYS == 1) ? 3 : ND;
@@ -130,10 +134,10 @@ __device__ __forceinline__ float spec_primitive(float (&u)[NC], float gamma, flo
     u[1 + d] = vel[d];
   }
   if constexpr (PHYS == 0) {
-    const float pr = g1 * (u[NC - 1] - 0.5f * rho * kin);
+    const float pr = __fmul_rn(g1, fmaf(-0.5f * rho, kin, u[NC - 1]));
     u[NC - 1] = pr;
     if (!speed) return 0.0f;
-    const float cs = sqrtf(gamma * (pr + pref) * rinv);
+    const float cs = sqrtf(gamma * __fadd_rn(pr, pref) * rinv);
     float um = fabsf(vel[0]);
     if (ND == 3) um = fmaxf(um, fmaxf(fabsf(vel[1]), fabsf(vel[NV - 1])));
     return um + cs;  // 2D keeps |u_x| + a only (equations.py:137-147)
@@ -188,7 +192,7 @@ __device__ __forceinline__ void spec_fluxes(const SpecXArgs& a, const PF& pf, co
       if (j == decltype(jc)::value) f(jc);
     });
   };
-  const float href = a.gamma * er;
+  const float href = __fmul_rn(a.gamma, er);
   const float ig1 = 1.0f / g1;
   // Euler flux pair j = (F_2j, F_2j+1) along the (runtime) direction dir.
   // The direction enters by selects, so one body per pair serves the ND
@@ -198,7 +202,7 @@ __device__ __forceinline__ void spec_fluxes(const SpecXArgs& a, const PF& pf, co
   auto flux_pair = [&](auto jc, int dir, int n2) -> float2 {
     constexpr int c = 2 * decltype(jc)::value;
     const float un = (dir == 0) ? q(1, n2) : (ND == 2 || dir == 1) ? q(2, n2) : q((ND == 3) ? 3 : 2, n2);
-    const float mn = q(0, n2) * un;
+    const float mn = __fmul_rn(q(0, n2), un);
     auto comp = [&](auto cc) -> float {
       constexpr int C = decltype(cc)::value;
       const float pr = q(NC - 1, n2);
@@ -207,10 +211,10 @@ __device__ __forceinline__ void spec_fluxes(const SpecXArgs& a, const PF& pf, co
         float kin = 0.0f;
 #pragma unroll
         for (int d = 0; d < ND; ++d) kin = fmaf(q(1 + d, n2), q(1 + d, n2), kin);
-        const float Ep = fmaf(pr, ig1, 0.5f * q(0, n2) * kin);  // E' = E - E_ref
-        return ((Ep + pr) + href) * un;                         // (E + p) u_dir
+        const float Ep = fmaf(pr, ig1, __fmul_rn(0.5f * q(0, n2), kin));      // E' = E - E_ref
+        return __fmul_rn(__fadd_rn(__fadd_rn(Ep, pr), href), un);  // (E + p) u_dir
       }
-      return mn * q(C, n2) + ((C - 1 == dir) ? pr : 0.0f);
+      return fmaf(mn, q(C, n2), (C - 1 == dir) ? pr : 0.0f);
     };
     float2 f = make_float2(comp(std::integral_constant<int, c>{}), 0.0f);
     if constexpr (c + 1 < NC) f.y = comp(std::integral_constant<int, c + 1>{});
@@ -311,7 +315,7 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_spec_x(SpecXArgs a) {
   const float er = (PHYS == 0) ? a.eref[sol] : 0.0f;
   const float eshift = a.shift_in ? er : 0.0f;
   const float g1 = a.gamma - 1.0f;
-  const float pref = g1 * er;
+  const float pref = __fmul_rn(g1, er);
   constexpr int CE = (PHYS == 1) ? 4 : NC - 1;  // energy component
   float q[NC][B];
 #pragma unroll
@@ -512,7 +516,7 @@ __global__ void __launch_bounds__(32 * NG, (PHYS == 1) ? 4 : 0) k_spec_xs(SpecXA
     const float er = (PHYS == 0) ? a.eref[sol] : 0.0f;
     const float eshift = a.shift_in ? er : 0.0f;
     const float g1 = a.gamma - 1.0f;
-    const float pref = g1 * er;
+    const float pref = __fmul_rn(g1, er);
     constexpr int CE = (PHYS == 1) ? 4 : NC - 1;
     auto slot = [&](int c, int n2) -> float& { return S.q[c][n2 * 32 + lane]; };
     // this thread's points in the middle part are n2 = grp + NG i; the stage

@@ -1,0 +1,55 @@
+"""A solve ends on the same bits alone and in a batch, whatever kernel shapes
+the batch's size selects: the Euler x rows in one warp per row group or in
+several that share them (csrc/spec_launch.cuh), each at sizes on both sides of
+that choice.  The arithmetic of a value is the same in every shape, so the
+tolerance is zero."""
+import numpy as np
+import pytest
+
+from test_gpu_truncated_spectra import euler_state
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+FP = {"enabled": True, "p": 8, "alpha": 36.0}
+
+
+def same_alone(U0, nsolve, run, **kw):
+    """run(plan, states) on a batch that repeats the states of U0, and on each alone."""
+    from phrike_gb300.engine import Plan
+    shape = U0.shape[2:]
+    lengths = (1.0,) * len(shape)
+    index = torch.arange(nsolve, device="cuda") % len(U0)
+    first = torch.as_tensor(U0.astype(np.float32), device="cuda")
+    batch = Plan(shape, lengths, nsolve=nsolve, **kw)
+    got = run(batch, first[index].contiguous())
+    for i in sorted({0, 1, min(2, nsolve - 1), nsolve // 2, nsolve - 1}):
+        V = run(Plan(shape, lengths, **kw), first[index[i]].clone())  # (a plan of its own: cadences count its steps)
+        assert torch.equal(got[i], V), (i, float((got[i] - V).abs().max()))
+    assert batch.status() == 0
+
+
+@pytest.mark.parametrize("filt,interval", [(None, 1), (FP, 1), (FP, 2)])
+@pytest.mark.parametrize("shape,nsolve", [((8, 8), 2500), ((8, 16), 1300), ((8, 32), 1300), ((64, 64), 80),
+                                          ((8, 128), 640), ((8, 256), 320), ((512, 512), 3), ((8, 8, 8), 320),
+                                          ((64, 64, 64), 2), ((8, 9, 128), 72)], ids=str)
+def test_euler_steps(shape, nsolve, filt, interval):
+    U0 = np.stack([euler_state(shape, i) for i in range(3)])
+    U0[2, -1] *= 0.45  # pressures below zero: the 2D clamp acts
+    U0[2, -1] += 0.3
+    dt = 0.02 / max(shape)
+    same_alone(U0, nsolve, lambda p, U: p.run_(U, 3, dt), filter_params=dict(filt or {}, interval=interval))
+
+
+@pytest.mark.parametrize("shape,nsolve", [((8, 8), 2500), ((9, 8), 2500), ((8, 16), 1300), ((8, 32), 1300),
+                                          ((64, 64), 80), ((8, 128), 640), ((8, 256), 320), ((512, 512), 3),
+                                          ((8, 8, 8), 320), ((64, 64, 64), 2)], ids=str)
+def test_euler_cfl_steps(shape, nsolve):
+    U0 = np.stack([euler_state(shape, i) for i in range(3)])
+
+    def run(plan, U):
+        f64 = dict(dtype=torch.float64, device="cuda")
+        plan.run_cfl_(U, 3, torch.zeros(plan.nsolve, **f64), torch.full((plan.nsolve,), 1.0, **f64))
+        return U
+
+    same_alone(U0, nsolve, run, filter_params=FP, cfl=0.3)
