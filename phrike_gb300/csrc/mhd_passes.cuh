@@ -297,12 +297,14 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_proj_y(ProjArgs a) {
       continue;
     }
     const float kyp = a.ky0 * (float)((k < N / 2) ? k : k - N);
-    const float k2 = kxp * kxp + kyp * kyp;
+    // products and sums rounded as written at every tile width (a solve gives
+    // the same bits alone and in a batch)
+    const float k2 = fmaf(kxp, kxp, __fmul_rn(kyp, kyp));
     const float inv = (k2 == 0.0f) ? 1.0f : 1.0f / k2;
-    const float cr = (kxp * X[r].x + kyp * Y[r].x) * inv;
-    const float ci = (kxp * X[r].y + kyp * Y[r].y) * inv;
-    X[r] = make_float2((X[r].x - kxp * cr) * scale, (X[r].y - kxp * ci) * scale);
-    Y[r] = make_float2((Y[r].x - kyp * cr) * scale, (Y[r].y - kyp * ci) * scale);
+    const float cr = __fmul_rn(fmaf(kxp, X[r].x, __fmul_rn(kyp, Y[r].x)), inv);
+    const float ci = __fmul_rn(fmaf(kxp, X[r].y, __fmul_rn(kyp, Y[r].y)), inv);
+    X[r] = make_float2(__fmul_rn(fmaf(-kxp, cr, X[r].x), scale), __fmul_rn(fmaf(-kxp, ci, X[r].y), scale));
+    Y[r] = make_float2(__fmul_rn(fmaf(-kyp, cr, Y[r].x), scale), __fmul_rn(fmaf(-kyp, ci, Y[r].y), scale));
   }
   pf.inv(X);
   pf.inv(Y);
@@ -370,7 +372,8 @@ __global__ void __launch_bounds__(Shape<N>::A * T) k_proj_xi(ProjArgs a) {
     if (e != nullptr) {
 #pragma unroll
       for (int n2 = 0; n2 < B; ++n2)
-        e[t + A * n2] = oe[n2] + 0.5f * ((z[n2].x * z[n2].x + z[n2].y * z[n2].y) - (ox[n2] * ox[n2] + oy[n2] * oy[n2]));
+        e[t + A * n2] = fmaf(0.5f, fmaf(z[n2].x, z[n2].x, __fmul_rn(z[n2].y, z[n2].y)) -
+                                       fmaf(ox[n2], ox[n2], __fmul_rn(oy[n2], oy[n2])), oe[n2]);
     }
 #pragma unroll
     for (int n2 = 0; n2 < B; ++n2) {

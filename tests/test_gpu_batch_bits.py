@@ -1,12 +1,12 @@
 """A solve ends on the same bits alone and in a batch, whatever kernel shapes
 the batch's size selects: the Euler x rows in one warp per row group or in
-several that share them (csrc/spec_launch.cuh), each at sizes on both sides of
-that choice.  The arithmetic of a value is the same in every shape, so the
+several that share them (csrc/spec_launch.cuh), the MHD projection's tile
+widths (csrc/mhd_passes.cuh), each at sizes on both sides of the choice.  The arithmetic of a value is the same in every shape, so the
 tolerance is zero."""
 import numpy as np
 import pytest
 
-from test_gpu_truncated_spectra import euler_state
+from test_gpu_truncated_spectra import euler_state, mhd_state
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
@@ -53,3 +53,14 @@ def test_euler_cfl_steps(shape, nsolve):
         return U
 
     same_alone(U0, nsolve, run, filter_params=FP, cfl=0.3)
+
+
+@pytest.mark.parametrize("shape,nsolve", [((8, 8), 2500), ((16, 256), 300), ((256, 16), 300), ((256, 32), 512),
+                                          ((64, 64), 80), ((512, 8), 200), ((8, 512), 200), ((1024, 8), 40),
+                                          ((16, 16, 16), 40), ((64, 8, 32), 20)], ids=str)
+@pytest.mark.parametrize("options", [{}, {"project_each_substage": False}, {"resistivity": 1e-3}], ids=str)
+def test_mhd_steps(shape, nsolve, options):
+    U0 = np.stack([mhd_state(shape, i) for i in range(3)])
+    dt = 0.02 / max(shape)
+    same_alone(U0, nsolve, lambda p, U: p.run_(U, 2, dt), filter_params=FP, equations="mhd", mhd_config=options,
+               gamma=5.0 / 3.0)
