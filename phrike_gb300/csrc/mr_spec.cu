@@ -1,5 +1,6 @@
 // Truncated-spectra passes for 5-smooth axes (see mr_spec.cuh).
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <math.h>
 
 #include <vector>
@@ -378,6 +379,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_mrs_x(SpecXArgs a, SpecAxis ax,
 }
 
 // ---------------------------------------------------------------- strided
+// One CTA per tile of columns and outer index (plane, or solve and outer line),
+// tiles fastest, all in gridDim.x: planes times solves pass the 65535 of gridDim.y.
+__device__ __forceinline__ int outer_of(int ncol, int lt, int* col0) {
+  const int tiles = (ncol + (1 << lt) - 1) >> lt;
+  const int o = blockIdx.x / tiles;
+  *col0 = (blockIdx.x - o * tiles) << lt;
+  return o;
+}
+
 // rows x T tile -> shared memory, row i at element at[i], 16 bytes at a time
 template <typename At>
 __device__ __forceinline__ void tile_in(float2* dst, int lt, int rows, const float2* src, long as, int col0, int ncol,
@@ -397,7 +407,8 @@ __global__ void __launch_bounds__(MAXT, 1) k_mrs_f(SpecFArgs a, SpecAxis ax, int
   const int T = 1 << lt, n = ax.n, M = 2 * ax.km + 1;
   const int stride = ax.len << lt;
   float2* buf = sm;
-  const int plane = blockIdx.y, col0 = blockIdx.x * T;
+  int col0;
+  const int plane = outer_of(a.ncol, lt, &col0);
   const Tables tb = load_tables(buf + 2 * stride, ax);
   dep_wait();
   if (a.active != nullptr && a.active[plane / a.pps] == 0) {
@@ -442,7 +453,8 @@ __global__ void __launch_bounds__(MAXT, 1) k_mrs_c(SpecCArgs a, SpecAxis ax, int
   const int T = 1 << lt, n = ax.n;
   const int stride = ax.len << lt;
   float2* buf = sm;
-  const int outer = blockIdx.y % a.nouter, sol = blockIdx.y / a.nouter, col0 = blockIdx.x * T;
+  int col0;
+  const int o = outer_of(a.ncol, lt, &col0), outer = o % a.nouter, sol = o / a.nouter;
   const Tables tb = load_tables(buf + 2 * stride, ax);
   dep_wait();
   if (a.active != nullptr && a.active[sol] == 0) {
@@ -505,7 +517,8 @@ __global__ void __launch_bounds__(MAXT, 1) k_mrs_i(SpecIArgs a, SpecAxis ax, int
   extern __shared__ __align__(16) float2 sm[];
   const int T = 1 << lt, n = ax.n, M = 2 * ax.km + 1;
   float2* buf = sm;
-  const int plane = blockIdx.y, col0 = blockIdx.x * T;
+  int col0;
+  const int plane = outer_of(a.ncol, lt, &col0);
   const Tables tb = load_tables(buf + (ax.len << lt), ax);
   dep_wait();
   if (a.active != nullptr && a.active[plane / a.pps] == 0) {
@@ -753,7 +766,9 @@ cudaError_t launch_mrs_x(int nd, bool inc, bool flux, const SpecXArgs& a, const 
     size_t sm = 0;                                                                             \
     const int lt = strided_lt(ax, NSIG, a.ncol, OUTER, &sm);                                   \
     const int threads = strided_threads(ax, lt, NSIG);                                         \
-    const dim3 grid((a.ncol + (1 << lt) - 1) >> lt, OUTER);                                    \
+    const long ctas = (long)((a.ncol + (1 << lt) - 1) >> lt) * (OUTER);                        \
+    if (ctas > INT_MAX) return cudaErrorInvalidConfiguration;                                  \
+    const int grid = (int)ctas;                                                                \
     cudaError_t e;                                                                             \
     if (threads > kThreads) {                                                                  \
       if ((e = set_smem(KERNEL<kWide>, kSmemMax)) != cudaSuccess) return e;                    \
@@ -763,7 +778,7 @@ cudaError_t launch_mrs_x(int nd, bool inc, bool flux, const SpecXArgs& a, const 
     return launch_dep(KERNEL<kThreads>, grid, threads, sm, s, a, ax, lt);                      \
   }
 PS_MRS_STRIDED(launch_mrs_f, SpecFArgs, k_mrs_f, 2, a.planes)
-PS_MRS_STRIDED(launch_mrs_c, SpecCArgs, k_mrs_c, 2, a.nouter * a.nsolve)
+PS_MRS_STRIDED(launch_mrs_c, SpecCArgs, k_mrs_c, 2, (long)a.nouter * a.nsolve)
 PS_MRS_STRIDED(launch_mrs_i, SpecIArgs, k_mrs_i, 1, a.planes)
 
 cudaError_t launch_mrs_filter(const MrFilterArgs& a, const SpecAxis& ax, int nsolve, cudaStream_t s) {

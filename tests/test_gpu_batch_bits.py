@@ -64,3 +64,19 @@ def test_mhd_steps(shape, nsolve, options):
     dt = 0.02 / max(shape)
     same_alone(U0, nsolve, lambda p, U: p.run_(U, 2, dt), filter_params=FP, equations="mhd", mhd_config=options,
                gamma=5.0 / 3.0)
+
+
+@pytest.mark.parametrize("shape,nsolve", [((15, 6, 5), 4400), ((5, 27, 5), 3500)], ids=str)
+def test_euler_batches_of_many_planes(shape, nsolve):
+    """3D grids on 2^a 3^b 5^c axes whose planes (first) or kept y modes
+    (second) times solves pass 65535, the limit of two of a launch's three
+    grid dimensions."""
+    U0 = np.stack([euler_state(shape, i) for i in range(3)])
+
+    def run(plan, U):
+        f64 = dict(dtype=torch.float64, device="cuda")
+        plan.run_(U, 2, 0.02 / max(shape))
+        plan.run_cfl_(U, 2, torch.zeros(plan.nsolve, **f64), torch.full((plan.nsolve,), 1.0, **f64))
+        return U
+
+    same_alone(U0, nsolve, run, filter_params=FP, cfl=0.3)
