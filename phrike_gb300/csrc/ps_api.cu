@@ -1197,6 +1197,11 @@ int spec_last(ps_plan p, const SpecBufs& b, int stage, double dt, const double* 
 int steps_spec(ps_plan p, float* U, int nsteps, double dt, const double* d_dt, double* d_t, const double* d_tend,
                cudaStream_t s, ps::StepLimits lim = {}) {
   int rc;
+  // the filter passes hold the solves (power-of-two 3D grids: planes times
+  // solves) in gridDim.y; refused here, while U is still as given
+  if ((long)p->nsolve * ((p->nd == 3 && !p->mr) ? p->n[2] : 1) > 65535)
+    return fail(PS_ERR_UNSUPPORTED, "a batch of %d solves is too large to step (at most 65535%s)", p->nsolve,
+                (p->nd == 3 && !p->mr) ? " planes of all solves" : "");
   const SpecBufs b = spec_bufs(p);
   const bool cfl = d_t != nullptr;
   const int* act = cfl ? p->active : nullptr;

@@ -80,3 +80,18 @@ def test_euler_batches_of_many_planes(shape, nsolve):
         return U
 
     same_alone(U0, nsolve, run, filter_params=FP, cfl=0.3)
+
+
+@pytest.mark.parametrize("shape,nsolve", [((8, 8), 65536), ((9, 8), 65536), ((8, 8, 8), 8192)], ids=str)
+def test_batches_past_the_launch_limits_leave_the_state_alone(shape, nsolve):
+    from phrike_gb300.engine import Plan
+    U0 = torch.as_tensor(euler_state(shape, 0).astype(np.float32), device="cuda").expand(nsolve, -1, *shape).contiguous()
+    plan = Plan(shape, (1.0,) * len(shape), nsolve=nsolve, filter_params=FP, cfl=0.3)
+    f64 = dict(dtype=torch.float64, device="cuda")
+    t, end = torch.zeros(nsolve, **f64), torch.full((nsolve,), 1.0, **f64)
+    for run in (lambda U: plan.run_(U, 2, 1e-3), lambda U: plan.run_cfl_(U, 2, t, end)):
+        U = U0.clone()
+        with pytest.raises(RuntimeError):
+            run(U)
+        assert torch.equal(U, U0)
+    assert float(t.abs().max()) == 0.0
