@@ -123,9 +123,10 @@ int eo_n_tile(int h, long mt) {
 // C[par][m][n] = sum_k A[par][m][k] B[par][n][k]: rows m = (solve, component,
 // line) of the operand, n < h.  One CTA per 128 x NT tile, 128 threads:
 // thread 0 issues the TMA loads, thread 32 the MMAs, all four warps drain
-// TMEM.  blockIdx.z = parity (+ 2 for y).  x products are stored as rows of
-// ldx; y products with the lanes along x (rows m = (solve, c, i) go to
-// [solve, c][n][i]).
+// TMEM.  blockIdx.x = column tile (fastest) and row tile, since the row tiles
+// of a batch pass the 65535 of gridDim.y; blockIdx.z = parity (+ 2 for y).  x
+// products are stored as rows of ldx; y products with the lanes along x (rows
+// m = (solve, c, i) go to [solve, c][n][i]).
 // ---------------------------------------------------------------------------
 template <int NT>
 struct EoSmem {
@@ -154,7 +155,8 @@ __global__ void __launch_bounds__(128, 1)
   const EoAxis& ax = ydir ? g.b.y : g.b.x;
   const int line = ydir ? g.b.x.n : g.b.y.n;  // lines per component
   const int M = g.nsolve * 4 * line, N = ax.h;
-  const int m0 = blockIdx.y * 128, n0 = blockIdx.x * NT;
+  const int mt = blockIdx.x / g.ntiles;
+  const int m0 = mt * 128, n0 = (blockIdx.x - mt * g.ntiles) * NT;
   if (m0 >= M || n0 >= N) return;
   const CUtensorMap* mA = ydir ? &mAy : &mAx;
   const CUtensorMap* mB = ydir ? &mBy : &mBx;
@@ -315,7 +317,7 @@ __global__ void __launch_bounds__(128, 1)
 
 namespace {
 template <int NT>
-cudaError_t eo_gemm_t(const EoGemmArgs& a, cudaStream_t s) {
+cudaError_t eo_gemm_t(EoGemmArgs a, cudaStream_t s) {
   constexpr int bytes = EoSmem<NT>::kBytes;
   cudaError_t e;
   if ((e = set_smem(k_eo_gemm<NT>, bytes)) != cudaSuccess) return e;
@@ -324,7 +326,8 @@ cudaError_t eo_gemm_t(const EoGemmArgs& a, cudaStream_t s) {
   const int rx = x ? a.nsolve * 4 * b.y.n : 0, ry = y ? a.nsolve * 4 * b.x.n : 0;
   const int hx = x ? b.x.h : 0, hy = y ? b.y.h : 0;
   const int rows = rx > ry ? rx : ry, h = hx > hy ? hx : hy;
-  const dim3 grid((h + NT - 1) / NT, (rows + 127) / 128, (x && y) ? 4 : 2);
+  a.ntiles = (h + NT - 1) / NT;
+  const dim3 grid(a.ntiles * ((rows + 127) / 128), 1, (x && y) ? 4 : 2);
   return launch_dep(k_eo_gemm<NT>, grid, 128, bytes, s, b.mX, a.filter ? b.mFx : b.mDx, b.mY,
                     a.filter ? b.mFy : b.mDy, a);
 }

@@ -82,6 +82,16 @@ def test_euler_batches_of_many_planes(shape, nsolve):
     same_alone(U0, nsolve, run, filter_params=FP, cfl=0.3)
 
 
+@pytest.mark.parametrize("shape,nsolve", [((65, 3), 32300), ((3, 65), 32300)], ids=str)
+@pytest.mark.parametrize("filt", [None, FP], ids=["plain", "filter"])
+def test_lgl_batches_of_many_rows(shape, nsolve, filt):
+    """Solves times rows of an LGL grid beyond 65535 tiles of 128."""
+    r = np.random.RandomState(0)
+    U0 = np.stack([euler_state(shape, i) for i in range(3)])
+    U0[:, 1:3] *= 0.1 + 0.01 * r.standard_normal(shape)
+    same_alone(U0, nsolve, lambda p, U: p.run_(U, 2, 1e-5), basis="legendre", filter_params=filt)
+
+
 @pytest.mark.parametrize("shape,nsolve", [((8, 8), 65536), ((9, 8), 65536), ((8, 8, 8), 8192)], ids=str)
 def test_batches_past_the_launch_limits_leave_the_state_alone(shape, nsolve):
     from phrike_gb300.engine import Plan
