@@ -106,9 +106,12 @@ typedef struct {
    * phrike_gb300/autotune.py picks it by timing. */
   int tile_cols;
   /* LGL x LGL plans with PS_GEMM_BF16X3: N tile of the tcgen05 contractions,
-   * 64, 128, 176 or 256 columns; 0 (default): the smallest tile whose grid
-   * fits one wave, else 256.  Every output element is the same dot product
-   * for every tile; phrike_gb300/autotune.py picks it by timing. */
+   * 64, 128, 176 or 256 columns; 0 (default): a rule on the grid and batch.
+   * Plans that step by even and odd parts (filter_interval 1, no gravity) take
+   * 48, 64, 80 or 144 columns in the half-size contractions of their steps for
+   * the four values, and the value itself in ps_rhs.  Every output element is
+   * the same dot product for every tile; phrike_gb300/autotune.py picks it by
+   * timing. */
   int umma_n_tile;
 } ps_plan_desc;
 

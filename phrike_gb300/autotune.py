@@ -6,9 +6,11 @@
   and fewer, larger CTAs; narrower ones more CTAs for small grids and
   batches.
 * The tcgen05 contractions of LGL plans at split-BF16x3 compute 128 x NT
-  output tiles, NT = 64, 128, 176 or 256 (``umma_n_tile``), with a TMA ring
-  of 2-3 stages in 100-210 KB of shared memory: wider tiles re-read the D
-  matrix less, narrower ones keep more stages of smaller loads in flight.
+  output tiles.  ``umma_n_tile`` 64, 128, 176 or 256 selects NT = 48, 64, 80
+  or 144 for the half-size contractions of steps by even and odd parts (filter
+  after every step, no gravity) and is NT itself in the other plans and in
+  ``rhs``.  Wider tiles read the row operand less often and run in fewer
+  waves, narrower ones fill the SMs of a small grid.
 
 The arithmetic of every output value is the same for every choice, so it
 changes speed only.  The tuners build the plan at each allowed value, time a

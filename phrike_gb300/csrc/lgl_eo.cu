@@ -105,10 +105,9 @@ int encode_eo_map(CUtensorMap* m, const void* base, int h, int rows, int kp, int
 // 513 nodes (257 pairs) alone take 144 columns (136 CTAs, one wave), 257 nodes
 // (129 pairs) 48 (108 CTAs).
 int eo_n_tile(int h, long mt) {
-  const int cand[4] = {48, 64, 80, 144};
   int best = 144;
   long cost = -1;
-  for (int nt : cand) {
+  for (int nt : kEoTiles) {
     const long waves = (mt * ((h + nt - 1) / nt) + 147) / 148;
     const long c = waves * (nt + 64);
     if (cost < 0 || c < cost) {
@@ -334,8 +333,13 @@ cudaError_t eo_gemm_t(EoGemmArgs a, cudaStream_t s) {
 }  // namespace
 
 cudaError_t launch_eo_gemm(const EoGemmArgs& a, cudaStream_t s) {
-  const int nt = a.b.ntx;  // one tile for both directions (maps are encoded with it)
-  return nt == 48 ? eo_gemm_t<48>(a, s) : nt == 64 ? eo_gemm_t<64>(a, s) : nt == 80 ? eo_gemm_t<80>(a, s) : eo_gemm_t<144>(a, s);
+  switch (a.b.ntx) {  // one tile for both directions (maps are encoded with it)
+    case kEoTiles[0]: return eo_gemm_t<kEoTiles[0]>(a, s);
+    case kEoTiles[1]: return eo_gemm_t<kEoTiles[1]>(a, s);
+    case kEoTiles[2]: return eo_gemm_t<kEoTiles[2]>(a, s);
+    case kEoTiles[3]: return eo_gemm_t<kEoTiles[3]>(a, s);
+    default: return cudaErrorInvalidValue;
+  }
 }
 
 // ---------------------------------------------------------------------------

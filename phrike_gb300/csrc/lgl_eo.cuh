@@ -6,6 +6,8 @@
 namespace ps {
 
 constexpr int kEoParts = 3;  // bf16 parts of an operand
+// N tiles of the contractions; ps_plan_desc.umma_n_tile 64, 128, 176, 256 in turn
+constexpr int kEoTiles[4] = {48, 64, 80, 144};
 
 // One axis: n nodes, h = ceil(n/2) mirrored pairs (the centre of an odd n is
 // its own mirror), split matrices and the operand pitch.

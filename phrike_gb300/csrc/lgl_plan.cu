@@ -87,6 +87,8 @@ bool eo_plan(const ps_plan_desc* d) {
          d->filter_interval == 1 && d->gravity[0] == 0.0 && d->gravity[1] == 0.0;
 }
 
+constexpr int kUmmaTiles[4] = {64, 128, 176, 256};  // values of ps_plan_desc.umma_n_tile
+
 struct EoSizes {
   int hx, hy, kx, ky, ldx;
   size_t X, Y, mats, C;  // bf16 elements of the operands and matrices, floats of the products
@@ -115,6 +117,9 @@ int eo_setup(ps_plan p) {
   b.ldx = z.ldx;
   const int nmax = p->n[0] > p->n[1] ? p->n[0] : p->n[1];
   b.ntx = eo_n_tile(z.hx > z.hy ? z.hx : z.hy, 4 * (((long)p->nsolve * 4 * nmax + 127) / 128));
+  if (p->gemm == PS_GEMM_BF16X3 && p->desc.umma_n_tile != 0)  // an explicit tile (autotuner)
+    for (int i = 0; i < 4; ++i)
+      if (p->desc.umma_n_tile == kUmmaTiles[i]) b.ntx = kEoTiles[i];
   unsigned short *X = nullptr, *Y = nullptr, *M = nullptr;
   if ((rc = plan_alloc(p, &X, z.X)) != PS_OK || (rc = plan_alloc(p, &Y, z.Y)) != PS_OK ||
       (rc = plan_alloc(p, &M, z.mats)) != PS_OK || (rc = plan_alloc(p, &b.CX, z.C)) != PS_OK)
@@ -510,7 +515,9 @@ int lgl_setup(ps_plan p) {
     p->nt_y = umma_n_tile(nx, ny, p->nsolve * 4);
     const int nt = p->desc.umma_n_tile;
     if (nt != 0) {  // an explicit tile (autotuner)
-      if (nt != 64 && nt != 128 && nt != 176 && nt != 256)
+      bool known = false;
+      for (int t : kUmmaTiles) known = known || nt == t;
+      if (!known)
         return errorf(PS_ERR_INVALID, "umma_n_tile must be 0, 64, 128, 176 or 256 (got %d)", nt);
       p->nt_x = p->nt_y = nt;
     }
