@@ -1,10 +1,10 @@
 """Tile autotuning by measurement.
 
-* The strided passes of 2D Fourier plans (the y pass of the right-hand side,
-  the filter and the operators) process ``tile_cols`` adjacent columns per
-  CTA: 4, 8 or 16 (at most the plan's cap).  Wider tiles make longer TMA rows
-  and fewer, larger CTAs; narrower ones more CTAs for small grids and
-  batches.
+* The strided passes of 2D Fourier plans (the y pass of the steps and of the
+  right-hand side, the filter and the operators) process ``tile_cols``
+  adjacent columns per CTA: 4, 8 or 16 (at most the plan's cap, at least one
+  full warp).  Wider tiles make longer rows and fewer, larger CTAs; narrower
+  ones more CTAs for small grids and batches.
 * The tcgen05 contractions of LGL plans at split-BF16x3 compute 128 x NT
   output tiles.  ``umma_n_tile`` 64, 128, 176 or 256 selects NT = 48, 64, 80
   or 144 for the half-size contractions of steps by even and odd parts (filter

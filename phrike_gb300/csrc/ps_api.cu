@@ -1178,6 +1178,7 @@ int spec_last(ps_plan p, const SpecBufs& b, int stage, double dt, const double* 
   c.dt_dev = d_dt;
   c.dt = dt;
   c.active = act;
+  c.tile = (p->nd == 2 && !p->mr) ? p->desc.tile_cols : 0;
   const double in = 8.0 * b.ncol * p->n[ax] * c.nouter * p->nsolve;
   const double ac = in * ps::spec_modes(p->n[ax]) / p->n[ax];
   ProfScope prof(p, s, PS_KIND_LAST, 3.0 * in + ac * (stage == 0 || stage == 3 ? 1 : 2));

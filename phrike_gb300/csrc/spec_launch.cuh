@@ -8,17 +8,19 @@
 
 namespace ps {
 
-// Columns per CTA of the strided passes: the largest of 16, 8 and 4 (8 and 4
-// at 1024 points; a CTA has at least one full warp) that gives two CTAs per
-// SM.  A pencil's arithmetic does not depend on it.
+// Columns per CTA of the strided passes: asked for (ps_plan_desc.tile_cols, the
+// nearest width that is built), or the largest of 16, 8 and 4 (8 and 4 from 512
+// points; a CTA has at least one full warp) that gives two CTAs per SM.  A
+// pencil's arithmetic does not depend on it.
 template <int NN, typename F>
-cudaError_t dispatch_spec_cols(int ncol, long outer, F&& f) {
+cudaError_t dispatch_spec_cols(int ncol, long outer, int asked, F&& f) {
   constexpr int TMAX = (NN >= 512) ? 8 : 16;
   constexpr int TMIN = cmax_int(4, 32 / Shape<NN>::A);
+  auto take = [&](int T) { return asked > 0 ? asked >= T : (ncol + T - 1) / T * outer >= 2L * 148; };
   if constexpr (TMAX >= 16 && TMIN < 16)
-    if ((ncol + 15) / 16 * outer >= 2L * 148) return f(std::integral_constant<int, 16>{});
+    if (take(16)) return f(std::integral_constant<int, 16>{});
   if constexpr (TMIN < 8 && TMAX >= 8)
-    if ((ncol + 7) / 8 * outer >= 2L * 148) return f(std::integral_constant<int, 8>{});
+    if (take(8)) return f(std::integral_constant<int, 8>{});
   return f(std::integral_constant<int, TMIN>{});
 }
 
@@ -77,9 +79,9 @@ cudaError_t spec_xs_mode(bool inc, bool flux, const SpecXArgs& a, cudaStream_t s
 #define PS_DEFINE_SPEC_STRIDED(NN, NAME, ARGS, KERNEL, SMEM, OUTER)                                   \
   template <>                                                                                         \
   cudaError_t NAME<NN>(const ARGS& a, cudaStream_t s) {                                               \
-    return dispatch_spec_cols<NN>(a.ncol, OUTER, [&](auto tw) -> cudaError_t {                        \
+    return dispatch_spec_cols<NN>(a.ncol, OUTER, a.tile, [&](auto tw) -> cudaError_t {                \
       constexpr int T = decltype(tw)::value;                                                          \
-      const size_t sm = sizeof(SMEM<NN, T>);                                                                \
+      const size_t sm = sizeof(SMEM<NN, T>);                                                          \
       cudaError_t e;                                                                                  \
       int grid;                                                                                       \
       if ((e = set_smem(KERNEL<NN, T>, sm)) != cudaSuccess) return e;                                 \

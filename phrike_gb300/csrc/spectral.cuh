@@ -739,6 +739,7 @@ struct SpecFArgs {
   int planes, pps;   // planes of all solves, of one solve
   AxisOps ax;
   const int* active;
+  int tile;          // columns per tile, 0: by rule
 };
 
 template <int N, int T>
@@ -834,6 +835,7 @@ struct SpecCArgs {
   const double* dt_dev;
   double dt;
   const int* active;
+  int tile;          // columns per tile, 0: by rule
 };
 
 template <int N, int T>
@@ -948,6 +950,7 @@ struct SpecIArgs {
   int planes, pps;
   AxisOps ax;
   const int* active;
+  int tile;           // columns per tile, 0: by rule
 };
 
 template <int N, int T>
