@@ -294,8 +294,13 @@ cudaError_t launch_conserved(int nd, const float* U, long cells, long ss, int ns
                              cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(out, 0, sizeof(double) * (nd + 2) * nsolve, s);
   if (e != cudaSuccess) return e;
-  // four cells per thread: the blocks' float64 atomics queue on nd + 2 words
-  const dim3 grid(reduce_blocks((cells + 3) / 4, nsolve), nsolve);
+  // a cell per thread, four from four blocks per SM: there the blocks' float64
+  // atomics, which queue on nd + 2 words, take longer than the cells (one against
+  // four cells: 64^2 10.3 / 18.4 us, 256^2 14.4 / 18.5, 512^2 37.0 / 30.8, 64^3
+  // 46.6 / 38.6, 64^2 x 128 66.5 / 57.0; equal from 2 M cells)
+  int blocks = reduce_blocks(cells, nsolve);
+  if ((long)blocks * nsolve >= 4L * 152) blocks = reduce_blocks((cells + 3) / 4, nsolve);
+  const dim3 grid(blocks, nsolve);
   if (nd == 1) k_conserved<1><<<grid, 256, 0, s>>>(U, cells, ss, gamma, out);
   else if (nd == 2) k_conserved<2><<<grid, 256, 0, s>>>(U, cells, ss, gamma, out);
   else k_conserved<3><<<grid, 256, 0, s>>>(U, cells, ss, gamma, out);
