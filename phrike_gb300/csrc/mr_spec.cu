@@ -3,6 +3,7 @@
 #include <limits.h>
 #include <math.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "launch.cuh"
@@ -542,9 +543,10 @@ __global__ void __launch_bounds__(MAXT, 1) k_mrs_i(SpecIArgs a, SpecAxis ax, int
 
 // ---------------------------------------------------------------- filter
 // Complementary filter along one axis, pairs of real fields in one complex
-// signal.  ROWS (x): pg pencils per CTA; strided: T adjacent pencils.
-template <bool ROWS>
-__global__ void __launch_bounds__(kThreads, 1) k_mrs_filter(MrFilterArgs a, SpecAxis ax, int lt) {
+// signal.  ROWS (x): T pencils of one solve per CTA; strided: T adjacent pencils.
+// PER: CTAs per SM that the registers are cut for.
+template <bool ROWS, int PER>
+__global__ void __launch_bounds__(kThreads, PER) k_mrs_filter(MrFilterArgs a, SpecAxis ax, int lt) {
   extern __shared__ __align__(16) float2 sm[];
   const int n = ax.n, T = 1 << lt;
   const int stride = ROWS ? ax.len : ax.len << lt;
@@ -781,26 +783,44 @@ PS_MRS_STRIDED(launch_mrs_f, SpecFArgs, k_mrs_f, 2, a.planes)
 PS_MRS_STRIDED(launch_mrs_c, SpecCArgs, k_mrs_c, 2, (long)a.nouter * a.nsolve)
 PS_MRS_STRIDED(launch_mrs_i, SpecIArgs, k_mrs_i, 1, a.planes)
 
+namespace {
+// Registers of the filter pass: 128 a thread while all CTAs run at once that way,
+// else 64 (with a few spills), where more of them fit an SM beside one another.
+// 128 against 64: 480^2 46.0 / 49.3 us, 96 x 90 x 32 35.7 / 39.2; 540 x 960 84.5 /
+// 58.0, 90 x 96 x 100 177 / 133, 250^2 x 32 240 / 178, 3840 x 2160 795 / 736.
+template <bool ROWS>
+cudaError_t mrs_filter(const MrFilterArgs& a, const SpecAxis& ax, dim3 grid, int threads, size_t sm, int lt,
+                       cudaStream_t s) {
+  cudaError_t e;
+  auto per_sm = [&](int regs) { return std::min(65536 / (regs * threads), (int)((227 * 1024) / (sm + 1024))); };
+  if (per_sm(64) > per_sm(128) && (long)grid.x * grid.y * grid.z > 152L * per_sm(128)) {
+    if ((e = set_smem(k_mrs_filter<ROWS, 2>, kSmemMax)) != cudaSuccess) return e;
+    return launch_dep(k_mrs_filter<ROWS, 2>, grid, threads, sm, s, a, ax, lt);
+  }
+  if ((e = set_smem(k_mrs_filter<ROWS, 1>, kSmemMax)) != cudaSuccess) return e;
+  return launch_dep(k_mrs_filter<ROWS, 1>, grid, threads, sm, s, a, ax, lt);
+}
+}  // namespace
+
 cudaError_t launch_mrs_filter(const MrFilterArgs& a, const SpecAxis& ax, int nsolve, cudaStream_t s) {
   const int rmax = ax.radix[0], pairs = (a.nf + 1) / 2;
-  int lt;
+  auto tiles = [&](int l) { return (a.npen + (1L << l) - 1) >> l; };
+  auto bytes = [&](int l) { return ((size_t)(ax.len << l) + 2 * ax.n) * sizeof(float2); };
+  // one more doubling of the pencils per CTA, while that leaves two CTAs per SM
+  auto wider = [&](int l) { return tiles(l) > 1 && tiles(l + 1) * pairs * nsolve >= 2 * 152; };
+  const bool rows = a.es == 1;
+  int lt = 0;
   size_t sm;
-  cudaError_t e;
-  if (a.es == 1) {
-    lt = 0;
-    auto bytes = [&](int l) { return ((size_t)(ax.len << l) + 2 * ax.n) * sizeof(float2); };
-    while (lt < 6 && ((long)(ax.n / rmax) << lt) < 256 && bytes(lt + 1) <= kSmemMax / 3 &&
-           ((a.npen >> (lt + 1)) * pairs * nsolve) >= 2 * 148)
-      ++lt;
-    sm = bytes(lt);
-    if ((e = set_smem(k_mrs_filter<true>, kSmemMax)) != cudaSuccess) return e;
-    return launch_dep(k_mrs_filter<true>, dim3((unsigned)((a.npen + (1 << lt) - 1) >> lt), nsolve, pairs),
-                      threads_for((long)(ax.n / rmax) << lt), sm, s, a, ax, lt);
+  if (rows) {
+    while (lt < 6 && ((long)(ax.n / rmax) << lt) < 256 && bytes(lt + 1) <= kSmemMax / 3 && wider(lt)) ++lt;
+  } else {  // short axes: tiles of up to 1024 points
+    lt = strided_lt(ax, 1, a.npen, (long)pairs * nsolve, &sm);
+    while (lt >= 4 && lt < 8 && (ax.n << (lt + 1)) <= 1024 && wider(lt)) ++lt;
   }
-  lt = strided_lt(ax, 1, a.npen, (long)pairs * nsolve, &sm);
-  if ((e = set_smem(k_mrs_filter<false>, kSmemMax)) != cudaSuccess) return e;
-  return launch_dep(k_mrs_filter<false>, dim3((unsigned)((a.npen + (1 << lt) - 1) >> lt), nsolve, pairs),
-                    threads_for((long)(ax.n / rmax) << lt), sm, s, a, ax, lt);
+  sm = bytes(lt);
+  const dim3 grid((unsigned)tiles(lt), nsolve, pairs);
+  const int threads = threads_for((long)(ax.n / rmax) << lt);
+  return rows ? mrs_filter<true>(a, ax, grid, threads, sm, lt, s) : mrs_filter<false>(a, ax, grid, threads, sm, lt, s);
 }
 
 }  // namespace ps

@@ -1,7 +1,9 @@
 """A solve ends on the same bits alone and in a batch, whatever kernel shapes
 the batch's size selects: the Euler x rows in one warp per row group or in
 several that share them (csrc/spec_launch.cuh), the MHD projection's tile
-widths (csrc/mhd_passes.cuh), each at sizes on both sides of the choice.  The arithmetic of a value is the same in every shape, so the
+widths (csrc/mhd_passes.cuh), the tiles and registers of the filter on
+2^a 3^b 5^c axes (csrc/mr_spec.cu), each at sizes on both sides of the choice.
+The arithmetic of a value is the same in every shape, so the
 tolerance is zero."""
 import numpy as np
 import pytest
@@ -64,6 +66,14 @@ def test_mhd_steps(shape, nsolve, options):
     dt = 0.02 / max(shape)
     same_alone(U0, nsolve, lambda p, U: p.run_(U, 2, dt), filter_params=FP, equations="mhd", mhd_config=options,
                gamma=5.0 / 3.0)
+
+
+@pytest.mark.parametrize("shape,nsolve", [((9, 8), 2500), ((3, 1000), 200), ((2, 300), 300), ((6, 45), 500),
+                                          ((12, 10), 2000), ((96, 90), 64), ((250, 250), 8), ((3, 4096), 40),
+                                          ((15, 10, 12), 300), ((30, 30, 30), 8), ((4, 3, 250), 100)], ids=str)
+def test_filter_on_mixed_radix_axes(shape, nsolve):
+    U0 = np.stack([euler_state(shape, i) for i in range(3)])
+    same_alone(U0, nsolve, lambda p, U: p.filter(U), filter_params=FP)
 
 
 @pytest.mark.parametrize("shape,nsolve", [((15, 6, 5), 4400), ((5, 27, 5), 3500)], ids=str)
