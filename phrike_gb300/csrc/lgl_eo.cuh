@@ -44,7 +44,7 @@ struct EoGemmArgs {
   int filter;          // the filter's complements I - F instead of D
   const int* active;
   int* status;
-  int ntiles;          // column tiles (set by the launch)
+  int ntiles, stages;  // column tiles, ring depth (set by the launch)
 };
 cudaError_t launch_eo_gemm(const EoGemmArgs& a, cudaStream_t s);
 
