@@ -21,7 +21,7 @@ struct EoBufs {
   EoAxis x, y;
   void* X;     // x operand  [P][2 (even, odd)][nsolve*4*ny][x.kp]
   void* Y;     // y operand  [P][2][nsolve*4*nx][y.kp]
-  float* CX;   // x products [2][nsolve*4*ny][ldx], parity of the operand
+  float* CX;   // x products [2][nsolve*4*ny][ldx], parity of the operand (the plan's G)
   int ldx;
   float* CY;   // y products [2][nsolve*4][y.h][nx]
   CUtensorMap mX, mY, mDx, mDy, mFx, mFy;

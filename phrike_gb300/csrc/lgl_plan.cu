@@ -122,8 +122,9 @@ int eo_setup(ps_plan p) {
       if (p->desc.umma_n_tile == kUmmaTiles[i]) b.ntx = kEoTiles[i];
   unsigned short *X = nullptr, *Y = nullptr, *M = nullptr;
   if ((rc = plan_alloc(p, &X, z.X)) != PS_OK || (rc = plan_alloc(p, &Y, z.Y)) != PS_OK ||
-      (rc = plan_alloc(p, &M, z.mats)) != PS_OK || (rc = plan_alloc(p, &b.CX, z.C)) != PS_OK)
+      (rc = plan_alloc(p, &M, z.mats)) != PS_OK)
     return rc;
+  b.CX = p->G;  // sized for the products (lgl_g_floats)
   b.X = X;
   b.Y = Y;
   b.CY = b.CX + (size_t)2 * p->nsolve * 4 * p->n[1] * z.ldx;
@@ -164,8 +165,6 @@ int step_eo(ps_plan p, float* U, double dt, const double* dtp, bool shift_in, bo
   a.out = U;
   a.acc_in = p->acc;
   a.acc_out = p->Us;
-  a.S = p->G;
-  a.V = p->G + 4 * p->cells * p->nsolve;
   a.nsolve = p->nsolve;
   a.dt_dev = dtp;
   a.dt = dt;
@@ -204,6 +203,10 @@ int step_eo(ps_plan p, float* U, double dt, const double* dtp, bool shift_in, bo
     LGL_CU(launch_eo_stage(a, kEoStage, kEoOut, s), "LGL stage");
     return PS_OK;
   }
+  // the new state takes the increments' idle buffer, and the x-filtered state the
+  // other one, whose last readers are done by then
+  a.S = a.acc_out;
+  a.V = const_cast<float*>(a.acc_in);
   ProfScope prof(p, s, PS_KIND_OP, 24.0 * fb + 2.0 * op);
   LGL_CU(launch_eo_stage(a, kEoStage, kEoFilterX, s), "LGL stage and filter operand");
   g.filter = 1;
@@ -422,6 +425,15 @@ int lgl_validate(const ps_plan_desc* d) {
   return PS_OK;
 }
 
+// Floats of the plan's G: the flux derivatives (8 fields) or, from the same
+// buffer, the products of the even/odd contractions.
+size_t lgl_g_floats(const ps_plan_desc* d, int nsolve) {
+  const size_t g = (size_t)8 * d->n[0] * d->n[1] * nsolve;
+  if (!eo_plan(d)) return g;
+  const size_t c = eo_sizes(d, nsolve).C;
+  return c > g ? c : g;
+}
+
 size_t lgl_scratch_bytes(const ps_plan_desc* d, int nsolve) {
   size_t b = 0;
   if (d->ndim == 1) {
@@ -436,11 +448,12 @@ size_t lgl_scratch_bytes(const ps_plan_desc* d, int nsolve) {
   if (d->gemm_precision == PS_GEMM_BF16X3) {
     const size_t nx = d->n[0], ny = d->n[1], px = (nx + 7) / 8 * 8, py = (ny + 7) / 8 * 8;
     b += 4 * (nx * px + ny * py);                             // split D planes
-    b += 4 * 4 * (size_t)nsolve * (ny * px + nx * py);       // split flux planes
+    if (!eo_plan(d)) b += 4 * 4 * (size_t)nsolve * (ny * px + nx * py);  // split flux planes
   }
   if (eo_plan(d)) {
     const EoSizes e = eo_sizes(d, nsolve);
-    b += 2 * (e.X + e.Y + e.mats) + 4 * e.C;
+    b += 2 * (e.X + e.Y + e.mats);
+    b += 4 * (lgl_g_floats(d, nsolve) - (size_t)8 * d->n[0] * d->n[1] * nsolve);
   }
   return b;
 }
@@ -488,6 +501,7 @@ int lgl_setup(ps_plan p) {
     LGL_CU(cudaDeviceSynchronize(), "1D LGL tables");
     return PS_OK;
   }
+  if (eo_plan(&p->desc) && (rc = eo_setup(p)) != PS_OK) return rc;
   if (p->gemm == PS_GEMM_BF16X3) {
     const int nx = p->n[0], ny = p->n[1];
     p->pitch[0] = (nx + 7) / 8 * 8;
@@ -500,16 +514,26 @@ int lgl_setup(ps_plan p) {
       LGL_CU(launch_split_matrix(p->D32[a], n, n, p->pitch[a], q, 0), "split D");
       p->Dsplit[a] = q;
     }
-    unsigned short* fx = nullptr;
-    unsigned short* fyt = nullptr;
     const size_t nfx = 2 * (size_t)p->nsolve * 4 * ny * p->pitch[0];
     const size_t nfy = 2 * (size_t)p->nsolve * 4 * nx * p->pitch[1];
-    if ((rc = plan_alloc(p, &fx, nfx)) != PS_OK) return rc;
-    if ((rc = plan_alloc(p, &fyt, nfy)) != PS_OK) return rc;
-    LGL_CU(cudaMemset(fx, 0, sizeof(unsigned short) * nfx), "flux planes clear");
-    LGL_CU(cudaMemset(fyt, 0, sizeof(unsigned short) * nfy), "flux planes clear");
-    p->FX = fx;
-    p->FYT = fyt;
+    if (p->eo) {
+      // the two-part flux planes of ps_rhs take the operands' place (three parts
+      // of even and odd halves, so never smaller); what is loaded is written
+      // ahead of each load, and the maps end at the last node
+      const EoSizes z = eo_sizes(&p->desc, p->nsolve);
+      if (nfx > z.X || nfy > z.Y) return errorf(PS_ERR_CUDA, "flux planes exceed the even/odd operands");
+      p->FX = p->eob.X;
+      p->FYT = p->eob.Y;
+    } else {
+      unsigned short* fx = nullptr;
+      unsigned short* fyt = nullptr;
+      if ((rc = plan_alloc(p, &fx, nfx)) != PS_OK) return rc;
+      if ((rc = plan_alloc(p, &fyt, nfy)) != PS_OK) return rc;
+      LGL_CU(cudaMemset(fx, 0, sizeof(unsigned short) * nfx), "flux planes clear");
+      LGL_CU(cudaMemset(fyt, 0, sizeof(unsigned short) * nfy), "flux planes clear");
+      p->FX = fx;
+      p->FYT = fyt;
+    }
     // A operands (128-row boxes): D_x and F_y^T; B operands (N-tile boxes): F_x and D_y
     p->nt_x = umma_n_tile(nx, p->nsolve * 4 * ny, 1);
     p->nt_y = umma_n_tile(nx, ny, p->nsolve * 4);
@@ -529,7 +553,6 @@ int lgl_setup(ps_plan p) {
       return errorf(PS_ERR_CUDA, "tensor map encoding for the split contractions failed (%d)", e);
     LGL_CU(cudaDeviceSynchronize(), "split tables");
   }
-  if (eo_plan(&p->desc) && (rc = eo_setup(p)) != PS_OK) return rc;
   return PS_OK;
 }
 

@@ -208,6 +208,7 @@ int plan_alloc(ps_plan p, Tp** ptr, size_t count) {
 // LGL x LGL plans (lgl_plan.cu)
 int lgl_validate(const ps_plan_desc* d);
 size_t lgl_scratch_bytes(const ps_plan_desc* d, int nsolve);
+size_t lgl_g_floats(const ps_plan_desc* d, int nsolve);
 int lgl_setup(ps_plan p);
 int lgl_rhs(ps_plan p, const float* U, float* rhs, cudaStream_t s);
 int lgl_steps(ps_plan p, float* U, int nsteps, double dt, const double* d_dt, double* d_t, const double* d_tend,

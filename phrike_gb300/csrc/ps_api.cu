@@ -1506,7 +1506,7 @@ int create(const ps_plan_desc* d, int nsolve, ps_plan* out) {
   } else {
     const bool mhd3 = p->mhd && p->nd == 3;
     const int ng = mhd3 ? 24 : p->mhd ? 16 : (p->nd == 3) ? 15 : 8;
-    if ((rc = dalloc(p, &p->G, ng * c)) != PS_OK) return cleanup(rc);
+    if ((rc = dalloc(p, &p->G, lgl ? ps::lgl_g_floats(d, nsolve) : (size_t)ng * c)) != PS_OK) return cleanup(rc);
     const size_t hplanes = mhd3 ? (size_t)3 * p->n[2] * p->n[1] : (size_t)2 * p->n[1];
     if (p->mhd && (rc = dalloc(p, &p->H, hplanes * nsolve * (p->n[0] / 2 + 1))) != PS_OK) return cleanup(rc);
     if (p->mhd && (d->mhd_resistivity != 0.0 || d->mhd_viscosity != 0.0) &&
