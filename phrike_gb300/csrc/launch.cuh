@@ -206,6 +206,19 @@ cudaError_t dispatch_proj_cols(long units, F&& f) {
   return f(std::integral_constant<int, TMAX>{});
 }
 
+// k_line1d, from 16 points (line1d_plan; at 8 k_step1d steps)
+template <int N>
+cudaError_t line1d_n(const Step1DArgs& a, const float2* tw, int nsolve, cudaStream_t s) {
+  if constexpr (N >= 16) {
+    const size_t sm = sizeof(LineSmem<N>);
+    cudaError_t e;
+    if ((e = set_smem(k_line1d<N>, sm)) != cudaSuccess) return e;
+    return launch_dep(k_line1d<N>, nsolve, Line<N>::BLOCK, sm, s, a, tw);
+  } else {
+    return cudaErrorInvalidValue;
+  }
+}
+
 // Launchers of the 2D/3D pencil lengths, in four groups so that the largest
 // lengths compile as four translation units in parallel: the x pass and the
 // operator and y passes, the 1D whole-step kernels, the last pass (every
@@ -269,10 +282,7 @@ cudaError_t dispatch_proj_cols(long units, F&& f) {
   }                                                                                                   \
   template <>                                                                                         \
   cudaError_t launch_line1d<NN>(const Step1DArgs& a, const float2* tw, int nsolve, cudaStream_t s) {  \
-    const size_t sm = sizeof(LineSmem<NN>);                                                           \
-    cudaError_t e;                                                                                    \
-    if ((e = set_smem(k_line1d<NN>, sm)) != cudaSuccess) return e;                                    \
-    return launch_dep(k_line1d<NN>, nsolve, Line<NN>::BLOCK, sm, s, a, tw);                           \
+    return line1d_n<NN>(a, tw, nsolve, s);                                                            \
   }                                                                                                   \
   template <>                                                                                         \
   cudaError_t launch_ark1d<NN>(const Ark1DArgs& a, int nsolve, cudaStream_t s) {                      \
@@ -379,10 +389,7 @@ cudaError_t dispatch_proj_cols(long units, F&& f) {
   }                                                                                                   \
   template <>                                                                                         \
   cudaError_t launch_line1d<NN>(const Step1DArgs& a, const float2* tw, int nsolve, cudaStream_t s) {  \
-    const size_t sm = sizeof(LineSmem<NN>);                                                           \
-    cudaError_t e;                                                                                    \
-    if ((e = set_smem(k_line1d<NN>, sm)) != cudaSuccess) return e;                                    \
-    return launch_dep(k_line1d<NN>, nsolve, Line<NN>::BLOCK, sm, s, a, tw);                           \
+    return line1d_n<NN>(a, tw, nsolve, s);                                                            \
   }                                                                                                   \
   template <>                                                                                         \
   cudaError_t launch_ark1d<NN>(const Ark1DArgs& a, int nsolve, cudaStream_t s) {                      \

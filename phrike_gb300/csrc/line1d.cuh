@@ -33,6 +33,7 @@ namespace ps {
 
 template <int N>
 struct Line {
+  static_assert(N >= 16, "at least one pass beside the fused one");
   static constexpr int TH = N / 4;  // threads that hold points
   static constexpr int NP = (ilog2(N) - 2) / 2;  // radix-4 passes with an exchange after them (lengths > 8)
   static constexpr int RF = N >> (2 * NP);        // radix of the fused middle pass: 4 or 8
@@ -76,7 +77,7 @@ struct LineFft {
   LineSmem<N>& S;
   const int tid;
   const bool own;  // holds points
-  float2 tw[Ln::TW_SMEM ? 1 : (NP > 0 ? NP : 1)][3];
+  float2 tw[Ln::TW_SMEM ? 1 : NP][3];
   float ds[RF], fs[RF];  // derivative and filter symbols of the fused pass's outputs
 
   __device__ __forceinline__ void sync() const {
@@ -122,15 +123,6 @@ struct LineFft {
   // v[f][q]: points tid + q N/4 of the two transforms.  op 0: v <- -D v;
   // op 1: v <- C v, the complement of the filter; op 2: of the filter twice.
   __device__ __forceinline__ void round_trip(float2 (&v)[2][4], int op) {
-    if constexpr (NP == 0) {
-      if (own) {
-#pragma unroll
-        for (int f = 0; f < 2; ++f)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) S.buf[f][line_swz(tid + q * TH)] = v[f][q];
-      }
-      sync();
-    }
     sfor<0, NP>([&](auto pc) {
       constexpr int p = decltype(pc)::value;
       constexpr int m = len(p) / 4;
@@ -206,15 +198,6 @@ struct LineFft {
       }
       if constexpr (p > 0) sync();
     });
-    if constexpr (NP == 0) {
-      if (own) {
-#pragma unroll
-        for (int f = 0; f < 2; ++f)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) v[f][q] = S.buf[f][line_swz(tid + q * TH)];
-      }
-      sync();
-    }
   }
 };
 

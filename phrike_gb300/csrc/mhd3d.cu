@@ -433,7 +433,6 @@ cudaError_t launch_proj3_y(int n, bool inverse, const Proj3Args& a, cudaStream_t
       if ((e = set_smem(k_proj3_y<NN, T, false>, sm)) != cudaSuccess) return e;
       return launch_dep(k_proj3_y<NN, T, false>, grid, Shape<NN>::A * T, sm, s, a);
     }
-    return cudaGetLastError();
   });
 }
 
