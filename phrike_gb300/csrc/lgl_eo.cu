@@ -100,16 +100,18 @@ int encode_eo_map(CUtensorMap* m, const void* base, int h, int rows, int kp, int
 }
 
 // N tile for h output columns and mt tiles of 128 rows: waves of CTAs (one per
-// SM) times the work of one, its columns plus about 64 columns' worth of row
-// operand and set-up.  Every output is the same dot product for every tile.
-// 513 nodes (257 pairs) alone take 144 columns (136 CTAs, one wave), 257 nodes
-// (129 pairs) 48 (108 CTAs).
+// SM) times the work of one, its columns plus 128 columns' worth of row operand
+// and set-up.  Every output is the same dot product for every tile.  513 nodes
+// (257 pairs) alone take 144 columns (136 CTAs, one wave), 257 nodes (129 pairs)
+// 48 (108 CTAs).  Of 24 grids and batches from 129 to 1025 nodes, each timed at
+// all four, the rule takes the fastest tile; with 64 columns' worth it took 80 for
+// 144 at 385^2 x 14 (834 / 748 us per step), 449^2 x 8 (627 / 568) and 769^2 (272 / 210).
 int eo_n_tile(int h, long mt) {
   int best = 144;
   long cost = -1;
   for (int nt : kEoTiles) {
     const long waves = (mt * ((h + nt - 1) / nt) + 147) / 148;
-    const long c = waves * (nt + 64);
+    const long c = waves * (nt + 128);
     if (cost < 0 || c < cost) {
       cost = c;
       best = nt;

@@ -12,8 +12,8 @@
 // or mode from its digits (a few multiplications by float reciprocals; tables
 // of places missed the small L1 left beside the shared memory).
 //
-// Measured per RK4 step against the Stockham passes: 3840 x 2160 12.2 -> 3.65
-// ms (x pass 390, last pass 300, filter passes 460 and 340 us; the transforms
+// Measured per RK4 step against the Stockham passes: 3840 x 2160 12.2 -> 3.56
+// ms (x pass 390, last pass 300, the two filter passes 732 us; the transforms
 // are bound by instruction issue and shared-memory latency at 12-16 warps per
 // SM, HBM at 15%), mixed 2D and 3D grids of 10^4 to 10^6 points 2.0 to 4.6
 // times faster.
