@@ -236,9 +236,10 @@ __global__ void __launch_bounds__(128, 1)
       }
       tc_fence_after();
       const uint32_t st = base + s * SM::kStage;
-      const int steps = min(4, (ax.h - kb * 64 + 15) / 16);  // what lies past h is zero
-#pragma unroll 1
-      for (int kk = 0; kk < steps; ++kk) {
+      const int rest = ax.h - kb * 64;
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        if (kk * 16 >= rest) break;    // what lies past h is zero
         const uint32_t off = kk * 32;  // 16 bf16 along K
         uint64_t dA[P], dB[P];
 #pragma unroll
