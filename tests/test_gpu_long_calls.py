@@ -75,7 +75,7 @@ def test_divergence_over_a_long_call(n, d, interval, cfl):
     step, each of which projects the B that its stages start from.  In the long
     call no more than four steps pass without a projection, so the rounding
     divergence of four steps meets that of one: sqrt(4) = 2, 2.5 with a margin.
-    (Projecting at the filter's cadence alone leaves 5 to 6 times as much.)"""
+    (Projecting at the filter's cadence alone leaves up to 23 times as much.)"""
     from phrike_gb300.engine import Plan
     U0 = torch.as_tensor(orszag_tang(n, d), dtype=torch.float32, device="cuda").contiguous()
     kw = dict(gamma=5.0 / 3.0, equations="mhd", mhd_config={}, cfl=0.2,
